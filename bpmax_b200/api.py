@@ -221,7 +221,7 @@ class Engine:
 
     TUNING_KEYS = {"r0_pairs_per_job": 0, "r0_merge_items": 1, "class_streams": 2, "wait_limit_us": 3,
                    "inject_wait_timeout": 4, "wide_stages": 5, "r0_variant": 6, "class_share": 7,
-                   "persistent": 8}
+                   "persistent": 8, "strip_tasks": 9}
     #: the tunables bpmax_gpu_autotune chooses, in the order it reports them
     AUTOTUNED = ("r0_pairs_per_job", "r0_merge_items", "class_streams", "r0_variant", "wide_stages", "class_share",
                  "persistent")

@@ -5,7 +5,8 @@
 //   clear F; single-strand tables S1, S2 of every pair;
 //   for d = 0 .. max(M)-1:                     (outer wavefront over j1-i1, V3/bpmax.c:300-323)
 //     R0+R3+R4 product kernel over the cells (i1, i1+d) of every pair with M > d: jobs of k1
-//       offset pairs (w, d-1-w), ordered by offset pair so both uses of a table meet in L2;
+//       offset pairs (w, d-1-w), ordered by offset pair so both uses of a table meet in L2; from a
+//       certain size on, the strip kernel takes most offsets of several diagonals in one launch;
 //     finalize kernel over the same cells (init, SW1, inner R1/R2/SW2 wavefront, FT copy).
 // The whole sequence is captured once per shape as a CUDA graph and replayed.
 #include <cuda_runtime.h>
@@ -30,6 +31,7 @@
 #include "bpmax_r0only.cuh"
 #include "bpmax_wide.cuh"
 #include "bpmax_persist.cuh"
+#include "bpmax_strip.cuh"
 
 using namespace bpmax;
 
@@ -66,6 +68,24 @@ long long r0_pairs_per_job(long long cells, long long P2, long long resident, lo
     return best_q;
 }
 
+// Stages per strip job, the same way: jobs of q of the cells' `stages` stages and one merge each
+// (`merge_items` items' worth, three items to a stage)
+long long strip_stages_per_job(long long cells, long long stages, long long resident, long long qmax,
+                               long long merge_items)
+{
+    long long best_q = std::min(qmax, stages), best_cost = -1;
+    for (long long nch = 1; nch <= std::min<long long>(stages, 64); ++nch) {
+        const long long q = std::min(qmax, (stages + nch - 1) / nch);
+        const long long jobs = cells * ((stages + q - 1) / q);
+        const long long cost = (jobs + resident - 1) / resident * (3 * q + merge_items);
+        if (best_cost < 0 || cost < best_cost) {
+            best_cost = cost;
+            best_q = q;
+        }
+    }
+    return best_q;
+}
+
 struct DevBuf {
     void *p = nullptr;
     size_t bytes = 0;
@@ -79,20 +99,20 @@ struct Plan {
     int bases_bytes = 0;
     int maxM = 0;
     // per diagonal and Np class (index NB-1): ranges in the job arrays
-    // np = inner table width class; part (product launches): 0 = reads only diagonals <= d-2,
-    // 1 = reads diagonal d-1 too
+    // np = inner table width class; strip (product launches): strips of diagonals d .. d+T-1
     // cap: at most this many CTAs (0: as many as are resident), from the class shares
-    struct Launch { int d, np, first, count, s1_first = 0, s1_count = 0, part = 1, cap = 0; };
+    struct Launch { int d, np, first, count, s1_first = 0, s1_count = 0; bool strip = false; int cap = 0; };
     std::vector<Launch> r0_launches, fin_launches;
     std::vector<R0Job> r0_jobs;
+    std::vector<StripJob> strip_jobs;  // jobs of strip launches (first/count index this array)
     std::vector<R0JobL> r0l_jobs;  // jobs of launches with np > WIDE_TILE_MAX_NP (first/count index this array)
     std::vector<R0JobW> r0w_jobs;  // jobs of launches with tile-image tables (first/count index this array)
     std::vector<CellJob> cell_jobs;
     std::vector<int> classes;  // distinct inner widths, ascending
     int pairs_per_job = 0, merge_items = 0, class_streams = 1;  // tunables the plan was built with
     int r0_variant = 0, wide_stages = 2, class_share = 0, persist = 0;
+    long strip_tasks = 0;
     bool r0_only = false;  // R0-only double max-plus (bpmax_gpu_r0_only) instead of the BPMax fill
-    bool split = true;     // the product's offset pair 0 may run as its own launch (one-class plans)
     std::vector<cudaEvent_t> diag_ev;  // one pair only: outer diagonal d finalized (recorded by the graph)
     // persistent fill (one launch per width class walking the diagonals with dependency counters):
     // the work queues of all classes back to back, each class's range and CTA count
@@ -116,23 +136,16 @@ struct bpmax_ctx {
     cudaStream_t class_stream[8] = {};  // MAX_CLASS_STREAMS
     cudaStream_t aux_stream = nullptr;  // reference-layout conversion and copy-out, overlapped with the fill
     cudaEvent_t fork_ev = nullptr, join_ev[8] = {};
-    // per width-class chain: a side stream for the product part that reads only diagonals <= d-2,
-    // its completion event, and the chain's finalize events of the last two diagonals
-    cudaStream_t side_stream[8] = {};
-    cudaEvent_t side_done_ev[8] = {}, fin_ev[8][2] = {}, side_join_ev[8] = {};
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     Weights W;
     std::string err;
-    DevBuf F, FT, S, bases, pairs, r0jobs, r0ljobs, r0wjobs, celljobs, scores, conv, tbstack, grads, tbstatus, errflag;
+    DevBuf F, FT, S, bases, pairs, r0jobs, stripjobs, r0ljobs, r0wjobs, celljobs, scores, conv, tbstack, grads, tbstatus, errflag;
     DevBuf r0vals;         // R0-only mode: seq1 then seq2 of the pair, as floats
     DevBuf pq, pcnt, pneed;  // persistent fill: work queue; counters (class heads, diagonals, cells); jobs per cell
     bool copyout = false;    // the next fill copies the reference layout out per diagonal (graph path)
     RefOut want_ref{nullptr, 0, 0};  // the next fill's finalize also writes the reference layout there
     DevBuf refdev;                   // that reference layout, diagonal-major
     bool r0_only = false;  // mode of the next prepare()
-    // schedule of the next prepare(): with the reference-layout copy-out running beside the fill
-    // (bpmax_gpu_fill), the unsplit product leaves the SMs the row conversions need
-    bool allow_split = true;
     int r0_occ_v[2][9] = {};  // resident product CTAs per SM, per shape variant and width class NB
     int wide_occ[4] = {};     // resident tile-product CTAs per SM, per stage count
     // schedule tunables (bpmax_gpu_set_tuning / bpmax_gpu_autotune); a plan is built with the
@@ -144,6 +157,7 @@ struct bpmax_ctx {
     int wide_stages = 2;                            // shared-memory stages of the tile-image product (2 or 3)
     int class_share = 0;                            // cap each width class's product CTAs by its share of the work
     int persist = 0;  // width classes <= 64 by the persistent kernel: 0 no, 1 side by side, 2 one after another
+    long strip_tasks = 3400;                        // least product tasks per SM of a strip launch
     int persist_occ[9] = {};                        // resident persistent-fill CTAs per SM, per width class
     // bounded waits of the product kernels: time limit of one wait, and the one-shot test mode in
     // which the next fill's product kernels issue no copies (their first waits run out)
@@ -314,11 +328,11 @@ int build_plan(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int
     P.pairs_per_job = ctx->r0_pairs_per_job;
     P.merge_items = ctx->r0_merge_items;
     P.class_streams = ctx->class_streams;
-    P.split = ctx->allow_split;
     P.r0_variant = ctx->r0_variant;
     P.wide_stages = ctx->wide_stages;
     P.class_share = ctx->class_share;
     P.persist = ctx->persist;
+    P.strip_tasks = ctx->strip_tasks;
     const auto tu = ctx->tuned.find(shape_key(Ms, Ns));
     if (tu != ctx->tuned.end()) {
         P.pairs_per_job = tu->second[0];
@@ -405,37 +419,57 @@ int build_plan(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int
             P.fin_launches.push_back(fl);
             if (d == 0) continue;
             if (np <= MAX_SMALL_NP) {
-                // jobs of q offset pairs (w, d-1-w), ordered by pair chunk, then pair, then cell: the
-                // two uses of a table (A of cell (a, a+d) at offset w, B of cell (a+w-d, a+w) at
-                // offset d-1-w) fall in the same pair chunk
+                // Strips of T cells (bpmax_strip.cuh), once per T diagonals d .. d+T-1 (d = 1 mod T): the
+                // offsets [T-1, d-1], which read only diagonals < d for every cell of a strip. The T-1
+                // offset pairs (w, d-1-w) at the ends of every cell's range are the jobs of r0_kernel,
+                // diagonal by diagonal (they repeat up to T-1 offsets of the strip: a maximum). Diagonals
+                // with little work keep r0_kernel alone: a strip launch adds a launch to the chain and
+                // clears T merge tiles per CTA. Fill ms with strips everywhere / from 3,400 tasks (28
+                // width-64 items) per SM / nowhere: 37x23 0.66 / 0.57 / 0.55, 128x64 6.69 / 6.57 / 6.52,
+                // 200x40 7.93 / 7.63 / 7.64, 200x64 13.8 / 13.7 / 14.2, 256x64 21.8 / 21.4 / 23.4.
                 const int NB = np / 8, G = R0_TAB_ITEMS[NB];
                 const long long P2 = (d + 1) / 2;  // offset pairs per cell
+                long long edge = P2;               // offset pairs per cell of r0_kernel's jobs
+                const int T = strip_cells(NB), d0 = d - (d - 1) % T;  // the strips' first diagonal
+                long long cells0 = 0;
+                for (int p = 0; p < n; ++p)
+                    if (P.pairs[p].Np == np && Ms[p] > d0) cells0 += Ms[p] - d0;
+                // tasks of an item: NB(NB+1)(NB+2)/6
+                if (NB >= STRIP_MIN_NB && d0 >= T &&
+                    cells0 * (d0 - T + 1) * (NB * (NB + 1) * (NB + 2) / 6) >= P.strip_tasks * ctx->sms) {
+                    edge = std::min<long long>(P2, T - 1);
+                    if (d == d0) {
+                        const long long stages = (d - T + G) / G;  // of G offsets
+                        const long long resident = capped(np, ctx->sms);
+                        const long long q =
+                            strip_stages_per_job(cells, stages, resident, std::max<long long>(1, 2LL * P.pairs_per_job / G),
+                                                 P.merge_items);
+                        Plan::Launch sl{d, np, (int)P.strip_jobs.size(), 0};
+                        sl.strip = true;
+                        sl.cap = (int)resident;
+                        for (long long w0 = T - 1; w0 < d; w0 += q * G)
+                            for (int p = 0; p < n; ++p)
+                                if (P.pairs[p].Np == np && Ms[p] > d)
+                                    for (int i1 = 0; i1 < Ms[p] - d; ++i1)
+                                        P.strip_jobs.push_back(StripJob{p, i1, (int)w0, (int)std::min<long long>(w0 + q * G, d)});
+                        sl.count = (int)P.strip_jobs.size() - sl.first;
+                        P.r0_launches.push_back(sl);
+                    }
+                }
+                // jobs of q offset pairs, ordered by pair chunk, then pair, then cell: the two uses of a
+                // table (A of cell (a, a+d) at offset w, B of cell (a+w-d, a+w) at offset d-1-w) fall in
+                // the same pair chunk
                 const long long resident =
                     capped(np, (long long)std::max(1, ctx->r0_occ_v[P.r0_variant][NB]) * ctx->sms);
                 const long long qmin = std::max(1, (G + 1) / 2), qmax = std::max<long long>(P.pairs_per_job, qmin);
-                // Offset pair 0 (offsets 0 and d-1) is the only one that reads diagonal d-1. In a plan
-                // of one width class, where one iteration holds at most 2 items, it becomes its own
-                // launch (part 1) and the other pairs (part 0, reading diagonals <= d-2) can run while
-                // diagonal d-1 is finalized (several classes already overlap each other's finalize).
-                const long long first_pair = (P.split && classes.size() == 1 && G <= 2 && P2 > 1) ? 1 : 0;
-                if (first_pair) {
-                    Plan::Launch rb{d, np, (int)P.r0_jobs.size(), 0};
-                    rb.cap = share.empty() ? 0 : (int)resident;
-                    for (int p = 0; p < n; ++p)
-                        if (P.pairs[p].Np == np && Ms[p] > d)
-                            for (int i1 = 0; i1 < Ms[p] - d; ++i1) P.r0_jobs.push_back(R0Job{p, i1, 0, 1});
-                    rb.count = (int)P.r0_jobs.size() - rb.first;
-                    P.r0_launches.push_back(rb);
-                }
-                const long long q = r0_pairs_per_job(cells, P2 - first_pair, resident, qmin, qmax, P.merge_items);
+                const long long q = r0_pairs_per_job(cells, edge, resident, qmin, qmax, P.merge_items);
                 Plan::Launch rl{d, np, (int)P.r0_jobs.size(), 0};
-                rl.part = first_pair ? 0 : 1;
                 rl.cap = share.empty() ? 0 : (int)resident;
-                for (long long c0 = first_pair; c0 < P2; c0 += q)
+                for (long long c0 = 0; c0 < edge; c0 += q)
                     for (int p = 0; p < n; ++p)
                         if (P.pairs[p].Np == np && Ms[p] > d)
                             for (int i1 = 0; i1 < Ms[p] - d; ++i1)
-                                P.r0_jobs.push_back(R0Job{p, i1, (int)c0, (int)std::min(c0 + q, P2)});
+                                P.r0_jobs.push_back(R0Job{p, i1, (int)c0, (int)std::min(c0 + q, edge)});
                 rl.count = (int)P.r0_jobs.size() - rl.first;
                 P.r0_launches.push_back(rl);
                 continue;
@@ -582,6 +616,14 @@ void launch_r0_v(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
 }
 
 template <int NB>
+void launch_strip(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
+{
+    r0_strip_kernel<NB><<<std::min(L.count, L.cap), StripCfg<NB>::THREADS, StripCfg<NB>::SMEM, s>>>(
+        (const StripJob *)ctx->stripjobs.p + L.first, L.count, (const PairDesc *)ctx->pairs.p, (float *)ctx->F.p, L.d,
+        wait_ctl(ctx));
+}
+
+template <int NB>
 void launch_persist(bpmax_ctx *ctx, const PersistCtl &pc, int ctas, cudaStream_t s)
 {
     fill_persistent_kernel<NB><<<ctas, R0Cfg<NB>::THREADS, R0Cfg<NB>::SMEM, s>>>(
@@ -592,6 +634,8 @@ void launch_persist(bpmax_ctx *ctx, const PersistCtl &pc, int ctas, cudaStream_t
 template <int NB>
 void launch_r0(bpmax_ctx *ctx, const Plan &P, const Plan::Launch &L, cudaStream_t s)
 {
+    if constexpr (NB >= STRIP_MIN_NB)
+        if (L.strip) return launch_strip<NB>(ctx, L, s);
     if (P.r0_variant == 1)
         launch_r0_v<NB, 1>(ctx, L, s);
     else
@@ -644,7 +688,7 @@ void launch_r0only_fin(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
 // The product kernels, the small finalize and the persistent fill prefer the largest shared-memory
 // carveout: an SM runs CTAs of different kernels side by side only when they use the same L1 /
 // shared-memory split (parallel graph branches of a batch, the persistent launches of its width
-// classes, the split product launches of one class).
+// classes).
 template <typename K>
 int prefer_smem(bpmax_ctx *ctx, K kernel)
 {
@@ -661,6 +705,10 @@ int set_smem_attr(bpmax_ctx *ctx)
         return st;
     if constexpr (8 * NB >= 48)
         if ((st = prefer_smem(ctx, finalize_small_kernel<8 * NB, FIN_BULK_THREADS>))) return st;
+    if constexpr (NB >= STRIP_MIN_NB) {
+        if ((st = prefer_smem(ctx, r0_strip_kernel<NB>))) return st;
+        CK(cudaFuncSetAttribute(r0_strip_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)StripCfg<NB>::SMEM));
+    }
     if (NB == 8)
         if ((st = prefer_smem(ctx, r0_wide_kernel<2>)) || (st = prefer_smem(ctx, r0_wide_kernel<3>)) ||
             (st = prefer_smem(ctx, r0_large_kernel)))
@@ -798,40 +846,15 @@ int enqueue_fill(bpmax_ctx *ctx, Plan &P, KernelProfile *kp = nullptr)
     };
     auto stream_of = [&](int np) { return fork ? ctx->class_stream[chain_of(np)] : ctx->stream; };
     const int nstreams = fork ? std::min((int)P.classes.size(), MAX_CLASS_STREAMS) : 0;
-    // product launches that read only diagonals <= d-2 (part 0) run on each chain's side stream,
-    // after the finalize of d-2, so they overlap the finalize of d-1; the chain's finalize of d
-    // waits for them
-    bool any_part0 = false;
-    for (const auto &L : P.r0_launches) any_part0 = any_part0 || L.part == 0;
-    const bool split = !prof && any_part0;
-    const int nside = split ? std::max(nstreams, 1) : 0;
-    if (fork || split) {
+    if (fork) {
         CK(cudaEventRecord(ctx->fork_ev, ctx->stream));
         for (int k = 0; k < nstreams; ++k) CK(cudaStreamWaitEvent(ctx->class_stream[k], ctx->fork_ev, 0));
-        for (int k = 0; k < nside; ++k) CK(cudaStreamWaitEvent(ctx->side_stream[k], ctx->fork_ev, 0));
     }
-    bool side_pending[MAX_CLASS_STREAMS] = {};
     size_t ri = 0, fi = 0;
     for (int d = 0; d < P.maxM; ++d) {
         for (; ri < P.r0_launches.size() && P.r0_launches[ri].d == d; ++ri, ++launches) {
             const auto &L = P.r0_launches[ri];
-            const int c = chain_of(L.np);
-            cudaStream_t st = stream_of(L.np);
-            if (split && L.part == 0) {
-                // Part 0 of diagonal d (offset pairs >= 1) may run beside the finalize of d-1 because:
-                //  1. it reads only tables of diagonals <= d-2, and waits here for the finalize of d-2,
-                //     the last writer of those tables and of the SW1 candidates pushed into the still
-                //     cleared tables of diagonal d (a finalize of diagonal e writes only the tables of
-                //     e, the S1 pieces of e and the pushes into e+2);
-                //  2. it writes the tables of diagonal d only through atomicMax of partial maxima,
-                //     which commutes with part 1's merges and with those pushes (all values >= +0);
-                //  3. the finalize of d-1 writes no table of diagonal d, and the finalize of d waits
-                //     for both parts (side_done_ev below).
-                // A finalize that wrote diagonal d, or a product merge that was not an atomic max,
-                // would race here.
-                st = ctx->side_stream[c];
-                if (d >= 2) CK(cudaStreamWaitEvent(st, ctx->fin_ev[c][d & 1], 0));  // finalize of d-2
-            }
+            const cudaStream_t st = stream_of(L.np);
             {
                 ProfScope ps(ctx, kp, 1);
                 switch (L.np > MAX_SMALL_NP ? 0 : L.np / 8) {
@@ -851,16 +874,10 @@ int enqueue_fill(bpmax_ctx *ctx, Plan &P, KernelProfile *kp = nullptr)
                 default: launch_r0<8>(ctx, P, L, st); break;
                 }
             }
-            if (split && L.part == 0) {
-                CK(cudaEventRecord(ctx->side_done_ev[c], st));
-                side_pending[c] = true;
-            }
         }
         for (; fi < P.fin_launches.size() && P.fin_launches[fi].d == d; ++fi, ++launches) {
             const auto &L = P.fin_launches[fi];
-            const int c = chain_of(L.np);
             const cudaStream_t st = stream_of(L.np);
-            if (side_pending[c]) CK(cudaStreamWaitEvent(st, ctx->side_done_ev[c], 0));
             {
                 ProfScope ps(ctx, kp, 2);
                 if (P.r0_only) {
@@ -879,17 +896,11 @@ int enqueue_fill(bpmax_ctx *ctx, Plan &P, KernelProfile *kp = nullptr)
                     }
                 }
             }
-            if (split) CK(cudaEventRecord(ctx->fin_ev[c][d & 1], st));
         }
-        for (bool &p : side_pending) p = false;
         // outer diagonal d is final: rows of the reference layout that end on it can be copied out
         // (events recorded as external nodes of the captured graph; eager runs record none)
         if (!P.diag_ev.empty() && !prof && capturing)
             CK(cudaEventRecordWithFlags(P.diag_ev[d], ctx->stream, cudaEventRecordExternal));
-    }
-    for (int k = 0; k < nside; ++k) {  // join the side streams back into the main stream
-        CK(cudaEventRecord(ctx->side_join_ev[k], ctx->side_stream[k]));
-        CK(cudaStreamWaitEvent(ctx->stream, ctx->side_join_ev[k], 0));
     }
     for (int k = 0; k < nstreams; ++k) {  // join the class chains back into the main stream
         CK(cudaEventRecord(ctx->join_ev[k], ctx->class_stream[k]));
@@ -913,11 +924,11 @@ int prepare(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int> &
     const bool same_tuning = ctx->plan.pairs_per_job == want[0] && ctx->plan.merge_items == want[1] &&
                              ctx->plan.class_streams == want[2] && ctx->plan.r0_variant == want[3] &&
                              ctx->plan.wide_stages == want[4] && ctx->plan.class_share == want[5] &&
-                             ctx->plan.persist == want[6] && ctx->plan.copyout == ctx->copyout &&
+                             ctx->plan.persist == want[6] && ctx->plan.strip_tasks == ctx->strip_tasks &&
+                             ctx->plan.copyout == ctx->copyout &&
                              ctx->plan.ref.out == ctx->want_ref.out && ctx->plan.ref.T == ctx->want_ref.T &&
                              ctx->plan.ref.Ns == ctx->want_ref.Ns;
-    if (!(ctx->plan_valid && ctx->plan.Ms == Ms && ctx->plan.Ns == Ns && same_tuning && ctx->plan.r0_only == ctx->r0_only &&
-          ctx->plan.split == ctx->allow_split)) {
+    if (!(ctx->plan_valid && ctx->plan.Ms == Ms && ctx->plan.Ns == Ns && same_tuning && ctx->plan.r0_only == ctx->r0_only)) {
         if (ctx->plan.graph) cudaGraphExecDestroy(ctx->plan.graph);
         ctx->plan.graph = nullptr;
         for (cudaEvent_t e : ctx->plan.diag_ev) cudaEventDestroy(e);
@@ -938,6 +949,7 @@ int prepare(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int> &
         if ((st = ensure(ctx, ctx->bases, P.bases_bytes + 16)) != BPMAX_OK) return st;
         if ((st = ensure(ctx, ctx->pairs, P.pairs.size() * sizeof(PairDesc))) != BPMAX_OK) return st;
         if ((st = ensure(ctx, ctx->r0jobs, P.r0_jobs.size() * sizeof(R0Job))) != BPMAX_OK) return st;
+        if ((st = ensure(ctx, ctx->stripjobs, P.strip_jobs.size() * sizeof(StripJob))) != BPMAX_OK) return st;
         if ((st = ensure(ctx, ctx->r0ljobs, P.r0l_jobs.size() * sizeof(R0JobL))) != BPMAX_OK) return st;
         if ((st = ensure(ctx, ctx->r0wjobs, P.r0w_jobs.size() * sizeof(R0JobW))) != BPMAX_OK) return st;
         if (P.persistent) {
@@ -955,6 +967,9 @@ int prepare(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int> &
         CK(cudaMemcpyAsync(ctx->pairs.p, P.pairs.data(), P.pairs.size() * sizeof(PairDesc), cudaMemcpyHostToDevice, ctx->stream));
         if (!P.r0_jobs.empty())
             CK(cudaMemcpyAsync(ctx->r0jobs.p, P.r0_jobs.data(), P.r0_jobs.size() * sizeof(R0Job), cudaMemcpyHostToDevice, ctx->stream));
+        if (!P.strip_jobs.empty())
+            CK(cudaMemcpyAsync(ctx->stripjobs.p, P.strip_jobs.data(), P.strip_jobs.size() * sizeof(StripJob),
+                               cudaMemcpyHostToDevice, ctx->stream));
         if (!P.r0w_jobs.empty())
             CK(cudaMemcpyAsync(ctx->r0wjobs.p, P.r0w_jobs.data(), P.r0w_jobs.size() * sizeof(R0JobW), cudaMemcpyHostToDevice,
                                ctx->stream));
@@ -1152,12 +1167,7 @@ int bpmax_gpu_create(int device, bpmax_ctx **out)
     if (st == BPMAX_OK && cudaStreamCreateWithFlags(&ctx->aux_stream, cudaStreamNonBlocking) != cudaSuccess) st = BPMAX_ECUDA;
     for (int k = 0; k < MAX_CLASS_STREAMS && st == BPMAX_OK; ++k)
         if (cudaStreamCreateWithFlags(&ctx->class_stream[k], cudaStreamNonBlocking) != cudaSuccess ||
-            cudaEventCreateWithFlags(&ctx->join_ev[k], cudaEventDisableTiming) != cudaSuccess ||
-            cudaStreamCreateWithFlags(&ctx->side_stream[k], cudaStreamNonBlocking) != cudaSuccess ||
-            cudaEventCreateWithFlags(&ctx->side_done_ev[k], cudaEventDisableTiming) != cudaSuccess ||
-            cudaEventCreateWithFlags(&ctx->side_join_ev[k], cudaEventDisableTiming) != cudaSuccess ||
-            cudaEventCreateWithFlags(&ctx->fin_ev[k][0], cudaEventDisableTiming) != cudaSuccess ||
-            cudaEventCreateWithFlags(&ctx->fin_ev[k][1], cudaEventDisableTiming) != cudaSuccess)
+            cudaEventCreateWithFlags(&ctx->join_ev[k], cudaEventDisableTiming) != cudaSuccess)
             st = BPMAX_ECUDA;
     if (st == BPMAX_OK) st = set_smem_attr<1>(ctx);
     if (st == BPMAX_OK) st = set_smem_attr<2>(ctx);
@@ -1183,7 +1193,7 @@ void bpmax_gpu_destroy(bpmax_ctx *ctx)
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     if (ctx->plan.graph) cudaGraphExecDestroy(ctx->plan.graph);
     for (DevBuf *b : {&ctx->tbstack, &ctx->grads, &ctx->tbstatus, &ctx->F, &ctx->FT, &ctx->S, &ctx->bases, &ctx->pairs,
-                      &ctx->r0jobs, &ctx->r0ljobs, &ctx->r0wjobs, &ctx->pq, &ctx->pcnt, &ctx->pneed, &ctx->celljobs,
+                      &ctx->r0jobs, &ctx->stripjobs, &ctx->r0ljobs, &ctx->r0wjobs, &ctx->pq, &ctx->pcnt, &ctx->pneed, &ctx->celljobs,
                       &ctx->scores, &ctx->conv, &ctx->refdev, &ctx->errflag,
                       &ctx->r0vals})
         if (b->p) cudaFree(b->p);
@@ -1199,9 +1209,6 @@ void bpmax_gpu_destroy(bpmax_ctx *ctx)
     for (int k = 0; k < MAX_CLASS_STREAMS; ++k) {
         if (ctx->class_stream[k]) cudaStreamDestroy(ctx->class_stream[k]);
         if (ctx->join_ev[k]) cudaEventDestroy(ctx->join_ev[k]);
-        if (ctx->side_stream[k]) cudaStreamDestroy(ctx->side_stream[k]);
-        for (cudaEvent_t e : {ctx->side_done_ev[k], ctx->side_join_ev[k], ctx->fin_ev[k][0], ctx->fin_ev[k][1]})
-            if (e) cudaEventDestroy(e);
     }
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
@@ -1336,9 +1343,8 @@ int bpmax_gpu_fill(bpmax_ctx *ctx, const int *seq1, long M, const int *seq2, lon
     if (!pinned && (st = ensure_host_stage(ctx, row_max * sizeof(float))) != BPMAX_OK) return st;
     // Widths <= 64 into pinned memory: the finalize launches themselves write every cell they
     // complete in the reference layout (diagonal-major, on the device), so only copy engines work
-    // beside the fill, which keeps its split schedule. Without room for that buffer, or wider,
-    // a conversion launch per diagonal does it (those launches share the SMs with the fill's,
-    // so the fill then runs unsplit).
+    // beside the fill. Without room for that buffer, or wider, a conversion launch per diagonal does
+    // it (those launches share the SMs with the fill's).
     const size_t fused_bytes = (size_t)(M * (M + 1) / 2) * cell_f * sizeof(float);
     bool fused = false;
     if (pinned && padded_width((int)N) <= MAX_SMALL_NP) {
@@ -1356,10 +1362,8 @@ int bpmax_gpu_fill(bpmax_ctx *ctx, const int *seq1, long M, const int *seq2, lon
         }
     }
     ctx->want_ref = fused ? RefOut{(float *)ctx->refdev.p, (int)N_tile, (int)Ns} : RefOut{nullptr, 0, 0};
-    ctx->allow_split = fused;
     ctx->copyout = true;
     st = fill_pairs(ctx, 1, &seq1, &M, &seq2, &N, true);
-    ctx->allow_split = true;
     ctx->copyout = false;
     ctx->want_ref = RefOut{nullptr, 0, 0};
     if (st != BPMAX_OK) return st;
@@ -1554,6 +1558,10 @@ int bpmax_gpu_set_tuning(bpmax_ctx *ctx, int key, long value)
     case BPMAX_TUNE_CLASS_SHARE:
         ctx->class_share = value != 0;
         break;
+    case BPMAX_TUNE_STRIP_TASKS:
+        if (value < 0) return fail(ctx, BPMAX_EINVAL, "strip tasks must be >= 0");
+        ctx->strip_tasks = std::min<long>(value, 1L << 40);
+        break;
     case BPMAX_TUNE_PERSISTENT:
         if (value < 0 || value > 2) return fail(ctx, BPMAX_EINVAL, "persistent mode must be 0, 1 or 2");
         ctx->persist = (int)value;
@@ -1575,6 +1583,7 @@ int bpmax_gpu_get_tuning(const bpmax_ctx *ctx, int key, long *value)
     case BPMAX_TUNE_WIDE_STAGES: *value = ctx->wide_stages; break;
     case BPMAX_TUNE_R0_VARIANT: *value = ctx->r0_variant; break;
     case BPMAX_TUNE_CLASS_SHARE: *value = ctx->class_share; break;
+    case BPMAX_TUNE_STRIP_TASKS: *value = ctx->strip_tasks; break;
     case BPMAX_TUNE_PERSISTENT: *value = ctx->persist; break;
     default: return BPMAX_EINVAL;
     }

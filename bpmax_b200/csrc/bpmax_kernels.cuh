@@ -200,11 +200,12 @@ __global__ void single_strand_kernel(const PairDesc *__restrict__ pairs, const u
 //   S1(i1,j1)+S2(i2,j2)
 //   SW2 = F(i1,j1,i2+1,j2-1)+intra(s2r[i2],s2r[j2]) if j2-i2>=4
 //   R1 (:614-640) max_{k2} F(i1,j1,i2,k2)+S2(k2+1,j2); R2 (:641-667) max_{k2} S2(i2,k2)+F(i1,j1,k2+1,j2)
-// F arrives holding max(R0,R3,R4,SW1) (or +0): SW1 = F(i1+1,j1-1,.)+intra(s1[i1],s1[j1])
-// (V3/bpmax_outer_south_west.c:115-160) was stored into this cell's still-cleared table by the
-// finalize of (i1+1, j1-1) two diagonals earlier, before any product touched it. Every literal-0
-// candidate is covered because every value is >= +0. Writes the cell's blocks (-inf outside the
-// logical triangle, S1(i1,j1) on the subdiagonal) and its S1 pieces.
+//   SW1 = F(i1+1,j1-1,.)+intra(s1[i1],s1[j1]) if j1-i1>=4     (V3/bpmax_outer_south_west.c:115-160)
+// F arrives holding max(R0,R3,R4) (or +0), merged there by products of any earlier launch since the
+// table was cleared: SW1 is read here from the table of (i1+1, j1-1), so nothing but products
+// writes a table before its own finalize, and those of diagonal d may run before the finalize of
+// d-1 and d-2. Every literal-0 candidate is covered because every value is >= +0. Writes the cell's
+// blocks (-inf outside the logical triangle, S1(i1,j1) on the subdiagonal) and its S1 pieces.
 // The inner wavefront pushes forward: every inner cell (i2,j2), e2 = j2-i2 >= 1, has one owner
 // thread that keeps its running maximum in a register. When inner diagonal e is final, each
 // owner adds its two candidates that read diagonal e,
@@ -347,8 +348,15 @@ finalize_small_kernel(const CellJob *__restrict__ jobs, int njobs, const CellJob
         *reinterpret_cast<float4 *>(S2s + 4 * q4) = *reinterpret_cast<const float4 *>(S2 + 4 * q4);
     for (int q = tid; q < NP; q += Sh::THREADS) sb[q] = q < N ? s2r[q] : 4;
     __syncthreads();
-    // accumulated value of inner cell (r, c), r <= c, from the cell image
-    auto img = [&](int r, int c) { return Fc[cbs[c >> 3] + 68 * (r >> 3) + 8 * (r & 7) + (c & 7)]; };
+    // start value of inner cell (r, c), r <= c: accumulated products, S1+S2, SW1
+    const bool sw1 = d >= 4;
+    const float w1 = sw1 ? score_w(wsh, s1[i1], s1[j1]) : 0.0f;
+    const float *Fi = sw1 ? F + pd.F_off + cell_index(M, i1 + 1, j1 - 1) * CELL : nullptr;
+    auto start = [&](int r, int c) {
+        const int o = cbs[c >> 3] + 68 * (r >> 3) + 8 * (r & 7) + (c & 7);
+        const float v = fmaxf(Fc[o], s1v + S2s[r * NP + c]);
+        return sw1 ? fmaxf(v, Fi[o] + w1) : v;
+    };
     // owned inner cells c = tid + THREADS*k among the N(N-1)/2 cells with e2 >= 1, ordered by
     // (e2, i2): running maxima start at max(accumulated, S1+S2)
     const int ncells = N * (N - 1) / 2;
@@ -366,12 +374,12 @@ finalize_small_kernel(const CellJob *__restrict__ jobs, int njobs, const CellJob
             while (rem >= N - e) { rem -= N - e; ++e; }
             cell_e[k] = e;
             cell_i[k] = rem;
-            acc[k] = fmaxf(img(rem, rem + e), s1v + S2s[rem * NP + rem + e]);
+            acc[k] = start(rem, rem + e);
             if (e >= 4) sw2[k] = score_w(wsh, sb[rem], sb[rem + e]);
         }
     }
     if (tid < N)  // inner diagonal 0
-        D[tid] = d == 0 ? score_w(wsh + 6, s1[i1], sb[tid]) : fmaxf(img(tid, tid), s1v + S2s[tid * NP + tid]);
+        D[tid] = d == 0 ? score_w(wsh + 6, s1[i1], sb[tid]) : start(tid, tid);
     __syncthreads();
     // slot k of every thread holds cells THREADS*k .. THREADS*(k+1)-1 of the (e2, i2) order, so the
     // slots whose cells are all final (e2 <= e) are the same for every thread: the step enters the
@@ -405,26 +413,19 @@ finalize_small_kernel(const CellJob *__restrict__ jobs, int njobs, const CellJob
         }
         __syncthreads();
     }
-    // write-back, 4 columns of one block row per step; SW1 candidate of cell (i1-1, j1+1), whose
-    // table nothing else has written yet
-    const bool push = i1 >= 1 && j1 + 1 < M && d + 2 >= 4;
-    const float wp = push ? score_w(wsh, s1[i1 - 1], s1[j1 + 1]) : 0.0f;
-    float *Fn = push ? F + pd.F_off + cell_index(M, i1 - 1, j1 + 1) * CELL : nullptr;
+    // write-back, 4 columns of one block row per step
     for (int q4 = tid; q4 < NBLK * 16; q4 += Sh::THREADS) {
         int BI, BJ;
         blk_decode(NB, q4 >> 4, BI, BJ);
         const int r = 8 * BI + ((q4 & 15) >> 1), c0 = 8 * BJ + 4 * (q4 & 1);
-        float v[4], u[4];
+        float v[4];
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
             const int c = c0 + t;
-            const bool valid = r <= c && c < N;
-            v[t] = valid ? D[(c - r) * NP + r] : (r == c + 1 ? s1v : NEG_INF);  // S1 on the subdiagonal
-            u[t] = valid ? v[t] + wp : 0.0f;
+            v[t] = r <= c && c < N ? D[(c - r) * NP + r] : (r == c + 1 ? s1v : NEG_INF);  // S1 on the subdiagonal
         }
-        const int o = cbs[BJ] + 68 * BI + 4 * (q4 & 15);  // block (BI, BJ), row r & 7, half
-        if (push) *reinterpret_cast<float4 *>(Fn + o) = make_float4(u[0], u[1], u[2], u[3]);
-        *reinterpret_cast<float4 *>(Fc + o) = make_float4(v[0], v[1], v[2], v[3]);
+        // block (BI, BJ), row r & 7, half
+        *reinterpret_cast<float4 *>(Fc + cbs[BJ] + 68 * BI + 4 * (q4 & 15)) = make_float4(v[0], v[1], v[2], v[3]);
     }
     if (tid < 2 * NB) {  // S1 piece of every block column: -inf x7, S1(i1,j1)
         const int BJ = tid >> 1, h = tid & 1;

@@ -140,7 +140,10 @@ int bpmax_gpu_grad_batch(bpmax_ctx *ctx, int num_pairs, const int *const *seq1s,
  *                                several width classes, 1 runs them side by side (each on its share of
  *                                the SMs), 2 one after another (each on every SM); 0: a graph of two
  *                                launches per outer diagonal. The R0-only mode and bpmax_gpu_fill's
- *                                per-diagonal copy-out keep the graph. */
+ *                                per-diagonal copy-out keep the graph.
+ *   BPMAX_TUNE_STRIP_TASKS       least product work of a strip launch (strand-2 lengths 9..64: one
+ *                                launch for several outer diagonals), in 8x8x8 tasks per SM; 0: strips
+ *                                wherever a diagonal has offsets for them (default 3400) */
 enum bpmax_tuning_key {
     BPMAX_TUNE_R0_PAIRS_PER_JOB = 0,
     BPMAX_TUNE_R0_MERGE_ITEMS = 1,
@@ -150,7 +153,8 @@ enum bpmax_tuning_key {
     BPMAX_TUNE_WIDE_STAGES = 5,
     BPMAX_TUNE_R0_VARIANT = 6,
     BPMAX_TUNE_CLASS_SHARE = 7,
-    BPMAX_TUNE_PERSISTENT = 8
+    BPMAX_TUNE_PERSISTENT = 8,
+    BPMAX_TUNE_STRIP_TASKS = 9
 };
 int bpmax_gpu_set_tuning(bpmax_ctx *ctx, int key, long value);
 int bpmax_gpu_get_tuning(const bpmax_ctx *ctx, int key, long *value);
