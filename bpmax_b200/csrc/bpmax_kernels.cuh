@@ -206,14 +206,21 @@ __global__ void single_strand_kernel(const PairDesc *__restrict__ pairs, const u
 // writes a table before its own finalize, and those of diagonal d may run before the finalize of
 // d-1 and d-2. Every literal-0 candidate is covered because every value is >= +0. Writes the cell's
 // blocks (-inf outside the logical triangle, S1(i1,j1) on the subdiagonal) and its S1 pieces.
-// The inner wavefront pushes forward: every inner cell (i2,j2), e2 = j2-i2 >= 1, has one owner
-// thread that keeps its running maximum in a register. When inner diagonal e is final, each
-// owner adds its two candidates that read diagonal e,
+// The inner wavefront goes by batches of FIN_BATCH = 5 inner diagonals of the cell's table in shared
+// memory, D[e][i2] = F[i2][i2+e], each open entry holding its running maximum. A final diagonal e
+// gives every entry (i2, j2) of diagonal e2 > e the candidates
 //   R1 with k2 = i2+e:    F[i2][i2+e] + S2(i2+e+1, j2)
 //   R2 with k2 = j2-e-1:  S2(i2, j2-e-1) + F[j2-e][j2]
-// to every open cell (e2 > e); the cells of diagonal e+1 have then seen all their R1/R2 terms
-// and are final after SW2. One CTA barrier per inner diagonal; the diagonals are kept in shared
-// memory diagonal-major, D[e][i2] = F[i2][i2+e].
+// S2 is 0 on spans <= 3, so those of e = e2-1 are F[i2][j2-1] and F[i2+1][j2] themselves, which are
+// never less than the ones of e = e2-2 .. e2-4 (each of those is a candidate of them, plus 0): only
+// e <= e2-5 is left to add. So within a batch an entry needs no more than its two neighbours of the
+// previous diagonal and SW2, and one warp runs the batch's five steps in registers, two rows per
+// lane and one shuffle per step, without a CTA barrier; the sums go to later batches in bulk: to the
+// next batch first, by all warps, then, while the first warp runs that batch, to all others by the
+// other warps. Two CTA barriers per batch (26 at width 64; one step per barrier took 63).
+// Bound: latency, about 6 us of a 64-wide cell in the inner wavefront and 3 us of dependent global loads
+// before it. Fill ms with one barriered step per inner diagonal / with batches: 37x23 0.57 / 0.53,
+// 128x64 6.52 / 4.83, 200x64 13.7 / 11.0, 1024x64 661 / 640, the 512-pair batch 460 / 428.
 // CTAs after the first njobs compute S1 on diagonal d+1 (V3/bpmax_verify.c:533-544), one warp
 // per cell, from S1 diagonals <= d (S1 is cleared to 0 before the fill; j-i <= 3 stays 0).
 // ------------------------------------------------------------------------------------------
@@ -221,10 +228,15 @@ struct CellJob {
     int pair, i1;
 };
 
-// threads per cell: the wavefront's serial work per step is K owned cells per thread. Fewer
-// threads per cell cost latency per cell but issue fewer instructions per step in total, which pays
-// when a launch holds many more cells than the GPU runs at once (FIN_WIDE_CELLS below)
-constexpr int fin_threads(int NP) { return NP >= 48 ? 512 : (NP >= 24 ? 256 : 64); }
+// threads per cell. Few cells: what counts is the latency of one cell, which the bulk sums to later
+// batches set, so many threads. Launches of FIN_BULK_CELLS cells or more (batches) fill every SM
+// several times over: fewer threads per cell then issue fewer idle lanes and barrier waits. Fill ms
+// at 128 / 256 / 384 / 512 / 768 threads: 128x32 2.82 / 2.50 / 2.46 / 2.47 / -, 128x64 - / 5.35 /
+// 4.94 / 4.81 / 4.74, 256x64 - / 18.97 / 18.33 / 18.11 / 18.72; the 512-pair batch 426-430 with the
+// smaller ones, 442 and 452 with 768 and 1024.
+constexpr int fin_threads(int NP) { return NP >= 48 ? 512 : (NP >= 24 ? 384 : 128); }
+constexpr int fin_bulk_threads(int NP) { return NP >= 48 ? 256 : 128; }
+constexpr int FIN_BULK_CELLS = 1024;
 // element (r, c) of tile (I2, J2) of an outer cell in the reference layout (tiles of T+1 rows, the
 // last one the halo; R = padding rows/columns of the first tile row/column); val(i2, j2) gives the
 // cell's inner value for 0 <= i2 <= j2 < N, the only entries read
@@ -272,17 +284,18 @@ struct RefOut {
     int T, Ns;
 };
 
-constexpr int FIN_BULK_THREADS = 256;  // widths >= 48, launches of FIN_BULK_CELLS cells or more
-constexpr int FIN_BULK_CELLS = 2048;
+constexpr int FIN_BATCH = 5;  // inner diagonals per batch: 1 + the largest span with S2 = 0, + 1
 
 template <int NP, int T = fin_threads(NP)>
 struct FinShape {
     static constexpr int THREADS = T;
     static constexpr int WARPS = THREADS / 32;
-    static constexpr int K = (NP * (NP - 1) / 2 + THREADS - 1) / THREADS;  // owned inner cells per thread
-    static constexpr int MINB = 1536 / THREADS;  // 48 resident warps per SM (at most 40 registers)
-    static_assert(K <= 8, "the step switch covers 8 slots");
-    static constexpr size_t SMEM = 2 * (size_t)NP * NP * sizeof(float) + NP;  // D, S2, bases
+    static constexpr int MINB = 1280 / THREADS;  // 40 resident warps per SM (48 registers)
+    // row pitch of D and of S2 by diagonals: entry (r, c) lies at (c-r)*LD + r, so rows r of a block
+    // column are LD-1 (odd) words apart and diagonals start on 8 bytes
+    static constexpr int LD = NP + 2;
+    static constexpr size_t SMEM = 2 * (size_t)NP * LD * sizeof(float) + NP;  // D, S2, bases
+    static_assert(WARPS >= 2 && NP <= 64, "one warp runs the batches, two rows per lane");
 };
 
 // first float of row e of a triangular diagonal-major table of width NP (row e holds NP - e entries)
@@ -303,15 +316,18 @@ finalize_small_kernel(const CellJob *__restrict__ jobs, int njobs, const CellJob
                       const uint8_t *__restrict__ bases, Weights W, int d, RefOut ro)
 {
     using Sh = FinShape<NP, T>;
-    constexpr int NB = NP / 8, NBLK = NB * (NB + 1) / 2, K = Sh::K;
+    constexpr int NB = NP / 8, NBLK = NB * (NB + 1) / 2;
     constexpr long long CELL = 4LL * R0_TAB_COLBASE[NB][NB];
     extern __shared__ __align__(16) float fsm[];
-    float *D = fsm, *S2s = fsm + NP * NP;
-    uint8_t *sb = reinterpret_cast<uint8_t *>(fsm + 2 * NP * NP);
+    constexpr int LD = Sh::LD;
+    float *D = fsm, *Sd = fsm + NP * LD;  // Sd[e][i] = S2(i, i+e)
+    uint8_t *sb = reinterpret_cast<uint8_t *>(fsm + 2 * NP * LD);
     __shared__ int cbs[NB];    // float offset of each block column in the cell image
     __shared__ float wsh[12];  // the weight table (indexed by pair type)
+    __shared__ float w5[25];   // intra-strand weight of bases a, b at 5a + b
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid < 12) wsh[tid] = W.w[tid];
+    if (tid >= 32 && tid < 57) w5[tid - 32] = score_w(W.w, (tid - 32) / 5, (tid - 32) % 5);
     if (tid < NB) cbs[tid] = 4 * c_img_colbase[NB][tid];
     __syncthreads();
     if ((int)blockIdx.x >= njobs) {  // S1 cells (i, i+d+1), one per warp
@@ -344,75 +360,90 @@ finalize_small_kernel(const CellJob *__restrict__ jobs, int njobs, const CellJob
     const uint8_t *s1 = bases + pd.seq1_off;
     const uint8_t *s2r = bases + pd.seq2_off;
     const float s1v = S1[i1 * M + j1];
-    for (int q4 = tid; q4 < NP * NP / 4; q4 += Sh::THREADS)
-        *reinterpret_cast<float4 *>(S2s + 4 * q4) = *reinterpret_cast<const float4 *>(S2 + 4 * q4);
     for (int q = tid; q < NP; q += Sh::THREADS) sb[q] = q < N ? s2r[q] : 4;
-    __syncthreads();
-    // start value of inner cell (r, c), r <= c: accumulated products, S1+S2, SW1
+    // start values (accumulated products, S1+S2, SW1; the inter-strand base on the diagonal of the
+    // diagonal cells) and S2, both by diagonals, 4 columns of one block row per step
     const bool sw1 = d >= 4;
     const float w1 = sw1 ? score_w(wsh, s1[i1], s1[j1]) : 0.0f;
-    const float *Fi = sw1 ? F + pd.F_off + cell_index(M, i1 + 1, j1 - 1) * CELL : nullptr;
-    auto start = [&](int r, int c) {
-        const int o = cbs[c >> 3] + 68 * (r >> 3) + 8 * (r & 7) + (c & 7);
-        const float v = fmaxf(Fc[o], s1v + S2s[r * NP + c]);
-        return sw1 ? fmaxf(v, Fi[o] + w1) : v;
-    };
-    // owned inner cells c = tid + THREADS*k among the N(N-1)/2 cells with e2 >= 1, ordered by
-    // (e2, i2): running maxima start at max(accumulated, S1+S2)
-    const int ncells = N * (N - 1) / 2;
-    int cell_i[K], cell_e[K];
-    float acc[K], sw2[K];  // running maximum; SW2 weight (-inf: no SW2 term)
+    const float *Fi = F + pd.F_off + (sw1 ? cell_index(M, i1 + 1, j1 - 1) * CELL : 0);
+    for (int q4 = tid; q4 < NBLK * 16; q4 += Sh::THREADS) {
+        int BI, BJ;
+        blk_decode(NB, q4 >> 4, BI, BJ);
+        const int r = 8 * BI + ((q4 & 15) >> 1), c0 = 8 * BJ + 4 * (q4 & 1), o = cbs[BJ] + 68 * BI + 4 * (q4 & 15);
+        const float4 f4 = *reinterpret_cast<const float4 *>(Fc + o), s4 = *reinterpret_cast<const float4 *>(S2 + r * NP + c0);
+        float4 p4 = make_float4(NEG_INF, NEG_INF, NEG_INF, NEG_INF);
+        if (sw1) p4 = *reinterpret_cast<const float4 *>(Fi + o);
+        const float fv[4] = {f4.x, f4.y, f4.z, f4.w}, sv[4] = {s4.x, s4.y, s4.z, s4.w}, pv[4] = {p4.x, p4.y, p4.z, p4.w};
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-        const int c = tid + Sh::THREADS * k;
-        cell_e[k] = NP;  // no cell: never open
-        cell_i[k] = 0;
-        acc[k] = NEG_INF;
-        sw2[k] = NEG_INF;
-        if (c < ncells) {
-            int e = 1, rem = c;
-            while (rem >= N - e) { rem -= N - e; ++e; }
-            cell_e[k] = e;
-            cell_i[k] = rem;
-            acc[k] = start(rem, rem + e);
-            if (e >= 4) sw2[k] = score_w(wsh, sb[rem], sb[rem + e]);
-        }
-    }
-    if (tid < N)  // inner diagonal 0
-        D[tid] = d == 0 ? score_w(wsh + 6, s1[i1], sb[tid]) : start(tid, tid);
-    __syncthreads();
-    // slot k of every thread holds cells THREADS*k .. THREADS*(k+1)-1 of the (e2, i2) order, so the
-    // slots whose cells are all final (e2 <= e) are the same for every thread: the step enters the
-    // unrolled slot sequence at the first slot still open (a CTA-uniform branch), instead of
-    // evaluating the closed slots under a false predicate
-    auto step = [&](auto kc, int e, const float *De) {
-        constexpr int k = decltype(kc)::value;
-        if constexpr (k < K) {
-            const int e2 = cell_e[k];
-            if (e2 > e && e2 < NP) {
-                const int i2 = cell_i[k], j2 = i2 + e2;
-                acc[k] = fmax3(acc[k], De[i2] + S2s[(i2 + e + 1) * NP + j2], S2s[i2 * NP + j2 - e - 1] + De[j2 - e]);
-                if (e2 == e + 1)  // all R1/R2 terms seen: SW2, then the cell is final
-                    D[e2 * NP + i2] = fmaxf(acc[k], D[max(e2 - 2, 0) * NP + i2 + 1] + sw2[k]);
+        for (int t = 0; t < 4; ++t) {
+            const int c = c0 + t;
+            if (r <= c && c < N) {
+                D[(c - r) * LD + r] = d == 0 && r == c ? score_w(wsh + 6, s1[i1], s2r[r])
+                                                       : fmax3(fv[t], s1v + sv[t], pv[t] + w1);
+                Sd[(c - r) * LD + r] = sv[t];
             }
         }
+    }
+    __syncthreads();
+    // the first warp's state: rows 2*lane and 2*lane+1 of the last two diagonals (p of e-1, q of e-2),
+    // and row 2*lane+2 of each
+    const int i0 = 2 * lane;
+    float p0 = 0.0f, p1 = 0.0f, q1 = 0.0f, q2 = 0.0f;
+    const int b0 = 5 * sb[min(i0, NP - 1)], b1 = 5 * sb[min(i0 + 1, NP - 1)];
+    auto run_batch = [&](int e0) {
+        float2 a[FIN_BATCH];
+        float wa[FIN_BATCH], wb[FIN_BATCH];
+#pragma unroll
+        for (int s = 0; s < FIN_BATCH; ++s) {
+            const int e = min(e0 + s, NP - 1);
+            a[s] = *reinterpret_cast<const float2 *>(D + e * LD + min(i0, NP - 2));
+            wa[s] = e >= 4 ? w5[b0 + sb[min(i0 + e, NP - 1)]] : NEG_INF;
+            wb[s] = e >= 4 ? w5[b1 + sb[min(i0 + 1 + e, NP - 1)]] : NEG_INF;
+        }
+#pragma unroll
+        for (int s = 0; s < FIN_BATCH; ++s) {
+            const int e = e0 + s;
+            if (e >= N) break;
+            float n0 = a[s].x, n1 = a[s].y;
+            const float p2 = __shfl_down_sync(0xffffffffu, p0, 1);
+            if (e > 0) {
+                n0 = fmaxf(fmax3(n0, p0, p1), q1 + wa[s]);
+                n1 = fmaxf(fmax3(n1, p1, p2), q2 + wb[s]);
+                if (i0 < NP) *reinterpret_cast<float2 *>(D + e * LD + i0) = make_float2(n0, n1);
+            }
+            q1 = p1;
+            q2 = p2;
+            p0 = n0;
+            p1 = n1;
+        }
     };
-    for (int e = 0; e + 1 < N; ++e) {
-        const float *De = D + e * NP;
-        const int first = (e * N - e * (e + 1) / 2) / Sh::THREADS;  // cells with e2 <= e come first
-        switch (first) {
-        case 0: step(std::integral_constant<int, 0>{}, e, De); [[fallthrough]];
-        case 1: step(std::integral_constant<int, 1>{}, e, De); [[fallthrough]];
-        case 2: step(std::integral_constant<int, 2>{}, e, De); [[fallthrough]];
-        case 3: step(std::integral_constant<int, 3>{}, e, De); [[fallthrough]];
-        case 4: step(std::integral_constant<int, 4>{}, e, De); [[fallthrough]];
-        case 5: step(std::integral_constant<int, 5>{}, e, De); [[fallthrough]];
-        case 6: step(std::integral_constant<int, 6>{}, e, De); [[fallthrough]];
-        case 7: step(std::integral_constant<int, 7>{}, e, De); [[fallthrough]];
-        default: break;
+    // candidates of the final diagonals e0 .. e0+4 for entry i of diagonal e2, those with e <= e2-5
+    auto push = [&](int e0, int e2, int i, int n) {
+        const float *De = D + e0 * LD + i, *Dj = De + (e2 - e0);              // F[i][i+e], F[j-e][j]
+        const float *Sj = Sd + (e2 - e0 - 1) * LD + i, *Se = Sj + e0 + 1;     // S2(i, j-e-1), S2(i+e+1, j)
+        float v = D[e2 * LD + i];
+#pragma unroll
+        for (int t = 0; t < FIN_BATCH; ++t)
+            if (t < n) v = fmax3(v, De[t * LD] + Se[-t * (LD - 1)], Sj[-t * LD] + Dj[t * (LD - 1)]);
+        D[e2 * LD + i] = v;
+    };
+    if (warp == 0) run_batch(0);
+    for (int e0 = 0; e0 + FIN_BATCH < N; e0 += FIN_BATCH) {  // diagonals e0 .. e0+4 are final
+        const int e1 = e0 + FIN_BATCH;
+        __syncthreads();
+        for (int u = warp; u < FIN_BATCH * ((NP + 31) / 32); u += Sh::WARPS) {  // to the next batch
+            const int s = FIN_BATCH - 1 - u % FIN_BATCH, i = lane + 32 * (u / FIN_BATCH);
+            if (i < N - (e1 + s)) push(e0, e1 + s, i, s + 1);
         }
         __syncthreads();
+        if (warp == 0) {
+            run_batch(e1);
+        } else {
+            for (int e2 = e1 + FIN_BATCH + warp - 1; e2 < N; e2 += Sh::WARPS - 1)
+                for (int i = lane; i < N - e2; i += 32) push(e0, e2, i, FIN_BATCH);
+        }
     }
+    __syncthreads();
     // write-back, 4 columns of one block row per step
     for (int q4 = tid; q4 < NBLK * 16; q4 += Sh::THREADS) {
         int BI, BJ;
@@ -422,7 +453,7 @@ finalize_small_kernel(const CellJob *__restrict__ jobs, int njobs, const CellJob
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
             const int c = c0 + t;
-            v[t] = r <= c && c < N ? D[(c - r) * NP + r] : (r == c + 1 ? s1v : NEG_INF);  // S1 on the subdiagonal
+            v[t] = r <= c && c < N ? D[(c - r) * LD + r] : (r == c + 1 ? s1v : NEG_INF);  // S1 on the subdiagonal
         }
         // block (BI, BJ), row r & 7, half
         *reinterpret_cast<float4 *>(Fc + cbs[BJ] + 68 * BI + 4 * (q4 & 15)) = make_float4(v[0], v[1], v[2], v[3]);
@@ -437,7 +468,7 @@ finalize_small_kernel(const CellJob *__restrict__ jobs, int njobs, const CellJob
                    // values the image holds), one warp per tile row of T floats
         const int TT = ro.T, R = (TT - N % TT) % TT, tile_rows = TT + 1, rows = ro.Ns * ro.Ns * tile_rows;
         float *dst = ro.out + ((long long)d * M - (long long)d * (d - 1) / 2 + i1) * ((long long)rows * TT);
-        auto dval = [&](int i2, int j2) { return D[(j2 - i2) * NP + i2]; };
+        auto dval = [&](int i2, int j2) { return D[(j2 - i2) * LD + i2]; };
         for (int rr = warp; rr < rows; rr += Sh::WARPS) {
             const int I2 = rr / (ro.Ns * tile_rows), rem = rr % (ro.Ns * tile_rows);
             const int J2 = rem / tile_rows, r = rem % tile_rows;

@@ -1,0 +1,44 @@
+"""The finalize of tables up to width 64 bit for bit against the oracle: strand-2 lengths around its
+batches of five inner diagonals, around the 32 lanes of a warp and at the ends of every width class,
+and launches of enough cells for the form with fewer threads per cell."""
+import numpy as np
+import pytest
+
+from bpmax_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def eng():
+    from bpmax_b200 import Engine
+
+    e = Engine(0)
+    yield e
+    e.close()
+
+
+def bits(a):
+    return np.ascontiguousarray(a, dtype=np.float32).view(np.uint32)
+
+
+@pytest.mark.parametrize("N", [1, 2, 4, 5, 6, 8, 9, 10, 11, 15, 16, 17, 20, 21, 25, 26, 31, 32, 33, 34, 40, 47, 51, 56, 61, 63, 64])
+def test_batches_vs_oracle(eng, oracle_mod, N):
+    M = 7  # SW1 starts at outer diagonal 4
+    s1, s2 = W.pair(M, N, 2000 + N)
+    for w in (W.INTEGER_WEIGHTS, W.random_weights(N)):
+        eng.set_weights(w)
+        F, score = eng.fill_compact(s1, s2)
+        Fo, _, _ = oracle_mod.fill(s1, s2, w)
+        assert np.array_equal(bits(F), bits(Fo))
+        assert score == oracle_mod.score(Fo, M, N)
+
+
+@pytest.mark.parametrize("N", [8, 16, 24, 40, 48, 64])
+def test_bulk_launches_vs_oracle(eng, oracle_mod, N):
+    rng = np.random.default_rng(N)
+    pairs = [(W.random_sequence(8, rng), W.random_sequence(N - p % 3, rng)) for p in range(160)]
+    eng.set_weights(W.REFERENCE_WEIGHTS)
+    got = eng.score_batch(pairs)
+    exp = [oracle_mod.score(oracle_mod.fill(a, b, W.REFERENCE_WEIGHTS)[0], len(a), len(b)) for a, b in pairs]
+    assert np.array_equal(bits(got), bits(np.array(exp, dtype=np.float32)))
