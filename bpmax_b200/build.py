@@ -15,8 +15,8 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libbpmax_gpu.so")
 
 SOURCES = ["bpmax_engine.cu", "bpmax_shim.cpp"]
-HEADERS = ["bpmax_kernels.cuh", "bpmax_kernels_large.cuh", "bpmax_r0.cuh", "bpmax_adjoint.cuh", "bpmax_r0only.cuh",
-           "bpmax_wide.cuh", "bpmax_persist.cuh", "bpmax_strip.cuh", "r0_tables.inc", "wide_tables.inc"]
+HEADERS = ["bpmax_kernels.cuh", "bpmax_r0.cuh", "bpmax_adjoint.cuh", "bpmax_r0only.cuh",
+           "bpmax_wide.cuh", "bpmax_persist.cuh", "bpmax_strip.cuh", "bpmax_tile.cuh", "r0_tables.inc", "wide_tables.inc"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-O3", "-lineinfo", "-std=c++17",

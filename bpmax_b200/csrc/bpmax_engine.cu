@@ -7,7 +7,7 @@
 //     R0+R3+R4 product kernel over the cells (i1, i1+d) of every pair with M > d: jobs of k1
 //       offset pairs (w, d-1-w), ordered by offset pair so both uses of a table meet in L2; from a
 //       certain size on, the strip kernel takes most offsets of several diagonals in one launch;
-//     finalize kernel over the same cells (init, SW1, inner R1/R2/SW2 wavefront, FT copy).
+//     finalize kernel over the same cells (init, SW1, inner R1/R2/SW2 wavefront).
 // The whole sequence is captured once per shape as a CUDA graph and replayed.
 #include <cuda_runtime.h>
 
@@ -25,13 +25,13 @@
 
 #include "../../include/bpmax_gpu.h"
 #include "bpmax_kernels.cuh"
-#include "bpmax_kernels_large.cuh"
 #include "bpmax_r0.cuh"
 #include "bpmax_adjoint.cuh"
 #include "bpmax_r0only.cuh"
 #include "bpmax_wide.cuh"
 #include "bpmax_persist.cuh"
 #include "bpmax_strip.cuh"
+#include "bpmax_tile.cuh"
 
 using namespace bpmax;
 
@@ -95,7 +95,6 @@ struct Plan {
     std::vector<int> Ms, Ns;
     std::vector<PairDesc> pairs;
     long long F_floats = 0, S_floats = 0;
-    bool any_large = false;  // some pair has Np > WIDE_TILE_MAX_NP (row-major tables + FT)
     int bases_bytes = 0;
     int maxM = 0;
     // per diagonal and Np class (index NB-1): ranges in the job arrays
@@ -105,7 +104,6 @@ struct Plan {
     std::vector<Launch> r0_launches, fin_launches;
     std::vector<R0Job> r0_jobs;
     std::vector<StripJob> strip_jobs;  // jobs of strip launches (first/count index this array)
-    std::vector<R0JobL> r0l_jobs;  // jobs of launches with np > WIDE_TILE_MAX_NP (first/count index this array)
     std::vector<R0JobW> r0w_jobs;  // jobs of launches with tile-image tables (first/count index this array)
     std::vector<CellJob> cell_jobs;
     std::vector<int> classes;  // distinct inner widths, ascending
@@ -139,7 +137,7 @@ struct bpmax_ctx {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     Weights W;
     std::string err;
-    DevBuf F, FT, S, bases, pairs, r0jobs, stripjobs, r0ljobs, r0wjobs, celljobs, scores, conv, tbstack, grads, tbstatus, errflag;
+    DevBuf F, S, bases, pairs, r0jobs, stripjobs, r0wjobs, celljobs, scores, conv, tbstack, grads, tbstatus, errflag;
     DevBuf r0vals;         // R0-only mode: seq1 then seq2 of the pair, as floats
     DevBuf pq, pcnt, pneed;  // persistent fill: work queue; counters (class heads, diagonals, cells); jobs per cell
     bool copyout = false;    // the next fill copies the reference layout out per diagonal (graph path)
@@ -354,17 +352,16 @@ int build_plan(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int
         if (pd.Np > MAX_NP) return fail(ctx, BPMAX_EINVAL, "strand-2 length %d > %d is not supported", Ns[p], MAX_NP);
         pd.F_off = f;
         f = align64(f + (long long)Ms[p] * (Ms[p] + 1) / 2 * cell_floats(pd.Np));
-        if (pd.Np > WIDE_TILE_MAX_NP) P.any_large = true;
         pd.S1_off = s;
         s = align64(s + (long long)Ms[p] * Ms[p]);
         pd.S2_off = s;
         s = align64(s + (long long)pd.Np * pd.Np);
-        pd.S2m_off = s;  // masked copies of S2 read by the inner wavefront
-        s = align64(s + (long long)pd.Np * pd.Np);
-        pd.S2t_off = s;
-        s = align64(s + (long long)pd.Np * pd.Np);
-        pd.S2d_off = s;
-        if (pd.Np > MAX_SMALL_NP) s = align64(s + (long long)pd.Np * (pd.Np + 1) / 2);  // triangular S2D
+        if (pd.Np > MAX_SMALL_NP) {  // copies of S2 read by the tile finalize
+            pd.S2x_off = s;
+            s = align64(s + (long long)pd.Np * pd.Np);
+            pd.S2y_off = s;
+            s = align64(s + (long long)pd.Np * pd.Np);
+        }
         pd.seq1_off = b;
         b += Ms[p];
         pd.seq2_off = b;
@@ -404,7 +401,6 @@ int build_plan(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int
         return it == share.end() ? resident : std::max(1LL, (long long)std::llround(resident * it->second));
     };
     // jobs, grouped by diagonal then inner width class
-    const int target = 4 * ctx->sms;  // CTAs per diagonal launch worth splitting k1 for (wide tables)
     for (int d = 0; d < P.maxM; ++d) {
         for (int np : classes) {
             long long cells = 0;
@@ -474,58 +470,38 @@ int build_plan(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int
                 P.r0_launches.push_back(rl);
                 continue;
             }
-            if (np <= WIDE_TILE_MAX_NP) {
-                // tile images: one job per output tile (BI, BJ) of a cell and chunk of k1 offset pairs,
-                // each tile's chunk sized so that jobs cost about the same: cost per offset pair in
-                // warp task steps of both of its items, DD 3.3, DA and DB 12, F 16 per item
-                const int NT = np / 64;
-                const long long P2 = (d + 1) / 2;
-                const long long resident = capped(np, (long long)std::max(1, ctx->wide_occ[P.wide_stages]) * ctx->sms);
-                std::vector<std::pair<double, int>> tiles;  // (cost per offset pair, BI << 8 | BJ)
-                double per_pair = 0;
-                for (int BI = 0; BI < NT; ++BI)
-                    for (int BJ = BI; BJ < NT; ++BJ) {
-                        const double c = BI == BJ ? 2 * 3.3 : 2 * (24.0 + 16.0 * (BJ - BI - 1));
-                        tiles.push_back({c, BI << 8 | BJ});
-                        per_pair += c;
-                    }
-                std::stable_sort(tiles.begin(), tiles.end(), [](const auto &a, const auto &b) { return a.first > b.first; });
-                const double total = (double)cells * P2 * per_pair;
-                const double target = std::max(total / (3.0 * resident), 4.0 * 16.0);
-                const size_t first = P.r0w_jobs.size();
-                for (const auto &t : tiles) {
-                    const long long q = std::max(1LL, std::min(P2, (long long)std::llround(target / t.first)));
-                    for (long long c0 = 0; c0 < P2; c0 += q)
-                        for (int p = 0; p < n; ++p)
-                            if (P.pairs[p].Np == np && Ms[p] > d)
-                                for (int i1 = 0; i1 < Ms[p] - d; ++i1)
-                                    P.r0w_jobs.push_back(R0JobW{p, i1, t.second, (int)c0, (int)std::min(c0 + q, P2)});
+            // tile images: one job per output tile (BI, BJ) of a cell and chunk of k1 offset pairs,
+            // each tile's chunk sized so that jobs cost about the same: cost per offset pair in
+            // warp task steps of both of its items, DD 3.3, DA and DB 12, F 16 per item
+            const int NT = np / 64;
+            const long long P2 = (d + 1) / 2;
+            const long long resident = capped(np, (long long)std::max(1, ctx->wide_occ[P.wide_stages]) * ctx->sms);
+            std::vector<std::pair<double, int>> tiles;  // (cost per offset pair, BI << 8 | BJ)
+            double per_pair = 0;
+            for (int BI = 0; BI < NT; ++BI)
+                for (int BJ = BI; BJ < NT; ++BJ) {
+                    const double c = BI == BJ ? 2 * 3.3 : 2 * (24.0 + 16.0 * (BJ - BI - 1));
+                    tiles.push_back({c, BI << 8 | BJ});
+                    per_pair += c;
                 }
-                // jobs of the same offset pairs together (both uses of a table meet in L2), heavy tiles first
-                std::stable_sort(P.r0w_jobs.begin() + first, P.r0w_jobs.end(),
-                                 [](const R0JobW &a, const R0JobW &b) { return a.p0 < b.p0; });
-                Plan::Launch wl{d, np, (int)first, (int)(P.r0w_jobs.size() - first)};
-                wl.cap = share.empty() ? 0 : (int)resident;
-                P.r0_launches.push_back(wl);
-                continue;
+            std::stable_sort(tiles.begin(), tiles.end(), [](const auto &a, const auto &b) { return a.first > b.first; });
+            const double total = (double)cells * P2 * per_pair;
+            const double target = std::max(total / (3.0 * resident), 4.0 * 16.0);
+            const size_t first = P.r0w_jobs.size();
+            for (const auto &t : tiles) {
+                const long long q = std::max(1LL, std::min(P2, (long long)std::llround(target / t.first)));
+                for (long long c0 = 0; c0 < P2; c0 += q)
+                    for (int p = 0; p < n; ++p)
+                        if (P.pairs[p].Np == np && Ms[p] > d)
+                            for (int i1 = 0; i1 < Ms[p] - d; ++i1)
+                                P.r0w_jobs.push_back(R0JobW{p, i1, t.second, (int)c0, (int)std::min(c0 + q, P2)});
             }
-            const int nbk = np / 64;
-            const long long units = cells * (nbk * (nbk + 1) / 2);
-            long long chunks = std::max(1LL, std::min((long long)d, (target + units - 1) / units));
-            int csize = (int)((d + chunks - 1) / chunks);
-            Plan::Launch rl{d, np, (int)P.r0l_jobs.size(), 0};
-            for (int p = 0; p < n; ++p)
-                if (P.pairs[p].Np == np && Ms[p] > d)
-                    for (int i1 = 0; i1 < Ms[p] - d; ++i1)
-                        for (int k = i1; k < i1 + d; k += csize) {
-                            const int kb = std::min(k + csize, i1 + d);
-                            // heavier blocks (more k' blocks) first
-                            for (int D = nbk - 1; D >= 0; --D)
-                                for (int BI = 0; BI + D < nbk; ++BI)
-                                    P.r0l_jobs.push_back(R0JobL{p, i1, k, kb, (BI << 16) | (BI + D)});
-                        }
-            rl.count = (int)P.r0l_jobs.size() - rl.first;
-            P.r0_launches.push_back(rl);
+            // jobs of the same offset pairs together (both uses of a table meet in L2), heavy tiles first
+            std::stable_sort(P.r0w_jobs.begin() + first, P.r0w_jobs.end(),
+                             [](const R0JobW &a, const R0JobW &b) { return a.p0 < b.p0; });
+            Plan::Launch wl{d, np, (int)first, (int)(P.r0w_jobs.size() - first)};
+            wl.cap = share.empty() ? 0 : (int)resident;
+            P.r0_launches.push_back(wl);
         }
     }
     // S1 of diagonal d+1 is computed by the finalize launch of diagonal d (same class)
@@ -538,14 +514,6 @@ int build_plan(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int
     P.persistent = P.persist && !ctx->r0_only && !ctx->copyout && P.classes.back() <= MAX_SMALL_NP;
     if (P.persistent) build_queue(ctx, P);
     return BPMAX_OK;
-}
-
-void launch_r0_large(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
-{
-    const int grid = std::min(L.count, 3 * ctx->sms);
-    r0_large_kernel<<<grid, 128, WideShape::SMEM, s>>>(
-        (const R0JobL *)ctx->r0ljobs.p + L.first, L.count, (const PairDesc *)ctx->pairs.p, (float *)ctx->F.p,
-        (const float *)ctx->FT.p, (const float *)ctx->S.p, L.d);
 }
 
 template <int STAGES>
@@ -565,43 +533,31 @@ void launch_r0_wide(bpmax_ctx *ctx, const Plan &P, const Plan::Launch &L, cudaSt
         launch_r0_wide_t<2>(ctx, L, s);
 }
 
-// the finalize of one launch of cells wider than 64; returns the number of kernel launches
-int launch_fin_large(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
+// the finalize of one launch of cells wider than 64: one launch per tile diagonal t, with the slabs of
+// its tiles in a launch of their own where few tiles hold many; returns the number of kernel launches
+int launch_fin_tiles(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
 {
     const CellJob *jobs = (const CellJob *)ctx->celljobs.p + L.first;
     const CellJob *s1jobs = (const CellJob *)ctx->celljobs.p + L.s1_first;
     const PairDesc *pairs = (const PairDesc *)ctx->pairs.p;
-    const uint8_t *bases = (const uint8_t *)ctx->bases.p;
     float *F = (float *)ctx->F.p, *S = (float *)ctx->S.p;
-    if (L.np <= FIN_WIDE_MAX_NP) {
-        constexpr int WW = FIN_WIDE_THREADS / 32;
-        finalize_wide_kernel<<<L.count + (L.s1_count + WW - 1) / WW, FIN_WIDE_THREADS, fin_wide_smem(L.np), s>>>(
-            jobs, L.count, s1jobs, L.s1_count, pairs, F, S, bases, ctx->W, L.d);
-        return 1;
-    }
-    // row-major tables: start values, then per tile diagonal t the products over finished tiles and
-    // the tiles' own wavefronts, then the SW1 pushes, the S1 slots and S1 of diagonal d+1
-    float *FT = (float *)ctx->FT.p;
-    const int nt32 = L.np / 32, NT = L.np / LT;
+    const int NT = L.np / 64;
     int n = 0;
-    if (L.count > 0) {
-        large_init_kernel<<<dim3(nt32 * nt32, L.count), dim3(32, 8), 0, s>>>(jobs, pairs, F, FT, S, bases, ctx->W, L.d);
-        ++n;
-        for (int t = 0; t < NT; ++t) {
-            if (t > 0) {
-                large_tile_product_kernel<<<dim3(NT - t, L.count), 256, 0, s>>>(jobs, pairs, F, FT, S, L.d, t);
-                ++n;
-            }
-            large_tile_local_kernel<<<dim3(NT - t, L.count), 256, LARGE_LOCAL_SMEM, s>>>(jobs, pairs, F, FT, S, bases,
-                                                                                         ctx->W, L.d, t);
+    for (int t = 0; t < NT; ++t) {
+        const int tiles = L.count * (NT - t), slabs = 2 * t;
+        const int parts = tiles < ctx->sms ? std::min(slabs, (2 * ctx->sms + tiles - 1) / tiles) : 1;
+        const bool split = parts > 1;
+        if (split) {
+            tile_product_kernel<<<dim3(tiles, parts), TILE_THREADS, TILE_SMEM, s>>>(jobs, pairs, F, S, L.d, t, NT);
             ++n;
         }
+        const int s1_ctas = t == 0 ? (L.s1_count + TILE_THREADS / 32 - 1) / (TILE_THREADS / 32) : 0;
+        tile_final_kernel<<<tiles + s1_ctas, TILE_THREADS, TILE_SMEM, s>>>(jobs, L.count, s1jobs, L.s1_count, pairs, F, S,
+                                                                           (const uint8_t *)ctx->bases.p, ctx->W, L.d, t,
+                                                                           NT, !split);
+        ++n;
     }
-    const long long tile = (long long)L.np * L.np;
-    const int chunks = (int)((tile + LARGE_FINAL_CHUNK - 1) / LARGE_FINAL_CHUNK);
-    large_final_kernel<<<L.count * chunks + (L.s1_count + 7) / 8, 256, 0, s>>>(jobs, L.count, chunks, s1jobs, L.s1_count,
-                                                                             pairs, F, FT, S, bases, ctx->W, L.d);
-    return n + 1;
+    return n;
 }
 
 template <int NB, int V>
@@ -666,11 +622,7 @@ void launch_r0only_fin(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
     const float *vals = (const float *)ctx->r0vals.p;
     switch (L.np > MAX_SMALL_NP ? 0 : L.np / 8) {
     case 0:
-        if (L.np <= WIDE_TILE_MAX_NP)
-            r0only_finalize_tile_kernel<<<L.count, 256, 0, s>>>(jobs, pd, (float *)ctx->F.p, vals, L.d);
-        else
-            r0only_finalize_wide_kernel<<<dim3(L.count, L.np / R0ONLY_TILE), 256, 0, s>>>(jobs, pd, (float *)ctx->F.p,
-                                                                                         (float *)ctx->FT.p, vals, L.d);
+        r0only_finalize_tile_kernel<<<dim3(L.count, L.np / 64), 256, 0, s>>>(jobs, pd, (float *)ctx->F.p, vals, L.d);
         break;
     case 1: r0only_finalize_small_kernel<8><<<L.count, 128, 0, s>>>(jobs, pd, (float *)ctx->F.p, vals, L.d); break;
     case 2: r0only_finalize_small_kernel<16><<<L.count, 128, 0, s>>>(jobs, pd, (float *)ctx->F.p, vals, L.d); break;
@@ -708,10 +660,8 @@ int set_smem_attr(bpmax_ctx *ctx)
     }
     if (NB == 8)
         if ((st = prefer_smem(ctx, r0_wide_kernel<2>)) || (st = prefer_smem(ctx, r0_wide_kernel<3>)) ||
-            (st = prefer_smem(ctx, r0_large_kernel)))
+            (st = prefer_smem(ctx, tile_product_kernel)) || (st = prefer_smem(ctx, tile_final_kernel)))
             return st;
-    // (the wide finalize kernels keep the driver's choice: their S2 reads live on the L1 that a
-    // larger shared-memory carveout would take away, 389 vs 324 ms at 256x256)
     CK(cudaFuncSetAttribute(r0_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)R0Cfg<NB>::SMEM));
     CK(cudaFuncSetAttribute(r0_kernel<NB, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)R0Cfg<NB, 1>::SMEM));
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctx->r0_occ_v[1][NB], r0_kernel<NB, 1>, R0Cfg<NB, 1>::THREADS,
@@ -732,11 +682,8 @@ int set_smem_attr(bpmax_ctx *ctx)
         CK(cudaFuncSetAttribute(r0_wide_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WideCfg<3>::SMEM));
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctx->wide_occ[2], r0_wide_kernel<2>, 128, WideCfg<2>::SMEM));
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctx->wide_occ[3], r0_wide_kernel<3>, 128, WideCfg<3>::SMEM));
-        CK(cudaFuncSetAttribute(r0_large_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WideShape::SMEM));
-        CK(cudaFuncSetAttribute(finalize_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)fin_wide_smem(FIN_WIDE_MAX_NP)));
-        CK(cudaFuncSetAttribute(large_tile_local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)LARGE_LOCAL_SMEM));
+        CK(cudaFuncSetAttribute(tile_product_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TILE_SMEM));
+        CK(cudaFuncSetAttribute(tile_final_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TILE_SMEM));
     }
     return BPMAX_OK;
 }
@@ -776,21 +723,21 @@ int enqueue_fill(bpmax_ctx *ctx, Plan &P, KernelProfile *kp = nullptr)
     CK(cudaMemsetAsync(ctx->F.p, 0, (size_t)P.F_floats * sizeof(float), ctx->stream));
     CK(cudaMemsetAsync(ctx->S.p, 0, (size_t)P.S_floats * sizeof(float), ctx->stream));  // S1 starts at 0
     CK(cudaMemsetAsync(ctx->errflag.p, 0, sizeof(int), ctx->stream));
-    if (P.r0_only) {
-        ProfScope ps(ctx, kp, 0);
-        r0only_prep_kernel<<<(int)P.pairs.size(), 256, 0, ctx->stream>>>((const PairDesc *)ctx->pairs.p, (float *)ctx->S.p);
-        launches += 1;
-    } else {
+    if (!P.r0_only) {
         ProfScope ps(ctx, kp, 0);
         single_strand_kernel<<<(int)P.pairs.size(), 512, 0, ctx->stream>>>(
             (const PairDesc *)ctx->pairs.p, (const uint8_t *)ctx->bases.p, (float *)ctx->S.p, ctx->W);
         for (int p = 0; p < (int)P.pairs.size(); ++p)  // wider tables: one launch per diagonal of S2
-            if (P.pairs[p].Np > WIDE_TILE_MAX_NP)
+            if (P.pairs[p].Np > S2_ONE_CTA_NP)
                 for (int d = 4; d < P.pairs[p].N; ++d, ++launches)
                     s2_diag_kernel<<<(P.pairs[p].N - d + 7) / 8, 256, 0, ctx->stream>>>(
                         (const PairDesc *)ctx->pairs.p, p, (const uint8_t *)ctx->bases.p, (float *)ctx->S.p, ctx->W, d);
-        s2_aux_kernel<<<(int)P.pairs.size(), 256, 0, ctx->stream>>>((const PairDesc *)ctx->pairs.p, (float *)ctx->S.p);
-        launches += 2;
+        launches += 1;
+        if (P.classes.back() > MAX_SMALL_NP) {
+            s2_aux_kernel<<<dim3(64, (int)P.pairs.size()), 256, 0, ctx->stream>>>((const PairDesc *)ctx->pairs.p,
+                                                                                 (float *)ctx->S.p);
+            launches += 1;
+        }
     }
     const bool prof = kp && kp->on;
     if (P.persistent) {  // one persistent launch per width class: side by side on the class streams, or in turn
@@ -855,12 +802,7 @@ int enqueue_fill(bpmax_ctx *ctx, Plan &P, KernelProfile *kp = nullptr)
             {
                 ProfScope ps(ctx, kp, 1);
                 switch (L.np > MAX_SMALL_NP ? 0 : L.np / 8) {
-                case 0:
-                    if (L.np <= WIDE_TILE_MAX_NP)
-                        launch_r0_wide(ctx, P, L, st);
-                    else
-                        launch_r0_large(ctx, L, st);
-                    break;
+                case 0: launch_r0_wide(ctx, P, L, st); break;
                 case 1: launch_r0<1>(ctx, P, L, st); break;
                 case 2: launch_r0<2>(ctx, P, L, st); break;
                 case 3: launch_r0<3>(ctx, P, L, st); break;
@@ -881,7 +823,7 @@ int enqueue_fill(bpmax_ctx *ctx, Plan &P, KernelProfile *kp = nullptr)
                     launch_r0only_fin(ctx, L, st);
                 } else {
                     switch (L.np > MAX_SMALL_NP ? 0 : L.np / 8) {
-                    case 0: launches += launch_fin_large(ctx, L, st) - 1; break;
+                    case 0: launches += launch_fin_tiles(ctx, L, st) - 1; break;
                     case 1: launch_fin<1>(ctx, L, st); break;
                     case 2: launch_fin<2>(ctx, L, st); break;
                     case 3: launch_fin<3>(ctx, L, st); break;
@@ -940,14 +882,12 @@ int prepare(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int> &
             for (auto &e : P.diag_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         }
         if ((st = ensure(ctx, ctx->F, P.F_floats * sizeof(float))) != BPMAX_OK) return st;
-        if (P.any_large && (st = ensure(ctx, ctx->FT, P.F_floats * sizeof(float))) != BPMAX_OK) return st;
         if ((st = ensure(ctx, ctx->errflag, sizeof(int))) != BPMAX_OK) return st;
         if ((st = ensure(ctx, ctx->S, P.S_floats * sizeof(float))) != BPMAX_OK) return st;
         if ((st = ensure(ctx, ctx->bases, P.bases_bytes + 16)) != BPMAX_OK) return st;
         if ((st = ensure(ctx, ctx->pairs, P.pairs.size() * sizeof(PairDesc))) != BPMAX_OK) return st;
         if ((st = ensure(ctx, ctx->r0jobs, P.r0_jobs.size() * sizeof(R0Job))) != BPMAX_OK) return st;
         if ((st = ensure(ctx, ctx->stripjobs, P.strip_jobs.size() * sizeof(StripJob))) != BPMAX_OK) return st;
-        if ((st = ensure(ctx, ctx->r0ljobs, P.r0l_jobs.size() * sizeof(R0JobL))) != BPMAX_OK) return st;
         if ((st = ensure(ctx, ctx->r0wjobs, P.r0w_jobs.size() * sizeof(R0JobW))) != BPMAX_OK) return st;
         if (P.persistent) {
             if ((st = ensure(ctx, ctx->pq, P.pitems.size() * sizeof(PItem))) != BPMAX_OK) return st;
@@ -969,9 +909,6 @@ int prepare(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int> &
                                cudaMemcpyHostToDevice, ctx->stream));
         if (!P.r0w_jobs.empty())
             CK(cudaMemcpyAsync(ctx->r0wjobs.p, P.r0w_jobs.data(), P.r0w_jobs.size() * sizeof(R0JobW), cudaMemcpyHostToDevice,
-                               ctx->stream));
-        if (!P.r0l_jobs.empty())
-            CK(cudaMemcpyAsync(ctx->r0ljobs.p, P.r0l_jobs.data(), P.r0l_jobs.size() * sizeof(R0JobL), cudaMemcpyHostToDevice,
                                ctx->stream));
         CK(cudaMemcpyAsync(ctx->celljobs.p, P.cell_jobs.data(), P.cell_jobs.size() * sizeof(CellJob), cudaMemcpyHostToDevice, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
@@ -1189,8 +1126,8 @@ void bpmax_gpu_destroy(bpmax_ctx *ctx)
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     if (ctx->plan.graph) cudaGraphExecDestroy(ctx->plan.graph);
-    for (DevBuf *b : {&ctx->tbstack, &ctx->grads, &ctx->tbstatus, &ctx->F, &ctx->FT, &ctx->S, &ctx->bases, &ctx->pairs,
-                      &ctx->r0jobs, &ctx->stripjobs, &ctx->r0ljobs, &ctx->r0wjobs, &ctx->pq, &ctx->pcnt, &ctx->pneed, &ctx->celljobs,
+    for (DevBuf *b : {&ctx->tbstack, &ctx->grads, &ctx->tbstatus, &ctx->F, &ctx->S, &ctx->bases, &ctx->pairs,
+                      &ctx->r0jobs, &ctx->stripjobs, &ctx->r0wjobs, &ctx->pq, &ctx->pcnt, &ctx->pneed, &ctx->celljobs,
                       &ctx->scores, &ctx->conv, &ctx->refdev, &ctx->errflag,
                       &ctx->r0vals})
         if (b->p) cudaFree(b->p);
@@ -1702,8 +1639,8 @@ int bpmax_gpu_last_timing(const bpmax_ctx *ctx, float *fill_ms, long *launches)
 // Some callers cannot allocate device memory: code that runs inside another framework's
 // memory pool or under a fixed device-memory budget (where a raw cudaMalloc is forbidden or
 // would exceed the budget), and latency-sensitive callers that must not risk the implicit
-// device synchronisation cudaMalloc/cudaFree can cause. For them the fill's scratch (the F and
-// FT tables, S1/S2, the sequences and the job lists) lives in one fixed file-scope device array
+// device synchronisation cudaMalloc/cudaFree can cause. For them the fill's scratch (the F
+// tables, S1/S2, the sequences and the job lists) lives in one fixed file-scope device array
 // instead of the context's arenas. Every GPU that loads this library holds that array until
 // the process exits.
 // =========================================================================================
@@ -1820,8 +1757,8 @@ extern "C" int bpmax_gpu_score_noalloc(const int *seq1, long M, const int *seq2,
     const long long nF = (long long)M * (M + 1) / 2 * cell_floats(Np);
     const long long off_S = align64(nF);
     const long long S2_rel = align64((long long)M * M);
-    const long long S2m_rel = S2_rel + align64((long long)Np * Np), S2t_rel = S2m_rel + align64((long long)Np * Np);
-    const long long off_seq = off_S + S2t_rel + align64((long long)Np * Np);
+    // (S2 and as much again twice: the documented size limits count it)
+    const long long off_seq = off_S + S2_rel + 3 * align64((long long)Np * Np);
     const long long off_bases = off_seq + align64(M + N);
     const long long off_pd = off_bases + align64((M + N + 3) / 4);
     const long long off_score = off_pd + align64((long long)(sizeof(PairDesc) + 3) / 4);  // score, error flag
@@ -1859,8 +1796,6 @@ extern "C" int bpmax_gpu_score_noalloc(const int *seq1, long M, const int *seq2,
     pd.F_off = 0;
     pd.S1_off = 0;
     pd.S2_off = S2_rel;
-    pd.S2m_off = S2m_rel;
-    pd.S2t_off = S2t_rel;
     pd.seq1_off = 0;
     pd.seq2_off = (int)M;
     Weights W;
@@ -1879,7 +1814,6 @@ extern "C" int bpmax_gpu_score_noalloc(const int *seq1, long M, const int *seq2,
     }
     noalloc_prep_kernel<<<8, 256, 0, s>>>(seqs, (int)M, (int)N, bases, cj);
     single_strand_kernel<<<1, 512, 0, s>>>(pdp, bases, S, W);
-    s2_aux_kernel<<<1, 256, 0, s>>>(pdp, S);
     for (int d = 0; d < (int)M; ++d) {
         const int cells = (int)M - d;
         int n_r0 = 0;

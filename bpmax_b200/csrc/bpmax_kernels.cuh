@@ -19,9 +19,7 @@
 //       chunks (the pads spread the product kernel's shared loads over the bank groups). Inside
 //       diagonal blocks the entries below the diagonal are -inf except the subdiagonal, which
 //       holds S1 of the cell; padding rows/columns (>= N) are -inf.
-//     64 < Np <= 320 (a multiple of 64): tile images (below);
-//     Np > 320: row-major Np x Np with -inf outside the logical triangle and S1 on the
-//       subdiagonal, plus FT, the same table transposed (bpmax_kernels_large.cuh).
+//     Np > 64 (a multiple of 64): tile images (below).
 //   S1[M][M], S2[Np][Np] single-strand tables (S2 over the reversed strand 2)
 #pragma once
 #include <cstdint>
@@ -48,12 +46,11 @@ struct Weights {
 struct PairDesc {
     int M, N, Np;
     int cnt_off;       // persistent fill: offset of the pair's per-diagonal counters (M ints)
-    long long F_off;   // float offset of F[0] (and of FT[0] in the FT arena)
+    long long F_off;   // float offset of F[0]
     long long S1_off;  // float offset of S1 in the S arena
     long long S2_off;  // float offset of S2 in the S arena
-    long long S2m_off; // Np > 64 only: S2 with -inf outside its triangle
-    long long S2t_off; // Np > 64 only: ST1[j][k] = S2(k+1, j), -inf outside
-    long long S2d_off; // Np > 64 only: S2 diagonal-major and triangular, S2(i, i+e) at drow(Np, e) + i, -inf outside
+    long long S2x_off; // Np > 64 only: dense tile images of S2(i, k-1) (bpmax_tile.cuh)
+    long long S2y_off; // Np > 64 only: dense tile images of S2(k+1, j)
     int seq1_off;      // offset of seq1 in the base arena (uint8)
     int seq2_off;      // offset of the REVERSED seq2 in the base arena (uint8)
     long long cell_base;  // persistent fill: index of the pair's cell (0, 0) among all pairs' cells
@@ -85,21 +82,19 @@ __host__ __device__ __forceinline__ long long cell_index(int M, int i1, int j1)
 __device__ __forceinline__ float fmax3(float a, float b, float c) { return fmaxf(fmaxf(a, b), c); }
 
 // ------------------------------------------------------------------------------------------
-// Tile images: inner tables of width 64 < Np <= WIDE_TILE_MAX_NP (Np = 64 * NT) are stored per
-// outer cell as the upper triangle of NT x NT tiles of 64 x 64 in row-major tile-triangle order. A
+// Tile images: inner tables of width Np = 64 * NT > 64 are stored per outer cell as the upper triangle of NT x NT tiles of 64 x 64 in row-major tile-triangle order. A
 // diagonal tile is a width-64 cell image (above); an off-diagonal ("dense") tile holds all 64 of
 // its 8x8 blocks in block columns at WIDE_DENSE_COLBASE (wide_tables.inc), each column closed by a
 // halo piece: row 0 of block (0, bj) of the tile below, the row after the tile, so the row-shifted
 // operand of any tile is one image. Rows and columns >= N are -inf.
-// Wider tables (Np > WIDE_TILE_MAX_NP) are row-major with a transposed copy (bpmax_kernels_large.cuh).
 // ------------------------------------------------------------------------------------------
 #include "wide_tables.inc"
 
-constexpr int WIDE_TILE_MAX_NP = 320;                     // widest table stored as tile images
+constexpr int S2_ONE_CTA_NP = 320;                        // widest S2 filled by single_strand_kernel
 constexpr int WIDE_DIAG_CHUNKS = R0_TAB_COLBASE[8][8];    // diagonal tile image (width-64 cell image)
 constexpr int WIDE_DENSE_CHUNKS = WIDE_DENSE_COLBASE[8];  // dense tile image
 
-__host__ __device__ __forceinline__ bool is_tiled(int Np) { return Np > 64 && Np <= WIDE_TILE_MAX_NP; }
+__host__ __device__ __forceinline__ bool is_tiled(int Np) { return Np > 64; }
 
 // float offset of tile (I, J), I <= J, inside a cell's table of NT x NT tiles
 __host__ __device__ __forceinline__ long long wide_tile_off(int NT, int I, int J)
@@ -132,15 +127,13 @@ __host__ __device__ __forceinline__ long long wide_pos(int NT, int r, int c)
 __host__ __device__ __forceinline__ long long cell_floats(int Np)
 {
     if (Np <= 64) return 4LL * IMG_COLBASE(Np >> 3, Np >> 3);
-    if (Np <= WIDE_TILE_MAX_NP) return wide_cell_floats(Np >> 6);
-    return (long long)Np * Np;
+    return wide_cell_floats(Np >> 6);
 }
 
 // F(cell)[r][c] for any r, c < Np (entries below the diagonal as the tables define them)
 __device__ __forceinline__ float f_value(const PairDesc &pd, const float *__restrict__ F, long long cell, int r, int c)
 {
     const float *C = F + pd.F_off + cell * cell_floats(pd.Np);
-    if (pd.Np > WIDE_TILE_MAX_NP) return C[(long long)r * pd.Np + c];
     if (pd.Np > 64) {
         if (r > c) return r == c + 1 ? C[4 * 17 + 7] : NEG_INF;  // S1 piece of column 0 of tile (0, 0)
         return C[wide_pos(pd.Np >> 6, r, c)];
@@ -155,13 +148,13 @@ __device__ __forceinline__ float f_value(const PairDesc &pd, const float *__rest
 // S(i,j) = 0 if j-i<=3, else max(S(i+1,j-1)+intra(s[i],s[j]), max_{i<=k<j} S(i,k)+S(k+1,j)).
 // One CTA per pair; wavefront over the diagonal j-i. Cells outside the N x N upper triangle are
 // left at 0 and never read. (S1 is built diagonal by diagonal inside finalize_small_kernel.) Pairs
-// with tables wider than the tile images are left to s2_diag_kernel, one launch per diagonal.
+// wider than S2_ONE_CTA_NP are left to s2_diag_kernel, one launch per diagonal.
 // ------------------------------------------------------------------------------------------
 __global__ void single_strand_kernel(const PairDesc *__restrict__ pairs, const uint8_t *__restrict__ bases,
                                      float *__restrict__ S, Weights W)
 {
     const PairDesc pd = pairs[blockIdx.x];
-    if (pd.Np > WIDE_TILE_MAX_NP) return;  // row-major tables: one launch per diagonal (s2_diag_kernel)
+    if (pd.Np > S2_ONE_CTA_NP) return;  // one launch per diagonal (s2_diag_kernel)
     const bool second = true;
     const int L = second ? pd.N : pd.M;
     const int ld = second ? pd.Np : pd.M;

@@ -6,22 +6,13 @@
 //   F(i1,j1,i2,i2) = seq1[i1]                                                  (j1 > i1)
 //   F(i1,j1,i2,j2) = max_{i1<=k1<j1, i2<=k2<j2} F(i1,k1,i2,k2) + F(k1+1,j1,k2+1,j2)   (j1 > i1, j2 > i2)
 // The product kernels evaluate R0 + R3 + R4 as one shifted product whose extra terms read S1 on the
-// subdiagonal of every table (and, for wide tables, the S1 array): with -inf there, they evaluate
-// R0 alone. The finalize of this mode only writes the base values and -inf where the full fill
+// subdiagonal of every table: with -inf there, they evaluate R0 alone. The finalize of this mode only writes the base values and -inf where the full fill
 // writes S1; the sequences are non-negative, so every value is >= +0 and the product's integer
 // max merge stays exact.
 #pragma once
-#include "bpmax_kernels_large.cuh"
+#include "bpmax_kernels.cuh"
 
 namespace bpmax {
-
-// S1 := -inf for every pair (read by the wide product kernel at row 0 of A and the guard row of B)
-__global__ void r0only_prep_kernel(const PairDesc *__restrict__ pairs, float *__restrict__ S)
-{
-    const PairDesc pd = pairs[blockIdx.x];
-    float *S1 = S + pd.S1_off;
-    for (int q = threadIdx.x; q < pd.M * pd.M; q += blockDim.x) S1[q] = NEG_INF;
-}
 
 // Cell images (Np <= 64), one CTA per outer cell of diagonal d. vals = seq1 (M floats) then seq2
 // (N floats) of the pair, unreversed.
@@ -60,8 +51,8 @@ __global__ void __launch_bounds__(128) r0only_finalize_small_kernel(const CellJo
     }
 }
 
-// Tile images (64 < Np <= WIDE_TILE_MAX_NP): one CTA per outer cell of diagonal d rewrites every
-// block of every tile with the base values and -inf where the full fill writes S1, and writes the
+// Tile images (Np > 64): CTA (blockIdx.x, blockIdx.y) rewrites every block of tile row blockIdx.y of
+// outer cell blockIdx.x of diagonal d with the base values and -inf where the full fill writes S1, and writes the
 // closing pieces (S1 pieces of the diagonal tiles: -inf; halo pieces of the dense tiles: the row
 // after the tile, by the same rule). The rule is idempotent, so reading an entry another thread
 // has already rewritten gives the same value.
@@ -78,73 +69,36 @@ __global__ void __launch_bounds__(256) r0only_finalize_tile_kernel(const CellJob
     auto val = [&](int r, int c) {
         return !(r <= c && c < N) ? NEG_INF : (d == 0 ? v2[r] : (r == c ? v1[i1] : Fc[wide_pos(NT, r, c)]));
     };
-    for (int I = 0; I < NT; ++I)
-        for (int J = I; J < NT; ++J) {
-            const long long to = wide_tile_off(NT, I, J);
-            const int nblk = I == J ? 36 : 64;
-            for (int q4 = threadIdx.x; q4 < nblk * 16 + 16; q4 += blockDim.x) {
-                if (q4 >= nblk * 16) {
-                    const int bj = (q4 - nblk * 16) >> 1, h = q4 & 1;
-                    float v[4];
-#pragma unroll
-                    for (int t = 0; t < 4; ++t) v[t] = I == J ? NEG_INF : val(64 * I + 64, 64 * J + 8 * bj + 4 * h + t);
-                    const int cb = I == J ? c_img_colbase[8][bj] : c_wide_dense_colbase[bj];
-                    *reinterpret_cast<float4 *>(Fc + to + 4 * (cb + 17 * (I == J ? bj + 1 : 8)) + 4 * h) =
-                        make_float4(v[0], v[1], v[2], v[3]);
-                    continue;
-                }
-                int bi, bj;
-                if (I == J) {
-                    blk_decode(8, q4 >> 4, bi, bj);
-                } else {
-                    bi = (q4 >> 4) & 7;
-                    bj = q4 >> 7;
-                }
-                const int r = 64 * I + 8 * bi + ((q4 & 15) >> 1), c0 = 64 * J + 8 * bj + 4 * (q4 & 1);
+    const int I = blockIdx.y;
+    for (int J = I; J < NT; ++J) {
+        const long long to = wide_tile_off(NT, I, J);
+        const int nblk = I == J ? 36 : 64;
+        for (int q4 = threadIdx.x; q4 < nblk * 16 + 16; q4 += blockDim.x) {
+            if (q4 >= nblk * 16) {
+                const int bj = (q4 - nblk * 16) >> 1, h = q4 & 1;
                 float v[4];
 #pragma unroll
-                for (int t = 0; t < 4; ++t) v[t] = val(r, c0 + t);
-                const long long o = to + 4 * ((I == J ? c_img_colbase[8][bj] : c_wide_dense_colbase[bj]) + 17 * bi) +
-                                    4 * (q4 & 15);
-                *reinterpret_cast<float4 *>(Fc + o) = make_float4(v[0], v[1], v[2], v[3]);
+                for (int t = 0; t < 4; ++t) v[t] = I == J ? NEG_INF : val(64 * I + 64, 64 * J + 8 * bj + 4 * h + t);
+                const int cb = I == J ? c_img_colbase[8][bj] : c_wide_dense_colbase[bj];
+                *reinterpret_cast<float4 *>(Fc + to + 4 * (cb + 17 * (I == J ? bj + 1 : 8)) + 4 * h) =
+                    make_float4(v[0], v[1], v[2], v[3]);
+                continue;
             }
-        }
-}
-
-// Row-major tables and their transposes (Np > WIDE_TILE_MAX_NP): CTA (blockIdx.x, blockIdx.y) writes the 32-row
-// band blockIdx.y of cell blockIdx.x of diagonal d, one 32 x 32 tile at a time, and the matching
-// column band of the transpose through a shared tile (coalesced reads and writes on both sides).
-constexpr int R0ONLY_TILE = 32;
-__global__ void __launch_bounds__(256) r0only_finalize_wide_kernel(const CellJob *__restrict__ jobs,
-                                                                  const PairDesc *__restrict__ pairs,
-                                                                  float *__restrict__ F, float *__restrict__ FT,
-                                                                  const float *__restrict__ vals, int d)
-{
-    constexpr int TL = R0ONLY_TILE;
-    __shared__ float tile[TL][TL + 1];
-    const CellJob job = jobs[blockIdx.x];
-    const PairDesc pd = pairs[job.pair];
-    const int M = pd.M, N = pd.N, Np = pd.Np, i1 = job.i1;
-    const long long cell = cell_index(M, i1, i1 + d) * ((long long)Np * Np);
-    float *Fc = F + pd.F_off + cell;
-    float *FTc = FT + pd.F_off + cell;
-    const float *v1 = vals, *v2 = vals + M;
-    const int tx = threadIdx.x & (TL - 1), ty = threadIdx.x / TL;  // 32 x 8 threads
-    const int r0 = TL * blockIdx.y;
-    for (int c0 = 0; c0 < Np; c0 += TL) {
+            int bi, bj;
+            if (I == J) {
+                blk_decode(8, q4 >> 4, bi, bj);
+            } else {
+                bi = (q4 >> 4) & 7;
+                bj = q4 >> 7;
+            }
+            const int r = 64 * I + 8 * bi + ((q4 & 15) >> 1), c0 = 64 * J + 8 * bj + 4 * (q4 & 1);
+            float v[4];
 #pragma unroll
-        for (int y = ty; y < TL; y += 8) {
-            const int r = r0 + y, c = c0 + tx;
-            const long long q = (long long)r * Np + c;
-            const float f = !(r <= c && c < N) ? NEG_INF : (d == 0 ? v2[r] : (r == c ? v1[i1] : Fc[q]));
-            Fc[q] = f;
-            tile[y][tx] = f;
+            for (int t = 0; t < 4; ++t) v[t] = val(r, c0 + t);
+            const long long o = to + 4 * ((I == J ? c_img_colbase[8][bj] : c_wide_dense_colbase[bj]) + 17 * bi) +
+                                4 * (q4 & 15);
+            *reinterpret_cast<float4 *>(Fc + o) = make_float4(v[0], v[1], v[2], v[3]);
         }
-        __syncthreads();
-#pragma unroll
-        for (int y = ty; y < TL; y += 8)  // FT[c0 + y][r0 + tx] = F[r0 + tx][c0 + y]
-            FTc[(long long)(c0 + y) * Np + r0 + tx] = tile[tx][y];
-        __syncthreads();
     }
 }
 

@@ -28,7 +28,6 @@
 // whole ring waits for it), hence the cursor that only adds. r0_kernel took 1,240 with 20,160 bytes
 // per item, against 13,440 here. Fill: 1024x64 766 -> 661 ms, the 512-pair batch 523 -> 460 ms.
 #pragma once
-#include "bpmax_kernels_large.cuh"  // cp_async16
 #include "bpmax_r0.cuh"
 
 namespace bpmax {

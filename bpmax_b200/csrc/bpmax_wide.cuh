@@ -1,5 +1,5 @@
 // bpmax_wide.cuh -- the R0 + R3 + R4 product kernel for inner tables stored as tile images
-// (64 < Np <= WIDE_TILE_MAX_NP, Np = 64 * NT; layout in bpmax_kernels.cuh).
+// (Np = 64 * NT > 64; layout in bpmax_kernels.cuh).
 //
 // The triangular (max,+) product of one item of the width-64 kernel (bpmax_r0.cuh),
 //   max_{k in [i2-1, j2]} A[i2][k] + Bs[k][j2]      (R0, and R3 / R4 through S1 on the subdiagonals)

@@ -42,3 +42,33 @@ def test_bulk_launches_vs_oracle(eng, oracle_mod, N):
     got = eng.score_batch(pairs)
     exp = [oracle_mod.score(oracle_mod.fill(a, b, W.REFERENCE_WEIGHTS)[0], len(a), len(b)) for a, b in pairs]
     assert np.array_equal(bits(got), bits(np.array(exp, dtype=np.float32)))
+
+
+@pytest.mark.parametrize("N", [65, 66, 71, 72, 73, 96, 127, 128, 129, 137, 192, 193, 255, 320, 321, 385])
+def test_tile_tables_vs_oracle(eng, oracle_mod, N):
+    """Tables of 64x64 tiles: strand-2 lengths around whole tiles and whole 8x8 blocks. Few tiles: the
+    slabs over finished tiles run in their own launches."""
+    M = 6
+    s1, s2 = W.pair(M, N, 3000 + N)
+    w = W.random_weights(N) if N % 2 else W.INTEGER_WEIGHTS
+    eng.set_weights(w)
+    F, score = eng.fill_compact(s1, s2)
+    Fo, _, _ = oracle_mod.fill(s1, s2, w)
+    assert np.array_equal(bits(F), bits(Fo))
+    assert score == oracle_mod.score(Fo, M, N)
+
+
+@pytest.mark.parametrize("lo,hi", [(65, 128), (129, 192), (193, 200)])
+def test_tile_tables_of_many_cells_vs_oracle(eng, oracle_mod, lo, hi):
+    """More tiles in a launch than SMs: each CTA computes the slabs of its tile itself."""
+    rng = np.random.default_rng(lo)
+    pairs = [(W.random_sequence(5, rng), W.random_sequence(int(rng.integers(lo, hi + 1)), rng)) for _ in range(40)]
+    eng.set_weights(W.INTEGER_WEIGHTS)
+    got = eng.score_batch(pairs)
+    tables = [oracle_mod.fill(a, b, W.INTEGER_WEIGHTS)[0] for a, b in pairs]
+    exp = [oracle_mod.score(F, len(a), len(b)) for F, (a, b) in zip(tables, pairs)]
+    assert np.array_equal(bits(got), bits(np.array(exp, dtype=np.float32)))
+    for p in (0, 39):
+        win = eng.read_cells(p, 0, 5, 0, 5, len(pairs[p][1]))
+        iu, ju = np.triu_indices(5)
+        assert np.array_equal(bits(win[iu, ju]), bits(tables[p]))
