@@ -111,7 +111,7 @@ struct Plan {
     int r0_variant = 0, wide_stages = 2, class_share = 0, persist = 0;
     long strip_tasks = 0;
     bool r0_only = false;  // R0-only double max-plus (bpmax_gpu_r0_only) instead of the BPMax fill
-    std::vector<cudaEvent_t> diag_ev;  // one pair only: outer diagonal d finalized (recorded by the graph)
+    std::vector<cudaEvent_t> diag_ev;  // copy-out of one pair: outer diagonal d finalized (recorded by the graph)
     // persistent fill (one launch per width class walking the diagonals with dependency counters):
     // the work queues of all classes back to back, each class's range and CTA count
     bool persistent = false, copyout = false;
@@ -144,6 +144,7 @@ struct bpmax_ctx {
     RefOut want_ref{nullptr, 0, 0};  // the next fill's finalize also writes the reference layout there
     DevBuf refdev;                   // that reference layout, diagonal-major
     bool r0_only = false;  // mode of the next prepare()
+    bool one_chain = false;  // the fill being enqueued runs as one chain of launches
     int r0_occ_v[2][9] = {};  // resident product CTAs per SM, per shape variant and width class NB
     int wide_occ[4] = {};     // resident tile-product CTAs per SM, per stage count
     // schedule tunables (bpmax_gpu_set_tuning / bpmax_gpu_autotune); a plan is built with the
@@ -516,12 +517,34 @@ int build_plan(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int
     return BPMAX_OK;
 }
 
+// Launch of a kernel of a fill's chain. early: by programmatic dependent launch (chain_wait in the
+// kernel), where the chain is the only one of its fill (the early CTAs of several chains would hold each
+// other's room). That hides the launch and the first loads of a short kernel (37x23 0.53 -> 0.35 ms,
+// 200x8 2.42 -> 1.52, 128x32 2.44 -> 1.97), but places its CTAs where room comes free first, several to
+// an SM: kernels of a few hundred large CTAs start normally (early 512-thread finalizes 128x64 4.61 against
+// 4.21 ms, early tile kernels 16x750 17.1 against 16.2, early long tile products 256x256 737 against 709).
+template <class... P, class... A>
+void launch_chain(const bpmax_ctx *ctx, bool early, dim3 grid, int threads, size_t smem, cudaStream_t s, void (*kernel)(P...), A... args)
+{
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    c.attrs = &at;
+    c.numAttrs = early && ctx->one_chain ? 1 : 0;
+    cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 template <int STAGES>
 void launch_r0_wide_t(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
 {
     const int grid = std::min(L.count, L.cap > 0 ? L.cap : std::max(1, ctx->wide_occ[STAGES]) * ctx->sms);
-    r0_wide_kernel<STAGES><<<grid, WideCfg<STAGES>::THREADS, WideCfg<STAGES>::SMEM, s>>>(
-        (const R0JobW *)ctx->r0wjobs.p + L.first, L.count, (const PairDesc *)ctx->pairs.p, (float *)ctx->F.p, L.d,
+    launch_chain(
+        ctx, L.count <= 4 * grid, grid, WideCfg<STAGES>::THREADS, WideCfg<STAGES>::SMEM, s, r0_wide_kernel<STAGES>, (const R0JobW *)ctx->r0wjobs.p + L.first, L.count, (const PairDesc *)ctx->pairs.p, (float *)ctx->F.p, L.d,
         wait_ctl(ctx));
 }
 
@@ -548,13 +571,13 @@ int launch_fin_tiles(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
         const int parts = tiles < ctx->sms ? std::min(slabs, (2 * ctx->sms + tiles - 1) / tiles) : 1;
         const bool split = parts > 1;
         if (split) {
-            tile_product_kernel<<<dim3(tiles, parts), TILE_THREADS, TILE_SMEM, s>>>(jobs, pairs, F, S, L.d, t, NT);
+            launch_chain(ctx, false, dim3(tiles, parts), TILE_THREADS, TILE_SMEM, s, tile_product_kernel, jobs, pairs, F, S, L.d, t,
+                         NT);
             ++n;
         }
         const int s1_ctas = t == 0 ? (L.s1_count + TILE_THREADS / 32 - 1) / (TILE_THREADS / 32) : 0;
-        tile_final_kernel<<<tiles + s1_ctas, TILE_THREADS, TILE_SMEM, s>>>(jobs, L.count, s1jobs, L.s1_count, pairs, F, S,
-                                                                           (const uint8_t *)ctx->bases.p, ctx->W, L.d, t,
-                                                                           NT, !split);
+        launch_chain(ctx, false, tiles + s1_ctas, TILE_THREADS, TILE_SMEM, s, tile_final_kernel, jobs, L.count, s1jobs, L.s1_count,
+                     pairs, F, S, (const uint8_t *)ctx->bases.p, ctx->W, L.d, t, NT, !split);
         ++n;
     }
     return n;
@@ -566,16 +589,15 @@ void launch_r0_v(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
     using C = R0Cfg<NB, V>;
     // resident CTAs (or the class's share of them); each loops over jobs
     const int grid = std::min(L.count, L.cap > 0 ? L.cap : std::max(1, ctx->r0_occ_v[V][NB]) * ctx->sms);
-    r0_kernel<NB, V><<<grid, C::THREADS, C::SMEM, s>>>((const R0Job *)ctx->r0jobs.p + L.first, L.count,
-                                                       (const PairDesc *)ctx->pairs.p, (float *)ctx->F.p, L.d,
-                                                       wait_ctl(ctx));
+    launch_chain(ctx, true, grid, C::THREADS, C::SMEM, s, r0_kernel<NB, V>, (const R0Job *)ctx->r0jobs.p + L.first, L.count,
+                 (const PairDesc *)ctx->pairs.p, (float *)ctx->F.p, L.d, wait_ctl(ctx));
 }
 
 template <int NB>
 void launch_strip(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
 {
-    r0_strip_kernel<NB><<<std::min(L.count, L.cap), StripCfg<NB>::THREADS, StripCfg<NB>::SMEM, s>>>(
-        (const StripJob *)ctx->stripjobs.p + L.first, L.count, (const PairDesc *)ctx->pairs.p, (float *)ctx->F.p, L.d,
+    launch_chain(
+        ctx, true, std::min(L.count, L.cap), StripCfg<NB>::THREADS, StripCfg<NB>::SMEM, s, r0_strip_kernel<NB>, (const StripJob *)ctx->stripjobs.p + L.first, L.count, (const PairDesc *)ctx->pairs.p, (float *)ctx->F.p, L.d,
         wait_ctl(ctx));
 }
 
@@ -602,7 +624,8 @@ template <int NB, int T>
 void launch_fin_t(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
 {
     using Sh = FinShape<8 * NB, T>;
-    finalize_small_kernel<8 * NB, T><<<L.count + (L.s1_count + Sh::WARPS - 1) / Sh::WARPS, Sh::THREADS, Sh::SMEM, s>>>(
+    launch_chain(
+        ctx, T < 512, L.count + (L.s1_count + Sh::WARPS - 1) / Sh::WARPS, Sh::THREADS, Sh::SMEM, s, finalize_small_kernel<8 * NB, T>,
         (const CellJob *)ctx->celljobs.p + L.first, L.count, (const CellJob *)ctx->celljobs.p + L.s1_first, L.s1_count,
         (const PairDesc *)ctx->pairs.p, (float *)ctx->F.p, (float *)ctx->S.p, (const uint8_t *)ctx->bases.p, ctx->W,
         L.d, ctx->plan.ref);
@@ -622,16 +645,16 @@ void launch_r0only_fin(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
     const float *vals = (const float *)ctx->r0vals.p;
     switch (L.np > MAX_SMALL_NP ? 0 : L.np / 8) {
     case 0:
-        r0only_finalize_tile_kernel<<<dim3(L.count, L.np / 64), 256, 0, s>>>(jobs, pd, (float *)ctx->F.p, vals, L.d);
+        launch_chain(ctx, true, dim3(L.count, L.np / 64), 256, 0, s, r0only_finalize_tile_kernel, jobs, pd, (float *)ctx->F.p, vals, L.d);
         break;
-    case 1: r0only_finalize_small_kernel<8><<<L.count, 128, 0, s>>>(jobs, pd, (float *)ctx->F.p, vals, L.d); break;
-    case 2: r0only_finalize_small_kernel<16><<<L.count, 128, 0, s>>>(jobs, pd, (float *)ctx->F.p, vals, L.d); break;
-    case 3: r0only_finalize_small_kernel<24><<<L.count, 128, 0, s>>>(jobs, pd, (float *)ctx->F.p, vals, L.d); break;
-    case 4: r0only_finalize_small_kernel<32><<<L.count, 128, 0, s>>>(jobs, pd, (float *)ctx->F.p, vals, L.d); break;
-    case 5: r0only_finalize_small_kernel<40><<<L.count, 128, 0, s>>>(jobs, pd, (float *)ctx->F.p, vals, L.d); break;
-    case 6: r0only_finalize_small_kernel<48><<<L.count, 128, 0, s>>>(jobs, pd, (float *)ctx->F.p, vals, L.d); break;
-    case 7: r0only_finalize_small_kernel<56><<<L.count, 128, 0, s>>>(jobs, pd, (float *)ctx->F.p, vals, L.d); break;
-    default: r0only_finalize_small_kernel<64><<<L.count, 128, 0, s>>>(jobs, pd, (float *)ctx->F.p, vals, L.d); break;
+    case 1: launch_chain(ctx, true, L.count, 128, 0, s, r0only_finalize_small_kernel<8>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
+    case 2: launch_chain(ctx, true, L.count, 128, 0, s, r0only_finalize_small_kernel<16>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
+    case 3: launch_chain(ctx, true, L.count, 128, 0, s, r0only_finalize_small_kernel<24>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
+    case 4: launch_chain(ctx, true, L.count, 128, 0, s, r0only_finalize_small_kernel<32>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
+    case 5: launch_chain(ctx, true, L.count, 128, 0, s, r0only_finalize_small_kernel<40>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
+    case 6: launch_chain(ctx, true, L.count, 128, 0, s, r0only_finalize_small_kernel<48>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
+    case 7: launch_chain(ctx, true, L.count, 128, 0, s, r0only_finalize_small_kernel<56>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
+    default: launch_chain(ctx, true, L.count, 128, 0, s, r0only_finalize_small_kernel<64>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
     }
 }
 
@@ -720,6 +743,7 @@ struct ProfScope {
 int enqueue_fill(bpmax_ctx *ctx, Plan &P, KernelProfile *kp = nullptr)
 {
     long launches = 0;
+    ctx->one_chain = !(kp && kp->on) && !(P.classes.size() > 1 && P.class_streams);
     CK(cudaMemsetAsync(ctx->F.p, 0, (size_t)P.F_floats * sizeof(float), ctx->stream));
     CK(cudaMemsetAsync(ctx->S.p, 0, (size_t)P.S_floats * sizeof(float), ctx->stream));  // S1 starts at 0
     CK(cudaMemsetAsync(ctx->errflag.p, 0, sizeof(int), ctx->stream));
@@ -730,12 +754,12 @@ int enqueue_fill(bpmax_ctx *ctx, Plan &P, KernelProfile *kp = nullptr)
         for (int p = 0; p < (int)P.pairs.size(); ++p)  // wider tables: one launch per diagonal of S2
             if (P.pairs[p].Np > S2_ONE_CTA_NP)
                 for (int d = 4; d < P.pairs[p].N; ++d, ++launches)
-                    s2_diag_kernel<<<(P.pairs[p].N - d + 7) / 8, 256, 0, ctx->stream>>>(
-                        (const PairDesc *)ctx->pairs.p, p, (const uint8_t *)ctx->bases.p, (float *)ctx->S.p, ctx->W, d);
+                    launch_chain(
+                        ctx, true, (P.pairs[p].N - d + 7) / 8, 256, 0, ctx->stream, s2_diag_kernel, (const PairDesc *)ctx->pairs.p, p, (const uint8_t *)ctx->bases.p, (float *)ctx->S.p, ctx->W, d);
         launches += 1;
         if (P.classes.back() > MAX_SMALL_NP) {
-            s2_aux_kernel<<<dim3(64, (int)P.pairs.size()), 256, 0, ctx->stream>>>((const PairDesc *)ctx->pairs.p,
-                                                                                 (float *)ctx->S.p);
+            launch_chain(ctx, true, dim3(64, (int)P.pairs.size()), 256, 0, ctx->stream, s2_aux_kernel,
+                         (const PairDesc *)ctx->pairs.p, (float *)ctx->S.p);
             launches += 1;
         }
     }
@@ -877,7 +901,7 @@ int prepare(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int> &
         Plan &P = ctx->plan;
         P.r0_only = ctx->r0_only;
         P.ref = ctx->want_ref;
-        if (P.pairs.size() == 1) {
+        if (P.copyout) {
             P.diag_ev.assign(P.maxM, nullptr);
             for (auto &e : P.diag_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         }

@@ -79,6 +79,16 @@ __host__ __device__ __forceinline__ long long cell_index(int M, int i1, int j1)
     return (long long)i1 * M - (long long)i1 * (i1 - 1) / 2 + (j1 - i1);
 }
 
+// Launches of one chain follow each other by programmatic dependent launch: a kernel's CTAs may start
+// while the launch before it still runs, read what no kernel of the fill writes (job lists, pair
+// records, sequences, weights), and wait here until that launch is complete and its writes are visible.
+// Every thread of every kernel of a chain calls this before it touches S1, S2 or F, and only then lets
+// the next launch start, so whatever starts early has only the launch before it still running.
+__device__ __forceinline__ void chain_wait()
+{
+    asm volatile("griddepcontrol.wait;\n griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __device__ __forceinline__ float fmax3(float a, float b, float c) { return fmaxf(fmaxf(a, b), c); }
 
 // ------------------------------------------------------------------------------------------
@@ -325,11 +335,15 @@ finalize_small_kernel(const CellJob *__restrict__ jobs, int njobs, const CellJob
     __syncthreads();
     if ((int)blockIdx.x >= njobs) {  // S1 cells (i, i+d+1), one per warp
         const int q = ((int)blockIdx.x - njobs) * Sh::WARPS + warp;
-        if (q >= ns1) return;
+        if (q >= ns1) {
+            chain_wait();
+            return;
+        }
         const CellJob job = s1jobs[q];
         const PairDesc pd = pairs[job.pair];
         const int M = pd.M, i = job.i1, j = i + d + 1;
         float *S1 = S + pd.S1_off;
+        chain_wait();
         if (j - i <= 3) return;  // stays 0
         const uint8_t *s1 = bases + pd.seq1_off;
         float r0 = NEG_INF, r1 = NEG_INF;
@@ -352,12 +366,14 @@ finalize_small_kernel(const CellJob *__restrict__ jobs, int njobs, const CellJob
     const float *S2 = S + pd.S2_off;
     const uint8_t *s1 = bases + pd.seq1_off;
     const uint8_t *s2r = bases + pd.seq2_off;
-    const float s1v = S1[i1 * M + j1];
     for (int q = tid; q < NP; q += Sh::THREADS) sb[q] = q < N ? s2r[q] : 4;
+    const int x1 = s1[i1], y1 = s1[j1];
+    chain_wait();
+    const float s1v = S1[i1 * M + j1];
     // start values (accumulated products, S1+S2, SW1; the inter-strand base on the diagonal of the
     // diagonal cells) and S2, both by diagonals, 4 columns of one block row per step
     const bool sw1 = d >= 4;
-    const float w1 = sw1 ? score_w(wsh, s1[i1], s1[j1]) : 0.0f;
+    const float w1 = sw1 ? score_w(wsh, x1, y1) : 0.0f;
     const float *Fi = F + pd.F_off + (sw1 ? cell_index(M, i1 + 1, j1 - 1) * CELL : 0);
     for (int q4 = tid; q4 < NBLK * 16; q4 += Sh::THREADS) {
         int BI, BJ;
@@ -371,7 +387,7 @@ finalize_small_kernel(const CellJob *__restrict__ jobs, int njobs, const CellJob
         for (int t = 0; t < 4; ++t) {
             const int c = c0 + t;
             if (r <= c && c < N) {
-                D[(c - r) * LD + r] = d == 0 && r == c ? score_w(wsh + 6, s1[i1], s2r[r])
+                D[(c - r) * LD + r] = d == 0 && r == c ? score_w(wsh + 6, x1, s2r[r])
                                                        : fmax3(fv[t], s1v + sv[t], pv[t] + w1);
                 Sd[(c - r) * LD + r] = sv[t];
             }

@@ -366,6 +366,7 @@ r0_kernel(const R0Job *__restrict__ jobs, int njobs, const PairDesc *__restrict_
         }
     }
     __syncthreads();
+    chain_wait();
 #pragma unroll 1
     for (int s = 0; s < S; ++s)
         if (pj < njobs) {

@@ -26,6 +26,7 @@ __global__ void __launch_bounds__(128) r0only_finalize_small_kernel(const CellJo
     constexpr long long CELL = 4LL * R0_TAB_COLBASE[NB][NB];
     const CellJob job = jobs[blockIdx.x];
     const PairDesc pd = pairs[job.pair];
+    chain_wait();
     const int M = pd.M, N = pd.N, i1 = job.i1;
     float *Fc = F + pd.F_off + cell_index(M, i1, i1 + d) * CELL;
     const float *v1 = vals, *v2 = vals + M;
@@ -63,6 +64,7 @@ __global__ void __launch_bounds__(256) r0only_finalize_tile_kernel(const CellJob
 {
     const CellJob job = jobs[blockIdx.x];
     const PairDesc pd = pairs[job.pair];
+    chain_wait();
     const int M = pd.M, N = pd.N, NT = pd.Np >> 6, i1 = job.i1;
     float *Fc = F + pd.F_off + cell_index(M, i1, i1 + d) * wide_cell_floats(NT);
     const float *v1 = vals, *v2 = vals + M;

@@ -234,6 +234,7 @@ r0_strip_kernel(const StripJob *__restrict__ jobs, int njobs, const PairDesc *__
         __syncwarp();
     }
     __syncthreads();
+    chain_wait();
     if (warp == C::PW && !ctl.inject)
         for (int s = 0; s < S; ++s) produce(s);
 

@@ -60,6 +60,7 @@ __global__ void s2_aux_kernel(const PairDesc *__restrict__ pairs, float *__restr
 {
     const PairDesc pd = pairs[blockIdx.y];
     const int Np = pd.Np, N = pd.N, NT = Np >> 6;
+    chain_wait();
     if (Np <= 64) return;
     const float *S2 = S + pd.S2_off;
     float *S2X = S + pd.S2x_off, *S2Y = S + pd.S2y_off;
@@ -88,6 +89,7 @@ s2_diag_kernel(const PairDesc *__restrict__ pairs, int p, const uint8_t *__restr
     const PairDesc pd = pairs[p];
     const int L = pd.N, ld = pd.Np;
     const int i = (int)blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    chain_wait();
     if (i >= L - d) return;
     const int j = i + d;
     float *T = S + pd.S2_off, *TT = S + pd.S2x_off;
@@ -205,6 +207,7 @@ tile_product_kernel(const CellJob *__restrict__ jobs, const PairDesc *__restrict
     const PairDesc pd = pairs[job.pair];
     float *Fc = F + pd.F_off + cell_index(pd.M, job.i1, job.i1 + d) * wide_cell_floats(NT);
     const int Z = gridDim.y, z = blockIdx.y, s0 = 2 * t * z / Z, s1 = 2 * t * (z + 1) / Z;
+    chain_wait();
     if (s0 == s1) return;
     tile_slabs(sm, Fc, S + pd.S2x_off, S + pd.S2y_off, NT, I, t, s0, s1);
     const int *red = reinterpret_cast<const int *>(sm + TILE_OFF_SLAB);
@@ -236,6 +239,7 @@ tile_final_kernel(const CellJob *__restrict__ jobs, int ncells, const CellJob *_
     if ((int)blockIdx.x >= ncells * nt) {
         __syncthreads();
         const int q = ((int)blockIdx.x - ncells * nt) * (TILE_THREADS / 32) + warp;
+        chain_wait();
         if (q < ns1) s1_cell(s1jobs[q], pairs, S, bases, wsh, d, lane);
         return;
     }
@@ -253,6 +257,8 @@ tile_final_kernel(const CellJob *__restrict__ jobs, int ncells, const CellJob *_
         bI[tid] = 64 * I + tid < N ? s2r[64 * I + tid] : 4;
     else if (tid < 128)
         bJ[tid - 64] = 64 * J + tid - 64 < N ? s2r[64 * J + tid - 64] : 4;
+    const int x1 = s1[i1], y1 = s1[j1];
+    chain_wait();
     const float s1v = S[pd.S1_off + i1 * M + j1];
     if (fused && t > 0)
         tile_slabs(sm, Fc, S + pd.S2x_off, S + pd.S2y_off, NT, I, t, 0, 2 * t);
@@ -261,7 +267,7 @@ tile_final_kernel(const CellJob *__restrict__ jobs, int ncells, const CellJob *_
     // start values: accumulated products, S1+S2, SW1 (F(i1+1,j1-1,.)+intra if j1-i1 >= 4), the slabs; the
     // inter-strand base on the diagonal of the diagonal cells. Entries outside the table stay -inf.
     const bool sw1 = d >= 4;
-    const float w1 = sw1 ? score_w(wsh, s1[i1], s1[j1]) : 0.0f;
+    const float w1 = sw1 ? score_w(wsh, x1, y1) : 0.0f;
     const float *Fi = F + pd.F_off + (sw1 ? cell_index(M, i1 + 1, j1 - 1) * CELL : 0) + wide_tile_off(NT, I, J);
     const float *red = tsm + TILE_OFF_SLAB / 4;
     const int nblk = t == 0 ? 36 : 64;
@@ -303,7 +309,7 @@ tile_final_kernel(const CellJob *__restrict__ jobs, int ncells, const CellJob *_
             if (c < ncol && (t > 0 || r <= c)) {
                 float v = fmax3(fv[u], s1v + sv[u], pv[u] + w1);
                 if (fused && t > 0) v = fmaxf(v, red[tile_red_off(r, c)]);
-                if (d == 0 && t == 0 && r == c) v = score_w(wsh + 6, s1[i1], bI[r]);
+                if (d == 0 && t == 0 && r == c) v = score_w(wsh + 6, x1, bI[r]);
                 T[r * LD + c] = v;
             }
         }

@@ -129,6 +129,7 @@ r0_wide_kernel(const R0JobW *__restrict__ jobs, int njobs, const PairDesc *__res
         }
     };
     load_pjob(pj);
+    chain_wait();
     for (int s = 0; s < S; ++s)
         if (pj < njobs) {
             if (tid == 0 && !ctl.inject) fill_stage(s, pit);
