@@ -100,7 +100,16 @@ struct Plan {
     // per diagonal and Np class (index NB-1): ranges in the job arrays
     // np = inner table width class; strip (product launches): strips of diagonals d .. d+T-1
     // cap: at most this many CTAs (0: as many as are resident), from the class shares
-    struct Launch { int d, np, first, count, s1_first = 0, s1_count = 0; bool strip = false; int cap = 0; };
+    // r0_kernel launches of one pair: q offset pairs per job of `edge` (0: jobs from the list)
+    struct Launch {
+        int d, np, first, count, s1_first = 0, s1_count = 0;
+        bool strip = false;
+        int cap = 0, cells = 0, q = 0, edge = 0;
+        R0Jobs jobs(const void *list) const
+        {
+            return q ? R0Jobs{nullptr, cells, q, edge} : R0Jobs{(const R0Job *)list + first, 0, 0, 0};
+        }
+    };
     std::vector<Launch> r0_launches, fin_launches;
     std::vector<R0Job> r0_jobs;
     std::vector<StripJob> strip_jobs;  // jobs of strip launches (first/count index this array)
@@ -462,12 +471,19 @@ int build_plan(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int
                 const long long q = r0_pairs_per_job(cells, edge, resident, qmin, qmax, P.merge_items);
                 Plan::Launch rl{d, np, (int)P.r0_jobs.size(), 0};
                 rl.cap = share.empty() ? 0 : (int)resident;
-                for (long long c0 = 0; c0 < edge; c0 += q)
-                    for (int p = 0; p < n; ++p)
-                        if (P.pairs[p].Np == np && Ms[p] > d)
-                            for (int i1 = 0; i1 < Ms[p] - d; ++i1)
-                                P.r0_jobs.push_back(R0Job{p, i1, (int)c0, (int)std::min(c0 + q, edge)});
-                rl.count = (int)P.r0_jobs.size() - rl.first;
+                if (n == 1) {
+                    rl.cells = (int)cells;
+                    rl.q = (int)q;
+                    rl.edge = (int)edge;
+                    rl.count = (int)(cells * ((edge + q - 1) / q));
+                } else {
+                    for (long long c0 = 0; c0 < edge; c0 += q)
+                        for (int p = 0; p < n; ++p)
+                            if (P.pairs[p].Np == np && Ms[p] > d)
+                                for (int i1 = 0; i1 < Ms[p] - d; ++i1)
+                                    P.r0_jobs.push_back(R0Job{p, i1, (int)c0, (int)std::min(c0 + q, edge)});
+                    rl.count = (int)P.r0_jobs.size() - rl.first;
+                }
                 P.r0_launches.push_back(rl);
                 continue;
             }
@@ -524,7 +540,7 @@ int build_plan(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int
 // an SM: kernels of a few hundred large CTAs start normally (early 512-thread finalizes 128x64 4.61 against
 // 4.21 ms, early tile kernels 16x750 17.1 against 16.2, early long tile products 256x256 737 against 709).
 template <class... P, class... A>
-void launch_chain(const bpmax_ctx *ctx, bool early, dim3 grid, int threads, size_t smem, cudaStream_t s, void (*kernel)(P...), A... args)
+void launch_chain(bool early, dim3 grid, int threads, size_t smem, cudaStream_t s, void (*kernel)(P...), A... args)
 {
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -535,7 +551,7 @@ void launch_chain(const bpmax_ctx *ctx, bool early, dim3 grid, int threads, size
     c.dynamicSmemBytes = smem;
     c.stream = s;
     c.attrs = &at;
-    c.numAttrs = early && ctx->one_chain ? 1 : 0;
+    c.numAttrs = early ? 1 : 0;
     cudaLaunchKernelEx(&c, kernel, P(args)...);
 }
 
@@ -544,7 +560,7 @@ void launch_r0_wide_t(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
 {
     const int grid = std::min(L.count, L.cap > 0 ? L.cap : std::max(1, ctx->wide_occ[STAGES]) * ctx->sms);
     launch_chain(
-        ctx, L.count <= 4 * grid, grid, WideCfg<STAGES>::THREADS, WideCfg<STAGES>::SMEM, s, r0_wide_kernel<STAGES>, (const R0JobW *)ctx->r0wjobs.p + L.first, L.count, (const PairDesc *)ctx->pairs.p, (float *)ctx->F.p, L.d,
+        ctx->one_chain && L.count <= 4 * grid, grid, WideCfg<STAGES>::THREADS, WideCfg<STAGES>::SMEM, s, r0_wide_kernel<STAGES>, (const R0JobW *)ctx->r0wjobs.p + L.first, L.count, (const PairDesc *)ctx->pairs.p, (float *)ctx->F.p, L.d,
         wait_ctl(ctx));
 }
 
@@ -571,12 +587,12 @@ int launch_fin_tiles(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
         const int parts = tiles < ctx->sms ? std::min(slabs, (2 * ctx->sms + tiles - 1) / tiles) : 1;
         const bool split = parts > 1;
         if (split) {
-            launch_chain(ctx, false, dim3(tiles, parts), TILE_THREADS, TILE_SMEM, s, tile_product_kernel, jobs, pairs, F, S, L.d, t,
+            launch_chain(false, dim3(tiles, parts), TILE_THREADS, TILE_SMEM, s, tile_product_kernel, jobs, pairs, F, S, L.d, t,
                          NT);
             ++n;
         }
         const int s1_ctas = t == 0 ? (L.s1_count + TILE_THREADS / 32 - 1) / (TILE_THREADS / 32) : 0;
-        launch_chain(ctx, false, tiles + s1_ctas, TILE_THREADS, TILE_SMEM, s, tile_final_kernel, jobs, L.count, s1jobs, L.s1_count,
+        launch_chain(false, tiles + s1_ctas, TILE_THREADS, TILE_SMEM, s, tile_final_kernel, jobs, L.count, s1jobs, L.s1_count,
                      pairs, F, S, (const uint8_t *)ctx->bases.p, ctx->W, L.d, t, NT, !split);
         ++n;
     }
@@ -589,7 +605,7 @@ void launch_r0_v(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
     using C = R0Cfg<NB, V>;
     // resident CTAs (or the class's share of them); each loops over jobs
     const int grid = std::min(L.count, L.cap > 0 ? L.cap : std::max(1, ctx->r0_occ_v[V][NB]) * ctx->sms);
-    launch_chain(ctx, true, grid, C::THREADS, C::SMEM, s, r0_kernel<NB, V>, (const R0Job *)ctx->r0jobs.p + L.first, L.count,
+    launch_chain(ctx->one_chain, grid, C::THREADS, C::SMEM, s, r0_kernel<NB, V>, L.jobs(ctx->r0jobs.p), L.count,
                  (const PairDesc *)ctx->pairs.p, (float *)ctx->F.p, L.d, wait_ctl(ctx));
 }
 
@@ -597,7 +613,7 @@ template <int NB>
 void launch_strip(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
 {
     launch_chain(
-        ctx, true, std::min(L.count, L.cap), StripCfg<NB>::THREADS, StripCfg<NB>::SMEM, s, r0_strip_kernel<NB>, (const StripJob *)ctx->stripjobs.p + L.first, L.count, (const PairDesc *)ctx->pairs.p, (float *)ctx->F.p, L.d,
+        ctx->one_chain, std::min(L.count, L.cap), StripCfg<NB>::THREADS, StripCfg<NB>::SMEM, s, r0_strip_kernel<NB>, (const StripJob *)ctx->stripjobs.p + L.first, L.count, (const PairDesc *)ctx->pairs.p, (float *)ctx->F.p, L.d,
         wait_ctl(ctx));
 }
 
@@ -625,7 +641,7 @@ void launch_fin_t(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
 {
     using Sh = FinShape<8 * NB, T>;
     launch_chain(
-        ctx, T < 512, L.count + (L.s1_count + Sh::WARPS - 1) / Sh::WARPS, Sh::THREADS, Sh::SMEM, s, finalize_small_kernel<8 * NB, T>,
+        ctx->one_chain && T < 512, L.count + (L.s1_count + Sh::WARPS - 1) / Sh::WARPS, Sh::THREADS, Sh::SMEM, s, finalize_small_kernel<8 * NB, T>,
         (const CellJob *)ctx->celljobs.p + L.first, L.count, (const CellJob *)ctx->celljobs.p + L.s1_first, L.s1_count,
         (const PairDesc *)ctx->pairs.p, (float *)ctx->F.p, (float *)ctx->S.p, (const uint8_t *)ctx->bases.p, ctx->W,
         L.d, ctx->plan.ref);
@@ -645,16 +661,16 @@ void launch_r0only_fin(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
     const float *vals = (const float *)ctx->r0vals.p;
     switch (L.np > MAX_SMALL_NP ? 0 : L.np / 8) {
     case 0:
-        launch_chain(ctx, true, dim3(L.count, L.np / 64), 256, 0, s, r0only_finalize_tile_kernel, jobs, pd, (float *)ctx->F.p, vals, L.d);
+        launch_chain(ctx->one_chain, dim3(L.count, L.np / 64), 256, 0, s, r0only_finalize_tile_kernel, jobs, pd, (float *)ctx->F.p, vals, L.d);
         break;
-    case 1: launch_chain(ctx, true, L.count, 128, 0, s, r0only_finalize_small_kernel<8>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
-    case 2: launch_chain(ctx, true, L.count, 128, 0, s, r0only_finalize_small_kernel<16>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
-    case 3: launch_chain(ctx, true, L.count, 128, 0, s, r0only_finalize_small_kernel<24>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
-    case 4: launch_chain(ctx, true, L.count, 128, 0, s, r0only_finalize_small_kernel<32>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
-    case 5: launch_chain(ctx, true, L.count, 128, 0, s, r0only_finalize_small_kernel<40>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
-    case 6: launch_chain(ctx, true, L.count, 128, 0, s, r0only_finalize_small_kernel<48>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
-    case 7: launch_chain(ctx, true, L.count, 128, 0, s, r0only_finalize_small_kernel<56>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
-    default: launch_chain(ctx, true, L.count, 128, 0, s, r0only_finalize_small_kernel<64>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
+    case 1: launch_chain(ctx->one_chain, L.count, 128, 0, s, r0only_finalize_small_kernel<8>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
+    case 2: launch_chain(ctx->one_chain, L.count, 128, 0, s, r0only_finalize_small_kernel<16>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
+    case 3: launch_chain(ctx->one_chain, L.count, 128, 0, s, r0only_finalize_small_kernel<24>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
+    case 4: launch_chain(ctx->one_chain, L.count, 128, 0, s, r0only_finalize_small_kernel<32>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
+    case 5: launch_chain(ctx->one_chain, L.count, 128, 0, s, r0only_finalize_small_kernel<40>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
+    case 6: launch_chain(ctx->one_chain, L.count, 128, 0, s, r0only_finalize_small_kernel<48>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
+    case 7: launch_chain(ctx->one_chain, L.count, 128, 0, s, r0only_finalize_small_kernel<56>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
+    default: launch_chain(ctx->one_chain, L.count, 128, 0, s, r0only_finalize_small_kernel<64>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
     }
 }
 
@@ -755,10 +771,10 @@ int enqueue_fill(bpmax_ctx *ctx, Plan &P, KernelProfile *kp = nullptr)
             if (P.pairs[p].Np > S2_ONE_CTA_NP)
                 for (int d = 4; d < P.pairs[p].N; ++d, ++launches)
                     launch_chain(
-                        ctx, true, (P.pairs[p].N - d + 7) / 8, 256, 0, ctx->stream, s2_diag_kernel, (const PairDesc *)ctx->pairs.p, p, (const uint8_t *)ctx->bases.p, (float *)ctx->S.p, ctx->W, d);
+                        ctx->one_chain, (P.pairs[p].N - d + 7) / 8, 256, 0, ctx->stream, s2_diag_kernel, (const PairDesc *)ctx->pairs.p, p, (const uint8_t *)ctx->bases.p, (float *)ctx->S.p, ctx->W, d);
         launches += 1;
         if (P.classes.back() > MAX_SMALL_NP) {
-            launch_chain(ctx, true, dim3(64, (int)P.pairs.size()), 256, 0, ctx->stream, s2_aux_kernel,
+            launch_chain(ctx->one_chain, dim3(64, (int)P.pairs.size()), 256, 0, ctx->stream, s2_aux_kernel,
                          (const PairDesc *)ctx->pairs.p, (float *)ctx->S.p);
             launches += 1;
         }
@@ -1694,16 +1710,6 @@ __global__ void noalloc_prep_kernel(const int *__restrict__ seqs, int M, int N, 
     }
 }
 
-// product jobs of diagonal d: pair chunk c of q offset pairs for every cell (i1, i1+d), ordered by
-// chunk then cell, as the context path orders them
-__global__ void noalloc_r0_jobs_kernel(R0Job *__restrict__ jobs, int cells, int d, int q, int njobs)
-{
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= njobs) return;
-    const int P2 = (d + 1) / 2, c = t / cells, i1 = t % cells;
-    jobs[t] = R0Job{0, i1, c * q, min(c * q + q, P2)};
-}
-
 template <int NB>
 int noalloc_set_attr(int *occ)
 {
@@ -1748,17 +1754,17 @@ int noalloc_setup(int dev, NoallocDevice *out)
 }
 
 template <int NB>
-void noalloc_launch_diag(cudaStream_t s, const NoallocDevice &nd, int d, int n_r0, int n_cells, const R0Job *rj,
+void noalloc_launch_diag(cudaStream_t s, const NoallocDevice &nd, int d, const R0Jobs &rj, int n_r0, int n_cells,
                          const CellJob *cj, const PairDesc *pd, float *F, float *S, const uint8_t *bases, const Weights &W,
                          int *err)
 {
     if (d > 0)
-        r0_kernel<NB><<<std::min(n_r0, std::max(1, nd.occ[NB]) * nd.sms), R0Cfg<NB>::THREADS, R0Cfg<NB>::SMEM, s>>>(
-            rj, n_r0, pd, F, d, WaitCtl{err, NOALLOC_WAIT_NS, 0});
+        launch_chain(true, std::min(n_r0, std::max(1, nd.occ[NB]) * nd.sms), R0Cfg<NB>::THREADS, R0Cfg<NB>::SMEM, s,
+                     r0_kernel<NB>, rj, n_r0, pd, F, d, WaitCtl{err, NOALLOC_WAIT_NS, 0});
     const int n_s1 = n_cells - 1;  // S1 cells of diagonal d+1: the first n_cells-1 entries of cj
     using Sh = FinShape<8 * NB>;
-    finalize_small_kernel<8 * NB><<<n_cells + (n_s1 + Sh::WARPS - 1) / Sh::WARPS, Sh::THREADS, Sh::SMEM, s>>>(
-        cj, n_cells, cj, n_s1, pd, F, S, bases, W, d, RefOut{nullptr, 0, 0});
+    launch_chain(Sh::THREADS < 512, n_cells + (n_s1 + Sh::WARPS - 1) / Sh::WARPS, Sh::THREADS, Sh::SMEM, s,
+                 finalize_small_kernel<8 * NB>, cj, n_cells, cj, n_s1, pd, F, S, bases, W, d, RefOut{nullptr, 0, 0});
 }
 
 }  // namespace
@@ -1797,7 +1803,8 @@ extern "C" int bpmax_gpu_score_noalloc(const int *seq1, long M, const int *seq2,
     if (st) return st;
     const long long resident = (long long)std::max(1, nd.occ[nb]) * nd.sms;
     const int qmin = std::max(1, (R0_TAB_ITEMS[nb] + 1) / 2);
-    // jobs per diagonal <= M * ceil(P2 / qmin) <= M * ((M + 1) / 2)
+    // (room for the longest job list of a diagonal, M * ceil(P2 / qmin): the documented size limits count
+    // it, the jobs themselves are computed in the kernel)
     const long long off_rj = off_cj + align64(2LL * M);
     const long long max_jobs = (long long)M * (((M + 1) / 2 + qmin - 1) / qmin);
     const long long total = off_rj + 4LL * max_jobs;
@@ -1812,7 +1819,6 @@ extern "C" int bpmax_gpu_score_noalloc(const int *seq1, long M, const int *seq2,
     float *dscore = base + off_score;
     int *derr = reinterpret_cast<int *>(base + off_score + 1);
     CellJob *cj = reinterpret_cast<CellJob *>(base + off_cj);
-    R0Job *rj = reinterpret_cast<R0Job *>(base + off_rj);
     PairDesc pd{};
     pd.M = (int)M;
     pd.N = (int)N;
@@ -1841,21 +1847,20 @@ extern "C" int bpmax_gpu_score_noalloc(const int *seq1, long M, const int *seq2,
     for (int d = 0; d < (int)M; ++d) {
         const int cells = (int)M - d;
         int n_r0 = 0;
+        R0Jobs rj{nullptr, cells, 1, (d + 1) / 2};
         if (d > 0) {
-            const long long P2 = (d + 1) / 2;
-            const long long q = r0_pairs_per_job(cells, P2, resident, qmin, 1 << 20, 2);
-            n_r0 = (int)(cells * ((P2 + q - 1) / q));
-            noalloc_r0_jobs_kernel<<<(n_r0 + 255) / 256, 256, 0, s>>>(rj, cells, d, (int)q, n_r0);
+            rj.q = (int)r0_pairs_per_job(cells, rj.pairs, resident, qmin, 1 << 20, 2);
+            n_r0 = cells * ((rj.pairs + rj.q - 1) / rj.q);
         }
         switch (nb) {
-        case 1: noalloc_launch_diag<1>(s, nd, d, n_r0, cells, rj, cj, pdp, F, S, bases, W, derr); break;
-        case 2: noalloc_launch_diag<2>(s, nd, d, n_r0, cells, rj, cj, pdp, F, S, bases, W, derr); break;
-        case 3: noalloc_launch_diag<3>(s, nd, d, n_r0, cells, rj, cj, pdp, F, S, bases, W, derr); break;
-        case 4: noalloc_launch_diag<4>(s, nd, d, n_r0, cells, rj, cj, pdp, F, S, bases, W, derr); break;
-        case 5: noalloc_launch_diag<5>(s, nd, d, n_r0, cells, rj, cj, pdp, F, S, bases, W, derr); break;
-        case 6: noalloc_launch_diag<6>(s, nd, d, n_r0, cells, rj, cj, pdp, F, S, bases, W, derr); break;
-        case 7: noalloc_launch_diag<7>(s, nd, d, n_r0, cells, rj, cj, pdp, F, S, bases, W, derr); break;
-        default: noalloc_launch_diag<8>(s, nd, d, n_r0, cells, rj, cj, pdp, F, S, bases, W, derr); break;
+        case 1: noalloc_launch_diag<1>(s, nd, d, rj, n_r0, cells, cj, pdp, F, S, bases, W, derr); break;
+        case 2: noalloc_launch_diag<2>(s, nd, d, rj, n_r0, cells, cj, pdp, F, S, bases, W, derr); break;
+        case 3: noalloc_launch_diag<3>(s, nd, d, rj, n_r0, cells, cj, pdp, F, S, bases, W, derr); break;
+        case 4: noalloc_launch_diag<4>(s, nd, d, rj, n_r0, cells, cj, pdp, F, S, bases, W, derr); break;
+        case 5: noalloc_launch_diag<5>(s, nd, d, rj, n_r0, cells, cj, pdp, F, S, bases, W, derr); break;
+        case 6: noalloc_launch_diag<6>(s, nd, d, rj, n_r0, cells, cj, pdp, F, S, bases, W, derr); break;
+        case 7: noalloc_launch_diag<7>(s, nd, d, rj, n_r0, cells, cj, pdp, F, S, bases, W, derr); break;
+        default: noalloc_launch_diag<8>(s, nd, d, rj, n_r0, cells, cj, pdp, F, S, bases, W, derr); break;
         }
     }
     gather_scores_kernel<<<1, 32, 0, s>>>(pdp, F, 1, dscore);

@@ -55,6 +55,19 @@ struct R0Job {
     int pair, i1, p0, p1;
 };
 
+// the jobs of one launch: a list, or (list == nullptr) those of one pair's diagonal by arithmetic, ordered
+// as a list would be: chunks of q of the `pairs` offset pairs, and within a chunk the `cells` cells
+struct R0Jobs {
+    const R0Job *list;
+    int cells, q, pairs;
+    __device__ __forceinline__ R0Job operator[](int j) const
+    {
+        if (list) return list[j];
+        const int c = j / cells;
+        return R0Job{0, j - c * cells, c * q, min(c * q + q, pairs)};
+    }
+};
+
 __host__ __device__ __forceinline__ int r0_job_items(const R0Job &j, int d)
 {
     const int P = (d + 1) / 2;
@@ -241,7 +254,7 @@ __device__ __forceinline__ void r0_task(const float *__restrict__ As, const floa
 
 template <int NB, int V = 0>
 __global__ void __launch_bounds__(R0Cfg<NB, V>::THREADS, R0Cfg<NB, V>::MINB)
-r0_kernel(const R0Job *__restrict__ jobs, int njobs, const PairDesc *__restrict__ pairs, float *__restrict__ F, int d,
+r0_kernel(R0Jobs jobs, int njobs, const PairDesc *__restrict__ pairs, float *__restrict__ F, int d,
           WaitCtl ctl)
 {
     using C = R0Cfg<NB, V>;
