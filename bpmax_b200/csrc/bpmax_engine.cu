@@ -103,14 +103,15 @@ struct Plan {
     long long F_floats = 0, S_floats = 0;
     int bases_bytes = 0;
     int maxM = 0;
-    // per diagonal and Np class (index NB-1): ranges in the job arrays
-    // np = inner table width class; strip (product launches): strips of diagonals d .. d+T-1
+    // per step and Np class: ranges in the job arrays. d = the step: the outer diagonal, for tile tables the
+    // outer diagonal plus the tile diagonal. np = inner table width class; strip (product launches): strips of diagonals d .. d+T-1
     // cap: at most this many CTAs (0: as many as are resident), from the class shares
     // r0_kernel launches of one pair: q offset pairs per job of `edge` (0: jobs from the list)
     struct Launch {
         int d, np, first, count, s1_first = 0, s1_count = 0;
         bool strip = false;
         int cap = 0, cells = 0, q = 0, edge = 0;
+        int tile_first = 0, tile_count = 0;  // finalize launches of tile tables: the tiles (count: cells)
         R0Jobs jobs(const void *list) const
         {
             return q ? R0Jobs{nullptr, cells, q, edge} : R0Jobs{(const R0Job *)list + first, 0, 0, 0};
@@ -120,6 +121,8 @@ struct Plan {
     std::vector<R0Job> r0_jobs;
     std::vector<StripJob> strip_jobs;  // jobs of strip launches (first/count index this array)
     std::vector<R0JobW> r0w_jobs;  // jobs of launches with tile-image tables (first/count index this array)
+    std::vector<TileJob> tile_jobs;
+    int steps = 0;  // of the fill: outer diagonals, and the tile diagonals after the last
     std::vector<CellJob> cell_jobs;
     std::vector<int> classes;  // distinct inner widths, ascending
     int pairs_per_job = 0, merge_items = 0, class_streams = 1;  // tunables the plan was built with
@@ -153,7 +156,7 @@ struct bpmax_ctx {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     Weights W;
     std::string err;
-    DevBuf F, S, bases, pairs, r0jobs, stripjobs, r0wjobs, celljobs, scores, conv, tbstack, grads, tbstatus, errflag;
+    DevBuf F, S, bases, pairs, r0jobs, stripjobs, r0wjobs, tilejobs, celljobs, scores, conv, tbstack, grads, tbstatus, errflag;
     DevBuf r0vals;         // R0-only mode: seq1 then seq2 of the pair, as floats
     DevBuf pq, pcnt, pneed;  // persistent fill: work queue; counters (class heads, diagonals, cells); jobs per cell
     bool copyout = false;    // the next fill copies the reference layout out per diagonal (graph path)
@@ -336,6 +339,64 @@ void build_queue(bpmax_ctx *ctx, Plan &P)
     }
 }
 
+// Launches of one step of the tile tables of width np: tile diagonal t of outer diagonal d with d + t = step
+// (the R0-only mode keeps to outer diagonals: step = d, every tile)
+void build_tile_step(bpmax_ctx *ctx, Plan &P, int np, int step, long long resident, bool uncapped)
+{
+    const int NT = np / 64, n = (int)P.pairs.size();
+    // jobs: one per output tile of a cell and chunk of k1 offset pairs, and per chunk of the 2t terms over
+    // finished tiles, sized so that jobs cost about the same: cost per offset pair in warp task steps
+    // of both of its items, DD 3.3, DA and DB 12, F 16 per item
+    auto pair_cost = [](int t) { return t == 0 ? 2 * 3.3 : 2 * (24.0 + 16.0 * (t - 1)); };
+    auto each = [&](auto &&f) {  // (pair, d, t) of the step
+        for (int p = 0; p < n; ++p)
+            if (P.pairs[p].Np == np)
+                for (int t = ctx->r0_only ? 0 : std::max(0, step - P.pairs[p].M + 1); t < NT; ++t) {
+                    const int d = ctx->r0_only ? step : step - t;
+                    if (d >= 0 && d < P.pairs[p].M) f(p, d, t);
+                }
+    };
+    double total = 0;
+    Plan::Launch fl{step, np, (int)P.cell_jobs.size(), 0};
+    fl.tile_first = (int)P.tile_jobs.size();
+    each([&](int p, int d, int t) {
+        const double tiles = (double)(P.pairs[p].M - d) * (NT - t);
+        total += tiles * ((d + 1) / 2 * pair_cost(t) + (ctx->r0_only ? 0.0 : 2.0 * t * 16.0));
+    });
+    const double target = std::max(total / (3.0 * resident), 4.0 * 16.0);
+    const size_t first = P.r0w_jobs.size();
+    for (int T = NT - 1; T >= 0; --T)  // heavy tiles first
+        each([&](int p, int d, int t) {
+            if (t != T) return;
+            const int P2 = (d + 1) / 2, cells = P.pairs[p].M - d;
+            const int q = std::max(1, (int)std::min<long long>(P2, std::llround(target / pair_cost(t))));
+            const int qs = std::max(1, (int)std::min<long long>(2 * t, std::llround(target / 16.0)));
+            for (int I = 0; I + t < NT; ++I) {
+                if (!ctx->r0_only)
+                    for (int n0 = 0; n0 < 2 * t; n0 += qs)
+                        for (int i1 = 0; i1 < cells; ++i1)
+                            P.r0w_jobs.push_back(R0JobW{p, i1, d, I << 8 | (I + t), -1 - n0, std::min(n0 + qs, 2 * t)});
+                for (int c0 = 0; c0 < P2; c0 += q)
+                    for (int i1 = 0; i1 < cells; ++i1)
+                        P.r0w_jobs.push_back(R0JobW{p, i1, d, I << 8 | (I + t), c0, std::min(c0 + q, P2)});
+                if (!ctx->r0_only)
+                    for (int i1 = 0; i1 < cells; ++i1) P.tile_jobs.push_back(TileJob{p, i1, d, I << 8 | (I + t)});
+            }
+        });
+    // jobs of the same offset pairs together (both uses of a table meet in L2), heavy tiles first
+    std::stable_sort(P.r0w_jobs.begin() + first, P.r0w_jobs.end(),
+                     [](const R0JobW &a, const R0JobW &b) { return std::max(a.p0, -1) < std::max(b.p0, -1); });
+    Plan::Launch wl{step, np, (int)first, (int)(P.r0w_jobs.size() - first)};
+    wl.cap = uncapped ? 0 : (int)resident;
+    if (wl.count > 0) P.r0_launches.push_back(wl);
+    for (int p = 0; p < n; ++p)  // the cells of outer diagonal `step` (S1; the finalize of the R0-only mode)
+        if (P.pairs[p].Np == np && P.pairs[p].M > step)
+            for (int i1 = 0; i1 < P.pairs[p].M - step; ++i1) P.cell_jobs.push_back(CellJob{p, i1});
+    fl.count = (int)P.cell_jobs.size() - fl.first;
+    fl.tile_count = (int)P.tile_jobs.size() - fl.tile_first;
+    if (fl.count > 0 || fl.tile_count > 0) P.fin_launches.push_back(fl);
+}
+
 int build_plan(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int> &Ns, Plan &P)
 {
     P = Plan();
@@ -374,10 +435,8 @@ int build_plan(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int
         s = align64(s + (long long)Ms[p] * Ms[p]);
         pd.S2_off = s;
         s = align64(s + (long long)pd.Np * pd.Np);
-        if (pd.Np > MAX_SMALL_NP) {  // copies of S2 read by the tile finalize
+        if (pd.Np > MAX_SMALL_NP) {  // S2 as tile images
             pd.S2x_off = s;
-            s = align64(s + (long long)pd.Np * pd.Np);
-            pd.S2y_off = s;
             s = align64(s + (long long)pd.Np * pd.Np);
         }
         pd.seq1_off = b;
@@ -419,8 +478,15 @@ int build_plan(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int
         return it == share.end() ? resident : std::max(1LL, (long long)std::llround(resident * it->second));
     };
     // jobs, grouped by diagonal then inner width class
-    for (int d = 0; d < P.maxM; ++d) {
+    const int NTmax = classes.back() > MAX_SMALL_NP && !ctx->r0_only ? classes.back() / 64 : 1;
+    P.steps = P.maxM + NTmax - 1;
+    for (int d = 0; d < P.steps; ++d) {
         for (int np : classes) {
+            if (np > MAX_SMALL_NP) {
+                build_tile_step(ctx, P, np, d, capped(np, (long long)std::max(1, ctx->wide_occ[P.wide_stages]) * ctx->sms),
+                                share.empty());
+                continue;
+            }
             long long cells = 0;
             for (int p = 0; p < n; ++p)
                 if (P.pairs[p].Np == np && Ms[p] > d) cells += Ms[p] - d;
@@ -432,7 +498,7 @@ int build_plan(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int
             fl.count = (int)P.cell_jobs.size() - fl.first;
             P.fin_launches.push_back(fl);
             if (d == 0) continue;
-            if (np <= MAX_SMALL_NP) {
+            {
                 // Strips of T cells (bpmax_strip.cuh), once per T diagonals d .. d+T-1 (d = 1 mod T): the
                 // offsets [T-1, d-1], which read only diagonals < d for every cell of a strip. The T-1
                 // offset pairs (w, d-1-w) at the ends of every cell's range are the jobs of r0_kernel,
@@ -495,38 +561,6 @@ int build_plan(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int
                 P.r0_launches.push_back(rl);
                 continue;
             }
-            // tile images: one job per output tile (BI, BJ) of a cell and chunk of k1 offset pairs,
-            // each tile's chunk sized so that jobs cost about the same: cost per offset pair in
-            // warp task steps of both of its items, DD 3.3, DA and DB 12, F 16 per item
-            const int NT = np / 64;
-            const long long P2 = (d + 1) / 2;
-            const long long resident = capped(np, (long long)std::max(1, ctx->wide_occ[P.wide_stages]) * ctx->sms);
-            std::vector<std::pair<double, int>> tiles;  // (cost per offset pair, BI << 8 | BJ)
-            double per_pair = 0;
-            for (int BI = 0; BI < NT; ++BI)
-                for (int BJ = BI; BJ < NT; ++BJ) {
-                    const double c = BI == BJ ? 2 * 3.3 : 2 * (24.0 + 16.0 * (BJ - BI - 1));
-                    tiles.push_back({c, BI << 8 | BJ});
-                    per_pair += c;
-                }
-            std::stable_sort(tiles.begin(), tiles.end(), [](const auto &a, const auto &b) { return a.first > b.first; });
-            const double total = (double)cells * P2 * per_pair;
-            const double target = std::max(total / (3.0 * resident), 4.0 * 16.0);
-            const size_t first = P.r0w_jobs.size();
-            for (const auto &t : tiles) {
-                const long long q = std::max(1LL, std::min(P2, (long long)std::llround(target / t.first)));
-                for (long long c0 = 0; c0 < P2; c0 += q)
-                    for (int p = 0; p < n; ++p)
-                        if (P.pairs[p].Np == np && Ms[p] > d)
-                            for (int i1 = 0; i1 < Ms[p] - d; ++i1)
-                                P.r0w_jobs.push_back(R0JobW{p, i1, t.second, (int)c0, (int)std::min(c0 + q, P2)});
-            }
-            // jobs of the same offset pairs together (both uses of a table meet in L2), heavy tiles first
-            std::stable_sort(P.r0w_jobs.begin() + first, P.r0w_jobs.end(),
-                             [](const R0JobW &a, const R0JobW &b) { return a.p0 < b.p0; });
-            Plan::Launch wl{d, np, (int)first, (int)(P.r0w_jobs.size() - first)};
-            wl.cap = share.empty() ? 0 : (int)resident;
-            P.r0_launches.push_back(wl);
         }
     }
     // S1 of diagonal d+1 is computed by the finalize launch of diagonal d (same class)
@@ -546,7 +580,7 @@ int build_plan(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int
 // other's room). That hides the launch and the first loads of a short kernel (37x23 0.53 -> 0.35 ms,
 // 200x8 2.42 -> 1.52, 128x32 2.44 -> 1.97), but places its CTAs where room comes free first, several to
 // an SM: kernels of a few hundred large CTAs start normally (early 512-thread finalizes 128x64 4.61 against
-// 4.21 ms, early tile kernels 16x750 17.1 against 16.2, early long tile products 256x256 737 against 709).
+// 4.21 ms, early tile kernels 90x70 9.36 against 8.85, early tile products 256x256 737 against 709).
 template <class... P, class... A>
 void launch_chain(bool early, dim3 grid, int threads, size_t smem, cudaStream_t s, void (*kernel)(P...), A... args)
 {
@@ -568,8 +602,8 @@ void launch_r0_wide_t(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
 {
     const int grid = std::min(L.count, L.cap > 0 ? L.cap : std::max(1, ctx->wide_occ[STAGES]) * ctx->sms);
     launch_chain(
-        ctx->one_chain && L.count <= 4 * grid, grid, WideCfg<STAGES>::THREADS, WideCfg<STAGES>::SMEM, s, r0_wide_kernel<STAGES>, (const R0JobW *)ctx->r0wjobs.p + L.first, L.count, (const PairDesc *)ctx->pairs.p, (float *)ctx->F.p, L.d,
-        wait_ctl(ctx));
+        false, grid, WideCfg<STAGES>::THREADS, WideCfg<STAGES>::SMEM, s, r0_wide_kernel<STAGES>, (const R0JobW *)ctx->r0wjobs.p + L.first, L.count, (const PairDesc *)ctx->pairs.p, (float *)ctx->F.p,
+        (const float *)ctx->S.p, wait_ctl(ctx));
 }
 
 void launch_r0_wide(bpmax_ctx *ctx, const Plan &P, const Plan::Launch &L, cudaStream_t s)
@@ -580,31 +614,13 @@ void launch_r0_wide(bpmax_ctx *ctx, const Plan &P, const Plan::Launch &L, cudaSt
         launch_r0_wide_t<2>(ctx, L, s);
 }
 
-// the finalize of one launch of cells wider than 64: one launch per tile diagonal t, with the slabs of
-// its tiles in a launch of their own where few tiles hold many; returns the number of kernel launches
-int launch_fin_tiles(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
+// the tiles of one step, and S1 of outer diagonal step+1
+void launch_fin_tiles(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
 {
-    const CellJob *jobs = (const CellJob *)ctx->celljobs.p + L.first;
-    const CellJob *s1jobs = (const CellJob *)ctx->celljobs.p + L.s1_first;
-    const PairDesc *pairs = (const PairDesc *)ctx->pairs.p;
-    float *F = (float *)ctx->F.p, *S = (float *)ctx->S.p;
-    const int NT = L.np / 64;
-    int n = 0;
-    for (int t = 0; t < NT; ++t) {
-        const int tiles = L.count * (NT - t), slabs = 2 * t;
-        const int parts = tiles < ctx->sms ? std::min(slabs, (2 * ctx->sms + tiles - 1) / tiles) : 1;
-        const bool split = parts > 1;
-        if (split) {
-            launch_chain(false, dim3(tiles, parts), TILE_THREADS, TILE_SMEM, s, tile_product_kernel, jobs, pairs, F, S, L.d, t,
-                         NT);
-            ++n;
-        }
-        const int s1_ctas = t == 0 ? (L.s1_count + TILE_THREADS / 32 - 1) / (TILE_THREADS / 32) : 0;
-        launch_chain(false, tiles + s1_ctas, TILE_THREADS, TILE_SMEM, s, tile_final_kernel, jobs, L.count, s1jobs, L.s1_count,
-                     pairs, F, S, (const uint8_t *)ctx->bases.p, ctx->W, L.d, t, NT, !split);
-        ++n;
-    }
-    return n;
+    launch_chain(false, L.tile_count + (L.s1_count + TILE_THREADS / 32 - 1) / (TILE_THREADS / 32), TILE_THREADS, TILE_SMEM, s,
+                 tile_final_kernel, (const TileJob *)ctx->tilejobs.p + L.tile_first, L.tile_count,
+                 (const CellJob *)ctx->celljobs.p + L.s1_first, L.s1_count, (const PairDesc *)ctx->pairs.p, (float *)ctx->F.p,
+                 (float *)ctx->S.p, (const uint8_t *)ctx->bases.p, ctx->W, L.d);
 }
 
 template <int NB, int V>
@@ -707,7 +723,7 @@ int set_smem_attr(bpmax_ctx *ctx)
     }
     if (NB == 8)
         if ((st = prefer_smem(ctx, r0_wide_kernel<2>)) || (st = prefer_smem(ctx, r0_wide_kernel<3>)) ||
-            (st = prefer_smem(ctx, tile_product_kernel)) || (st = prefer_smem(ctx, tile_final_kernel)))
+            (st = prefer_smem(ctx, tile_final_kernel)))
             return st;
     CK(cudaFuncSetAttribute(r0_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)R0Cfg<NB>::SMEM));
     CK(cudaFuncSetAttribute(r0_kernel<NB, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)R0Cfg<NB, 1>::SMEM));
@@ -729,7 +745,6 @@ int set_smem_attr(bpmax_ctx *ctx)
         CK(cudaFuncSetAttribute(r0_wide_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WideCfg<3>::SMEM));
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctx->wide_occ[2], r0_wide_kernel<2>, 128, WideCfg<2>::SMEM));
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctx->wide_occ[3], r0_wide_kernel<3>, 128, WideCfg<3>::SMEM));
-        CK(cudaFuncSetAttribute(tile_product_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TILE_SMEM));
         CK(cudaFuncSetAttribute(tile_final_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TILE_SMEM));
     }
     return BPMAX_OK;
@@ -843,7 +858,9 @@ int enqueue_fill(bpmax_ctx *ctx, Plan &P, KernelProfile *kp = nullptr)
         for (int k = 0; k < nstreams; ++k) CK(cudaStreamWaitEvent(ctx->class_stream[k], ctx->fork_ev, 0));
     }
     size_t ri = 0, fi = 0;
-    for (int d = 0; d < P.maxM; ++d) {
+    // outer diagonal final after step d (tile tables: with its last tile diagonal)
+    const int lag = P.classes.back() > MAX_SMALL_NP && !P.r0_only ? P.classes.back() / 64 - 1 : 0;
+    for (int d = 0; d < P.steps; ++d) {
         for (; ri < P.r0_launches.size() && P.r0_launches[ri].d == d; ++ri, ++launches) {
             const auto &L = P.r0_launches[ri];
             const cudaStream_t st = stream_of(L.np);
@@ -871,7 +888,7 @@ int enqueue_fill(bpmax_ctx *ctx, Plan &P, KernelProfile *kp = nullptr)
                     launch_r0only_fin(ctx, L, st);
                 } else {
                     switch (L.np > MAX_SMALL_NP ? 0 : L.np / 8) {
-                    case 0: launches += launch_fin_tiles(ctx, L, st) - 1; break;
+                    case 0: launch_fin_tiles(ctx, L, st); break;
                     case 1: launch_fin<1>(ctx, L, st); break;
                     case 2: launch_fin<2>(ctx, L, st); break;
                     case 3: launch_fin<3>(ctx, L, st); break;
@@ -886,8 +903,8 @@ int enqueue_fill(bpmax_ctx *ctx, Plan &P, KernelProfile *kp = nullptr)
         }
         // outer diagonal d is final: rows of the reference layout that end on it can be copied out
         // (events recorded as external nodes of the captured graph; eager runs record none)
-        if (!P.diag_ev.empty() && !prof && P.diag_ev[d])
-            CK(cudaEventRecordWithFlags(P.diag_ev[d], ctx->stream, capturing ? cudaEventRecordExternal : cudaEventRecordDefault));
+        if (!P.diag_ev.empty() && !prof && d >= lag && P.diag_ev[d - lag])
+            CK(cudaEventRecordWithFlags(P.diag_ev[d - lag], ctx->stream, capturing ? cudaEventRecordExternal : cudaEventRecordDefault));
     }
     for (int k = 0; k < nstreams; ++k) {  // join the class chains back into the main stream
         CK(cudaEventRecord(ctx->join_ev[k], ctx->class_stream[k]));
@@ -940,6 +957,7 @@ int prepare(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int> &
         if ((st = ensure(ctx, ctx->r0jobs, P.r0_jobs.size() * sizeof(R0Job))) != BPMAX_OK) return st;
         if ((st = ensure(ctx, ctx->stripjobs, P.strip_jobs.size() * sizeof(StripJob))) != BPMAX_OK) return st;
         if ((st = ensure(ctx, ctx->r0wjobs, P.r0w_jobs.size() * sizeof(R0JobW))) != BPMAX_OK) return st;
+        if ((st = ensure(ctx, ctx->tilejobs, P.tile_jobs.size() * sizeof(TileJob))) != BPMAX_OK) return st;
         if (P.persistent) {
             if ((st = ensure(ctx, ctx->pq, P.pitems.size() * sizeof(PItem))) != BPMAX_OK) return st;
             if ((st = ensure(ctx, ctx->pneed, P.prod_need.size() * sizeof(int))) != BPMAX_OK) return st;
@@ -961,6 +979,9 @@ int prepare(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int> &
         if (!P.r0w_jobs.empty())
             CK(cudaMemcpyAsync(ctx->r0wjobs.p, P.r0w_jobs.data(), P.r0w_jobs.size() * sizeof(R0JobW), cudaMemcpyHostToDevice,
                                ctx->stream));
+        if (!P.tile_jobs.empty())
+            CK(cudaMemcpyAsync(ctx->tilejobs.p, P.tile_jobs.data(), P.tile_jobs.size() * sizeof(TileJob),
+                               cudaMemcpyHostToDevice, ctx->stream));
         CK(cudaMemcpyAsync(ctx->celljobs.p, P.cell_jobs.data(), P.cell_jobs.size() * sizeof(CellJob), cudaMemcpyHostToDevice, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
         ctx->plan_valid = true;
@@ -1238,7 +1259,7 @@ void bpmax_gpu_destroy(bpmax_ctx *ctx)
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     if (ctx->plan.graph) cudaGraphExecDestroy(ctx->plan.graph);
     for (DevBuf *b : {&ctx->tbstack, &ctx->grads, &ctx->tbstatus, &ctx->F, &ctx->S, &ctx->bases, &ctx->pairs,
-                      &ctx->r0jobs, &ctx->stripjobs, &ctx->r0wjobs, &ctx->pq, &ctx->pcnt, &ctx->pneed, &ctx->celljobs,
+                      &ctx->r0jobs, &ctx->stripjobs, &ctx->r0wjobs, &ctx->tilejobs, &ctx->pq, &ctx->pcnt, &ctx->pneed, &ctx->celljobs,
                       &ctx->scores, &ctx->conv, &ctx->refdev, &ctx->errflag,
                       &ctx->r0vals})
         if (b->p) cudaFree(b->p);

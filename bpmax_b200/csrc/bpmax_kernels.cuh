@@ -49,8 +49,7 @@ struct PairDesc {
     long long F_off;   // float offset of F[0]
     long long S1_off;  // float offset of S1 in the S arena
     long long S2_off;  // float offset of S2 in the S arena
-    long long S2x_off; // Np > 64 only: dense tile images of S2(i, k-1) (bpmax_tile.cuh)
-    long long S2y_off; // Np > 64 only: dense tile images of S2(k+1, j)
+    long long S2x_off; // Np > 64 only: dense tile images of S2 (bpmax_tile.cuh)
     int seq1_off;      // offset of seq1 in the base arena (uint8)
     int seq2_off;      // offset of the REVERSED seq2 in the base arena (uint8)
     long long cell_base;  // persistent fill: index of the pair's cell (0, 0) among all pairs' cells

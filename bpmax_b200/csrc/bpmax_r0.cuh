@@ -201,14 +201,13 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // pair p = (2p, 2p+1) only for rows i <= 2p+2, since A[i][k] = -inf for k < i-1; ROLE 2 (shifted B
 // block on the diagonal, kb == bj) evaluates k pair p only for column pairs jp >= p, since
 // Bs[k][j] = -inf for k > j; ROLE 3 (both blocks on the diagonal) applies both limits. The
-// skipped candidates are all -inf, so the maxima are unchanged. SHIFTED: Bs points at the row-shifted
-// block, whose row 7 lies past the spare chunk; otherwise at a block of rows 0..7.
+// skipped candidates are all -inf, so the maxima are unchanged.
 template <int ROLE>
 __device__ __forceinline__ bool r0_pair_used(int i, int jp, int p)
 {
     return ((ROLE & 1) == 0 || i <= 2 * p + 2) && ((ROLE & 2) == 0 || jp >= p);
 }
-template <int ROLE, bool SHIFTED = true>
+template <int ROLE>
 __device__ __forceinline__ void r0_task(const float *__restrict__ As, const float *__restrict__ Bs, float (&acc)[8][8])
 {
 #pragma unroll
@@ -216,7 +215,7 @@ __device__ __forceinline__ void r0_task(const float *__restrict__ As, const floa
         float2 bv[4][4];  // bv[k][jp] = (Bs[4q+k][2jp], Bs[4q+k][2jp+1])
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const int row = 4 * q + k, ro = 8 * row + (SHIFTED && row == 7 ? 4 : 0);  // row 7: next block / S1 piece
+            const int row = 4 * q + k, ro = 8 * row + (row == 7 ? 4 : 0);  // row 7: next block / S1 piece
             if (r0_pair_used<ROLE>(0, 0, 2 * q + k / 2) || r0_pair_used<ROLE>(0, 1, 2 * q + k / 2)) {  // row 0 widest
                 const float4 t0 = *reinterpret_cast<const float4 *>(Bs + ro);
                 bv[k][0] = make_float2(t0.x, t0.y); bv[k][1] = make_float2(t0.z, t0.w);

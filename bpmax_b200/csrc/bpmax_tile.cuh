@@ -1,16 +1,17 @@
 // bpmax_tile.cuh -- finalize of inner tables stored as tile images (Np = 64 * NT > 64, layout in
-// bpmax_kernels.cuh), by tile diagonals over the whole GPU.
+// bpmax_kernels.cuh), by tiles over the whole GPU.
 //
 // Tile (I, J) of a cell's table F (rows 64I.., columns 64J..) needs, beside its start values,
 //   R1  F[i2][k] + S2(k+1, j2), k in [i2, j2): k < 64J lies in the finished tiles (I, K), K < J;
 //       k >= 64J in the tile itself
 //   R2  S2(i2, k-1) + F[k][j2], k in (i2, j2]: k >= 64(I+1) lies in the finished tiles (K, J), K > I;
 //       k < 64(I+1) in the tile itself
-// so the tiles go by tile diagonal t = J - I. The terms over finished tiles are max-plus products of
-// 64x64 tile images: R1 slabs F(I, K) (x) S2Y(K, J), K = I .. J-1, and R2 slabs S2X(I, K) (x) F(K, J),
-// K = I+1 .. J, where the images S2Y[k][j] = S2(k+1, j) and S2X[i][k] = S2(i, k-1) (K < J, dense) hold
-// the shift. (F's diagonal tiles hold S1 on their subdiagonal: the term it gives is S1 + S2, a
-// candidate of the entry anyway.) The tile's own terms follow by 8x8 blocks, block diagonal by block
+// and the product R0+R3+R4 of the tile needs only tiles of other cells that lie at most as many tile
+// diagonals t = J - I up. So tile diagonal t of outer diagonal d runs in step d + t, beside the earlier tile
+// diagonals of later outer diagonals: M + NT - 1 steps of two launches, r0_wide_kernel (the products of
+// the step's tiles, and the terms over finished tiles as items of the same kind) and tile_final_kernel
+// (one CTA per tile of the step: start values, SW1, the tile's own terms, the tile image).
+// The tile's own terms go by 8x8 blocks, block diagonal by block
 // diagonal, one warp per block: first the terms over the finished blocks of the tile as products, four
 // lanes sharing the k of an 8-entry piece, then the block's own wavefront over its 15 diagonals in
 // registers, one row per lane and one shuffle per step. S2 is 0 on spans <= 3, so inside a block an
@@ -18,43 +19,34 @@
 // four diagonals back), SW2, and what lies five to seven columns left or rows below. The candidates
 // of neighbours outside a block or tile are in the products; SW2 from outside is read where it lies.
 //
-// tile_final_kernel does all of it for one tile per CTA, one launch per tile diagonal of every cell of
-// an outer diagonal (launch boundaries are the only barriers); where a launch has few tiles and many
-// slabs, tile_product_kernel spreads the slabs over more CTAs first and merges into F.
-//
 // Bound: latency of a tile's own terms (a tile of t >= 1 takes 26 us alone on an SM: 10 us in 15 block
-// diagonals of products, 11 us in their wavefronts, 5 us of loads), FP32 issue of the slabs (13,000
-// cycles each, two CTAs per SM). Finalize ms of a whole fill, before (one CTA per cell walking every inner
-// diagonal up to width 320; above, row-major tables with a barrier per tile diagonal) and now: 90x130
-// 16.9 -> 9.9, 256x256 316 -> 77, 16x750 36.3 -> 10.6, 32x1024 120 -> 46. Tried for the tile's own terms:
-// batches of five tile diagonals pushed to all later entries, 26 at 61 us a tile (the pushes of four
-// columns a step cost 2,800 cycles a batch); 512 and 1,024 threads a tile, no faster.
+// diagonals of products, 11 us in their wavefronts, 5 us of loads). Fill ms with one CTA per cell
+// walking every inner diagonal (up to width 320; above, row-major tables with a barrier per tile
+// diagonal) / with the tile diagonals of one outer diagonal after another, the terms over finished tiles
+// in launches of their own / in steps as here: 90x130 32.0 / 24.1 / 19.1,
+// 256x256 950 / 709 / 698, 16x750 47.6 / 16.9 / 9.9, 32x1024 238 / 110 / 83.
+// Tried for the tile's own terms: batches of five tile diagonals pushed to all later entries, 61 us a
+// tile (the pushes took 2,800 cycles a batch); 512 and 1,024 threads a tile, no faster.
 #pragma once
-#include "bpmax_r0.cuh"
+#include "bpmax_wide.cuh"
 
 namespace bpmax {
 
 constexpr int TILE_THREADS = 256;
 constexpr int TILE_LD = 68;  // row pitch of the tile and of the S2 blocks in shared memory: 17 16-byte chunks
-// one slab operand (a dense image) and the shared memory of the tile kernels: the tile, then two
-// stages of two operands, which later hold the merge tile or the two S2 blocks
-constexpr int TILE_SLOT = 16 * WIDE_DENSE_CHUNKS;
-// the tile: 64 rows, after 4 words and before one row of -inf; the pad columns of a row are -inf too, so
-// column -1 (the pad before the row), columns 64.. and row 64 may be read
-constexpr int TILE_OFF_SLAB = 4 * (65 * TILE_LD + 8);
-constexpr size_t TILE_SMEM = TILE_OFF_SLAB + 4 * TILE_SLOT;
-static_assert(4 * 65 * 64 <= 2 * TILE_SLOT && 2 * 4 * 64 * TILE_LD <= 4 * TILE_SLOT, "aliased regions");
-static_assert(2 * (TILE_SMEM + 1024) <= 228 * 1024, "two CTAs per SM");
+// shared memory: the tile (64 rows, after 4 words and before one row of -inf; the pad columns of a row
+// are -inf too, so column -1, the pad before the row, columns 64.. and row 64 may be read), the S2 blocks
+constexpr int TILE_OFF_S2 = 4 * (65 * TILE_LD + 8);
+constexpr size_t TILE_SMEM = TILE_OFF_S2 + 2 * 4 * 64 * TILE_LD;
 
-// index of the dense tile (I, J), I < J, among the shifted S2 images of a pair
-__host__ __device__ __forceinline__ long long s2_image_off(int NT, int I, int J)
-{
-    return ((long long)I * (NT - 1) - (long long)I * (I - 1) / 2 + (J - I - 1)) * (4LL * WIDE_DENSE_CHUNKS);
-}
+// tile (I, J) (tile = I << 8 | J) of the table of cell (i1, i1+d) of pair `pair`
+struct TileJob {
+    int pair, i1, d, tile;
+};
 
 // ------------------------------------------------------------------------------------------
-// The shifted images S2X, S2Y (above) of every pair with Np > 64, S2 over the reversed strand 2
-// (V3/bpmax_verify.c:560-571); -inf where a row or column is >= N.
+// The dense tile images (with halo pieces) of S2 of every pair with Np > 64, S2 over the reversed strand
+// 2 (V3/bpmax_verify.c:560-571); -inf in columns >= N.
 // ------------------------------------------------------------------------------------------
 __global__ void s2_aux_kernel(const PairDesc *__restrict__ pairs, float *__restrict__ S)
 {
@@ -63,15 +55,13 @@ __global__ void s2_aux_kernel(const PairDesc *__restrict__ pairs, float *__restr
     chain_wait();
     if (Np <= 64) return;
     const float *S2 = S + pd.S2_off;
-    float *S2X = S + pd.S2x_off, *S2Y = S + pd.S2y_off;
+    float *img = S + pd.S2x_off;
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < (long long)Np * Np;
          q += (long long)gridDim.x * blockDim.x) {
-        const int r = (int)(q / Np), c = (int)(q % Np), I = r >> 6, J = c >> 6;
-        if (I < J) {
-            const int o = 4 * (c_wide_dense_colbase[(c & 63) >> 3] + 17 * ((r & 63) >> 3)) + 8 * (r & 7) + (c & 7);
-            S2X[s2_image_off(NT, I, J) + o] = c - 1 < N ? S2[(long long)r * Np + c - 1] : NEG_INF;
-            S2Y[s2_image_off(NT, I, J) + o] = c < N ? S2[(long long)(r + 1) * Np + c] : NEG_INF;
-        }
+        const int r = (int)(q / Np), c = (int)(q % Np), I = r >> 6, J = c >> 6, o = 4 * c_wide_dense_colbase[(c & 63) >> 3];
+        const float v = c < N ? S2[q] : NEG_INF;
+        if (I < J) img[s2_image_off(NT, I, J) + o + 4 * 17 * ((r & 63) >> 3) + 8 * (r & 7) + (c & 7)] = v;
+        if ((r & 63) == 0 && I > 0 && I <= J) img[s2_image_off(NT, I - 1, J) + o + 4 * 17 * 8 + (c & 7)] = v;
     }
 }
 
@@ -79,7 +69,7 @@ __global__ void s2_aux_kernel(const PairDesc *__restrict__ pairs, float *__restr
 // S2 of one pair with Np > S2_ONE_CTA_NP, one launch per diagonal d of its wavefront
 // (single_strand_kernel's one CTA per pair took 2.2 s at N = 3000), one warp per cell. The column
 // operand S2(k+1, j) is read from ST[j][k], which the same launches fill as cells become final (in the
-// room of the shifted images, which s2_aux_kernel writes afterwards); S starts at 0, so ST holds the 0
+// room of the images, which s2_aux_kernel writes afterwards); S starts at 0, so ST holds the 0
 // of every cell with j-i <= 3.
 // ------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
@@ -131,122 +121,33 @@ __device__ __forceinline__ void s1_cell(const CellJob &job, const PairDesc *__re
     if (lane == 0) S1[i * M + j] = fmaxf(S1[(i + 1) * M + (j - 1)] + score_w(w, s1[i], s1[j]), red);
 }
 
-// The slabs [s0, s1) of tile (I, I+t), all threads: slab s < t is R1 with K = I+s, the others R2
-// with K = I+1+(s-t). Thread (tid & 127) has the micro-tile (bi, bj) of the wide product's lane table,
-// and TILE_THREADS/64 threads share a micro-tile's k blocks. The result (0 where no candidate is above 0) is left
-// in the merge tile `red`, blocks of 8x8 in row-major order at a pitch of 65 words.
-__device__ __forceinline__ void tile_slabs(char *sm, const float *Fc, const float *S2X, const float *S2Y, int NT, int I,
-                                           int t, int s0, int s1)
-{
-    const int tid = threadIdx.x, J = I + t;
-    auto load = [&](int s) {
-        char *st = sm + TILE_OFF_SLAB + ((s - s0) & 1) * 2 * TILE_SLOT;
-        const bool r1 = s < t;
-        const int K = r1 ? I + s : I + 1 + (s - t);
-        const float *A = r1 ? Fc + wide_tile_off(NT, I, K) : S2X + s2_image_off(NT, I, K);
-        const float *B = r1 ? S2Y + s2_image_off(NT, K, J) : Fc + wide_tile_off(NT, K, J);
-        const int na = r1 && K == I ? WIDE_DIAG_CHUNKS : WIDE_DENSE_CHUNKS;
-        const int nb = !r1 && K == J ? WIDE_DIAG_CHUNKS : WIDE_DENSE_CHUNKS;
-        for (int q = tid; q < na; q += TILE_THREADS) cp_async16(st + 16 * q, A + 4 * q);
-        for (int q = tid; q < nb; q += TILE_THREADS) cp_async16(st + TILE_SLOT + 16 * q, B + 4 * q);
-        cp_async_commit();
-    };
-    const unsigned char *lt = c_tile_lane[tid & 127];
-    const int bi = lt[0], bj = lt[1], h = lt[2] + 2 * (tid >> 7);
-    float acc[8][8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = NEG_INF;
-    load(s0);
-#pragma unroll 1
-    for (int s = s0; s < s1; ++s) {
-        if (s + 1 < s1) {
-            load(s + 1);
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
-        __syncthreads();
-        const float *As = reinterpret_cast<const float *>(sm + TILE_OFF_SLAB + ((s - s0) & 1) * 2 * TILE_SLOT);
-        const float *Bs = As + TILE_SLOT / 4;
-        const bool a_diag = s == 0, b_diag = s == 2 * t - 1;  // F(I, I) and F(J, J): upper block triangles
-        const int hi = b_diag ? bj : 7;
-#pragma unroll 1
-        for (int kb = (a_diag ? bi : 0) + h; kb <= hi; kb += TILE_THREADS / 64)
-            r0_task<0, false>(As + 4 * ((a_diag ? c_img_colbase[8][kb] : c_wide_dense_colbase[kb]) + 17 * bi),
-                              Bs + 4 * ((b_diag ? c_img_colbase[8][bj] : c_wide_dense_colbase[bj]) + 17 * kb), acc);
-        __syncthreads();  // the stage may be overwritten
-    }
-    int *red = reinterpret_cast<int *>(sm + TILE_OFF_SLAB);
-    for (int q = tid; q < 65 * 64; q += TILE_THREADS) red[q] = 0;
-    __syncthreads();
-    int *rb = red + 65 * (8 * bi + bj);
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int v = __float_as_int(acc[i][j]);
-            if (v > 0) atomicMax(rb + 8 * i + j, v);
-        }
-    __syncthreads();
-}
-
-// word offset of element (r, c) of the merge tile
-__device__ __forceinline__ int tile_red_off(int r, int c) { return 65 * (8 * (r >> 3) + (c >> 3)) + 8 * (r & 7) + (c & 7); }
-
-// grid ((NT - t) * cells, Z): part blockIdx.y of Z of the slabs of tile (I, I+t), merged into F
+// CTAs [0, njobs): one tile each; after them one warp per S1 cell (i, i+step+1)
 __global__ void __launch_bounds__(TILE_THREADS, 2)
-tile_product_kernel(const CellJob *__restrict__ jobs, const PairDesc *__restrict__ pairs, float *__restrict__ F,
-                    const float *__restrict__ S, int d, int t, int NT)
-{
-    extern __shared__ __align__(16) float tsm[];
-    char *sm = reinterpret_cast<char *>(tsm);
-    const int nt = NT - t, I = (int)blockIdx.x % nt, J = I + t;
-    const CellJob job = jobs[blockIdx.x / nt];
-    const PairDesc pd = pairs[job.pair];
-    float *Fc = F + pd.F_off + cell_index(pd.M, job.i1, job.i1 + d) * wide_cell_floats(NT);
-    const int Z = gridDim.y, z = blockIdx.y, s0 = 2 * t * z / Z, s1 = 2 * t * (z + 1) / Z;
-    chain_wait();
-    if (s0 == s1) return;
-    tile_slabs(sm, Fc, S + pd.S2x_off, S + pd.S2y_off, NT, I, t, s0, s1);
-    const int *red = reinterpret_cast<const int *>(sm + TILE_OFF_SLAB);
-    int *out = reinterpret_cast<int *>(Fc + wide_tile_off(NT, I, J));
-    for (int q = threadIdx.x; q < 4096; q += TILE_THREADS) {  // consecutive lanes, consecutive words of a block
-        const int b = q >> 6, x = q & 63, v = red[65 * b + x];
-        if (v > 0) atomicMax(out + 4 * (c_wide_dense_colbase[b & 7] + 17 * (b >> 3)) + x, v);
-    }
-}
-
-// CTAs [0, ncells * (NT - t)): tile (I, I+t) of the outer cells of diagonal d; after them (t = 0), one
-// warp per S1 cell (i, i+d+1). fused: the slabs of the tile are computed here; otherwise
-// tile_product_kernel has merged them into F.
-__global__ void __launch_bounds__(TILE_THREADS, 2)
-tile_final_kernel(const CellJob *__restrict__ jobs, int ncells, const CellJob *__restrict__ s1jobs, int ns1,
+tile_final_kernel(const TileJob *__restrict__ jobs, int njobs, const CellJob *__restrict__ s1jobs, int ns1,
                   const PairDesc *__restrict__ pairs, float *__restrict__ F, float *__restrict__ S,
-                  const uint8_t *__restrict__ bases, Weights W, int d, int t, int NT, bool fused)
+                  const uint8_t *__restrict__ bases, Weights W, int step)
 {
     constexpr int LD = TILE_LD;
     extern __shared__ __align__(16) float tsm[];
-    char *sm = reinterpret_cast<char *>(tsm);
     float *T = tsm + 4;
     __shared__ float wsh[12], w5[25];
     __shared__ __align__(16) float wt[5 * LD];  // wt[LD*x + c]: weight of base x and column c of the tile
     __shared__ uint8_t bI[64], bJ[64];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nt = NT - t;
+    __shared__ float below[64], s2r_end[64];  // F[64(I+1)][64J+c] and S2(64I+r, 64I+63)
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid < 12) wsh[tid] = W.w[tid];
     if (tid >= 32 && tid < 57) w5[tid - 32] = score_w(W.w, (tid - 32) / 5, (tid - 32) % 5);
-    if ((int)blockIdx.x >= ncells * nt) {
+    if ((int)blockIdx.x >= njobs) {
         __syncthreads();
-        const int q = ((int)blockIdx.x - ncells * nt) * (TILE_THREADS / 32) + warp;
+        const int q = ((int)blockIdx.x - njobs) * (TILE_THREADS / 32) + warp;
         chain_wait();
-        if (q < ns1) s1_cell(s1jobs[q], pairs, S, bases, wsh, d, lane);
+        if (q < ns1) s1_cell(s1jobs[q], pairs, S, bases, wsh, step, lane);
         return;
     }
-    const int I = (int)blockIdx.x % nt, J = I + t;
-    const CellJob job = jobs[blockIdx.x / nt];
+    const TileJob job = jobs[blockIdx.x];
+    const int I = job.tile >> 8, J = job.tile & 0xff, t = J - I, d = job.d;
     const PairDesc pd = pairs[job.pair];
-    const int M = pd.M, N = pd.N, Np = pd.Np, i1 = job.i1, j1 = i1 + d;
+    const int M = pd.M, N = pd.N, Np = pd.Np, NT = Np >> 6, i1 = job.i1, j1 = i1 + d;
     const int ncol = min(64, N - 64 * J);  // columns of the tile inside the table
     const long long CELL = wide_cell_floats(NT);
     float *Fc = F + pd.F_off + cell_index(M, i1, j1) * CELL;
@@ -260,16 +161,19 @@ tile_final_kernel(const CellJob *__restrict__ jobs, int ncells, const CellJob *_
     const int x1 = s1[i1], y1 = s1[j1];
     chain_wait();
     const float s1v = S[pd.S1_off + i1 * M + j1];
-    if (fused && t > 0)
-        tile_slabs(sm, Fc, S + pd.S2x_off, S + pd.S2y_off, NT, I, t, 0, 2 * t);
-    else
-        __syncthreads();
-    // start values: accumulated products, S1+S2, SW1 (F(i1+1,j1-1,.)+intra if j1-i1 >= 4), the slabs; the
+    // row 0 of the tile below: the halo pieces, and with the last column of S2's block I the one k of R2
+    // between this tile and the finished ones, S2(i2, 64I+63) + F[64(I+1)][j2]
+    const float *Fb = t > 0 ? Fc + wide_tile_off(NT, I + 1, J) : nullptr;
+    if (t > 0 && tid < 64)
+        below[tid] = Fb[4 * (t == 1 ? c_img_colbase[8][tid >> 3] : c_wide_dense_colbase[tid >> 3]) + (tid & 7)];
+    else if (t > 0 && tid < 128)
+        s2r_end[tid - 64] = S2[(long long)(64 * I + tid - 64) * Np + 64 * I + 63];
+    __syncthreads();
+    // start values: accumulated products, S1+S2, SW1 (F(i1+1,j1-1,.)+intra if j1-i1 >= 4); the
     // inter-strand base on the diagonal of the diagonal cells. Entries outside the table stay -inf.
     const bool sw1 = d >= 4;
     const float w1 = sw1 ? score_w(wsh, x1, y1) : 0.0f;
     const float *Fi = F + pd.F_off + (sw1 ? cell_index(M, i1 + 1, j1 - 1) * CELL : 0) + wide_tile_off(NT, I, J);
-    const float *red = tsm + TILE_OFF_SLAB / 4;
     const int nblk = t == 0 ? 36 : 64;
     for (int q = tid - 4; q < 65 * LD; q += TILE_THREADS)
         if (t == 0 || q < 0 || q % LD >= ncol || q >= 64 * LD) T[q] = NEG_INF;
@@ -308,7 +212,7 @@ tile_final_kernel(const CellJob *__restrict__ jobs, int ncells, const CellJob *_
             const int c = c0 + u;
             if (c < ncol && (t > 0 || r <= c)) {
                 float v = fmax3(fv[u], s1v + sv[u], pv[u] + w1);
-                if (fused && t > 0) v = fmaxf(v, red[tile_red_off(r, c)]);
+                if (t > 0) v = fmaxf(v, s2r_end[r] + below[c]);
                 if (d == 0 && t == 0 && r == c) v = score_w(wsh + 6, x1, bI[r]);
                 T[r * LD + c] = v;
             }
@@ -325,8 +229,7 @@ tile_final_kernel(const CellJob *__restrict__ jobs, int ncells, const CellJob *_
     }
     // S2 inside the tile's row block and column block: SX[x][y] = S2(64I+x, 64I+y-1) (y > x),
     // SJ[x][y] = S2(64J+x, 64J+y), -inf in columns outside the table
-    float *SX = tsm + TILE_OFF_SLAB / 4, *SJ = SX + 64 * LD;
-    __syncthreads();  // the merge tile has been read
+    float *SX = tsm + TILE_OFF_S2 / 4, *SJ = SX + 64 * LD;
 #pragma unroll
     for (int q = tid; q < 1024; q += TILE_THREADS) {
         const int x = q >> 4, y = 4 * (q & 15);
@@ -410,7 +313,7 @@ tile_final_kernel(const CellJob *__restrict__ jobs, int ncells, const CellJob *_
         float cx[3];  // S2(i2, i2+4 ..) for R2 from rows five to seven below, inside the block
 #pragma unroll
         for (int x = 0; x < 3; ++x) cx[x] = la + x + 5 < 8 ? SX[row * LD + row + 5 + x] : NEG_INF;
-        float n[15], below = NEG_INF, left = NEG_INF, diag = NEG_INF;  // (row+1, b), (row, b-1), (row+1, b-1)
+        float n[15], under = NEG_INF, left = NEG_INF, diag = NEG_INF;  // (row+1, b), (row, b-1), (row+1, b-1)
 #pragma unroll
         for (int s = 0; s < 15; ++s) {
             const int b = s - 7 + la;
@@ -423,13 +326,13 @@ tile_final_kernel(const CellJob *__restrict__ jobs, int ncells, const CellJob *_
                     const float r2 = __shfl_down_sync(0xffffffffu, n[s - 5 - x], 5 + x, 8) + cx[x];
                     far = fmax3(far, r1, r2);
                 }
-            below = s > 0 ? __shfl_down_sync(0xffffffffu, n[s - 1], 1, 8) : NEG_INF;
-            if (la == 7) below = NEG_INF;
+            under = s > 0 ? __shfl_down_sync(0xffffffffu, n[s - 1], 1, 8) : NEG_INF;
+            if (la == 7) under = NEG_INF;
             const float q = la == 7 ? qs[s < 8 ? s : 7] : (b == 0 ? qs[0] : diag);
-            const float r = fmaxf(fmax3(fmaxf(vs[s], far), left, below), q + ws[s]);
+            const float r = fmaxf(fmax3(fmaxf(vs[s], far), left, under), q + ws[s]);
             n[s] = b >= 0 && b < 8 && 8 * bj + b < ncol ? r : NEG_INF;
             if (lane < 8 && b >= 0 && b < 8 && 8 * bj + b < ncol) T[row * LD + 8 * bj + b] = n[s];
-            diag = below;
+            diag = under;
             left = n[s];
         }
     }
@@ -443,8 +346,8 @@ tile_final_kernel(const CellJob *__restrict__ jobs, int ncells, const CellJob *_
             if (t == 0) {
                 if (h == 1) v.w = s1v;
             } else {
-                v = *reinterpret_cast<const float4 *>(Fc + wide_tile_off(NT, I + 1, J) + 4 * h +
-                                                      4 * (t == 1 ? c_img_colbase[8][bj] : c_wide_dense_colbase[bj]));
+                v = make_float4(below[8 * bj + 4 * h], below[8 * bj + 4 * h + 1], below[8 * bj + 4 * h + 2],
+                                below[8 * bj + 4 * h + 3]);
             }
             *reinterpret_cast<float4 *>(Ft + 4 * ((t == 0 ? c_img_colbase[8][bj] + 17 * (bj + 1)
                                                           : c_wide_dense_colbase[bj] + 17 * 8) + h)) = v;

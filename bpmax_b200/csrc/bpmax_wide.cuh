@@ -24,10 +24,22 @@
 
 namespace bpmax {
 
+// float offset of the dense tile (I, J), I < J, among the S2 images of a pair
+__host__ __device__ __forceinline__ long long s2_image_off(int NT, int I, int J)
+{
+    return ((long long)I * (NT - 1) - (long long)I * (I - 1) / 2 + (J - I - 1)) * (4LL * WIDE_DENSE_CHUNKS);
+}
+
+// R1 and R2 over finished tiles of the cell itself are items of the same form: S2 is the table of an
+// empty strand-1 interval, so R1 is A = tile (BI, KB) of F(i1, j1), B = tile (KB, BJ) of S2, KB = BI .. BJ-1,
+// and R2 is A = tile (BI, KB) of S2, B = tile (KB, BJ) of F(i1, j1), KB = BI+1 .. BJ (S2 as dense tile
+// images with halo pieces; the one k between the two, 64(BI+1)-1 of R2, is left to tile_final_kernel).
+//
 // one job: output tile (BI, BJ) (tile = BI << 8 | BJ) of cell (i1, i1+d) of pair `pair`, k1 offset
-// pairs p in [p0, p1) (offsets w = p and d-1-p, as R0Job)
+// pairs p in [p0, p1) (offsets w = p and d-1-p, as R0Job); with p0 < 0 the R1/R2 items n in [-1-p0, p1),
+// the BJ-BI of R1 first
 struct R0JobW {
-    int pair, i1, tile, p0, p1;
+    int pair, i1, d, tile, p0, p1;
 };
 
 // Shape variants: STAGES = 2 keeps three CTAs per SM (168 registers), 3 two CTAs per SM.
@@ -50,7 +62,7 @@ struct WideCfg {
 template <int STAGES>
 __global__ void __launch_bounds__(128, WideCfg<STAGES>::MINB)
 r0_wide_kernel(const R0JobW *__restrict__ jobs, int njobs, const PairDesc *__restrict__ pairs, float *__restrict__ F,
-               int d, WaitCtl ctl)
+               const float *__restrict__ Sa, WaitCtl ctl)
 {
     using C = WideCfg<STAGES>;
     constexpr int S = STAGES;
@@ -73,13 +85,14 @@ r0_wide_kernel(const R0JobW *__restrict__ jobs, int njobs, const PairDesc *__res
 
     const unsigned smem_base = smem_u32(wsm);
     auto job_items = [&](const R0JobW &jb) {
-        return r0_job_items(R0Job{jb.pair, jb.i1, jb.p0, jb.p1}, d) * ((jb.tile & 0xff) - (jb.tile >> 8) + 1);
+        if (jb.p0 < 0) return jb.p1 + 1 + jb.p0;
+        return r0_job_items(R0Job{jb.pair, jb.i1, jb.p0, jb.p1}, jb.d) * ((jb.tile & 0xff) - (jb.tile >> 8) + 1);
     };
     // the producer's current job and its pair's M, Np and F_off, one copy per warp in shared memory,
     // refreshed when the warp's producer position moves to another job (as in r0_kernel: no
     // dependent global loads per refill)
     __shared__ R0JobW pjob_sh[C::WARPS];
-    __shared__ long long pfoff_sh[C::WARPS];
+    __shared__ long long pfoff_sh[C::WARPS], ps2_sh[C::WARPS];
     __shared__ int pm_sh[C::WARPS], pnp_sh[C::WARPS];
     const int warp_id = tid >> 5;
     auto load_pjob = [&](int j_) {
@@ -90,6 +103,7 @@ r0_wide_kernel(const R0JobW *__restrict__ jobs, int njobs, const PairDesc *__res
             pm_sh[warp_id] = pairs[jb.pair].M;
             pnp_sh[warp_id] = pairs[jb.pair].Np;
             pfoff_sh[warp_id] = pairs[jb.pair].F_off;
+            ps2_sh[warp_id] = pairs[jb.pair].S2x_off;
         }
         __syncwarp();
     };
@@ -98,20 +112,37 @@ r0_wide_kernel(const R0JobW *__restrict__ jobs, int njobs, const PairDesc *__res
     auto fill_stage = [&](int s, int n) {
         const R0JobW jb = pjob_sh[warp_id];
         const int M = pm_sh[warp_id];
-        const int BI = jb.tile >> 8, BJ = jb.tile & 0xff, nkb = BJ - BI + 1, KB = BI + n % nkb, NT = pnp_sh[warp_id] >> 6;
-        const int k1 = jb.i1 + r0_item_offset(R0Job{jb.pair, jb.i1, jb.p0, jb.p1}, d, n / nkb);
-        const int j1 = jb.i1 + d;
+        const int BI = jb.tile >> 8, BJ = jb.tile & 0xff, NT = pnp_sh[warp_id] >> 6;
+        const int j1 = jb.i1 + jb.d;
         const long long CELL = wide_cell_floats(NT);
-        const float *Fp = F + pfoff_sh[warp_id];
+        const float *Fp = F + pfoff_sh[warp_id], *A, *B;
+        int ab = 16 * WIDE_DENSE_CHUNKS, bb = ab;
+        if (jb.p0 >= 0) {
+            const int nkb = BJ - BI + 1, KB = BI + n % nkb;
+            const int k1 = jb.i1 + r0_item_offset(R0Job{jb.pair, jb.i1, jb.p0, jb.p1}, jb.d, n / nkb);
+            A = Fp + cell_index(M, jb.i1, k1) * CELL + wide_tile_off(NT, BI, KB);
+            B = Fp + cell_index(M, k1 + 1, j1) * CELL + wide_tile_off(NT, KB, BJ);
+            if (KB == BI) ab = 16 * WIDE_DIAG_CHUNKS;
+            if (KB == BJ) bb = 16 * WIDE_DIAG_CHUNKS;
+        } else {
+            const int m = n - 1 - jb.p0, t = BJ - BI;
+            const float *Fc = Fp + cell_index(M, jb.i1, j1) * CELL, *S2 = Sa + ps2_sh[warp_id];
+            if (m < t) {
+                A = Fc + wide_tile_off(NT, BI, BI + m);
+                B = S2 + s2_image_off(NT, BI + m, BJ);
+                if (m == 0) ab = 16 * WIDE_DIAG_CHUNKS;
+            } else {
+                A = S2 + s2_image_off(NT, BI, BI + 1 + m - t);
+                B = Fc + wide_tile_off(NT, BI + 1 + m - t, BJ);
+                if (m == 2 * t - 1) bb = 16 * WIDE_DIAG_CHUNKS;
+            }
+        }
         const unsigned bar = smem_u32(bars + s);
-        const int ab = 16 * (KB == BI ? WIDE_DIAG_CHUNKS : WIDE_DENSE_CHUNKS);
-        const int bb = 16 * (KB == BJ ? WIDE_DIAG_CHUNKS : WIDE_DENSE_CHUNKS);
         mbar_arrive_tx(bar, (unsigned)(ab + bb));
         armed[s] += 1;
         const unsigned dst = smem_base + (unsigned)(s * C::STAGE_BYTES);
-        bulk_g2s(dst, Fp + cell_index(M, jb.i1, k1) * CELL + wide_tile_off(NT, BI, KB), (unsigned)ab, bar);
-        bulk_g2s(dst + 16 * C::SLOT, Fp + cell_index(M, k1 + 1, j1) * CELL + wide_tile_off(NT, KB, BJ), (unsigned)bb,
-                 bar);
+        bulk_g2s(dst, A, (unsigned)ab, bar);
+        bulk_g2s(dst + 16 * C::SLOT, B, (unsigned)bb, bar);
     };
 
     // consumer position (job jid, item it of items) and producer position S items ahead
@@ -153,10 +184,13 @@ r0_wide_kernel(const R0JobW *__restrict__ jobs, int njobs, const PairDesc *__res
     unsigned phase = 0;
     int stage = 0;
     bool bad = false;  // as in r0_kernel: a wait ran out; no more copies, leave at the next job end
-    int tile = jobs[jid].tile, kbi = 0;  // the job's output tile; k tile of the item = BI + kbi
+    // the job's output tile; k tile of the item = BI + kbi; first R1/R2 item of the job (-1: R0 items)
+    int tile = jobs[jid].tile, slab = jobs[jid].p0 < 0 ? -1 - jobs[jid].p0 : -1, kbi = 0;
 #pragma unroll 1
     while (true) {
-        const int BI = tile >> 8, BJ = tile & 0xff, KB = BI + kbi;
+        const int BI = tile >> 8, BJ = tile & 0xff;
+        if (slab >= 0) kbi = slab + it < BJ - BI ? slab + it : slab + it - (BJ - BI) + 1;
+        const int KB = BI + kbi;
         if (!bad && !mbar_wait(smem_u32(bars + stage), (phase >> stage) & 1u, ctl.wait_ns)) {
             atomicExch(ctl.err, 1);
             bad = true;
@@ -231,7 +265,7 @@ r0_wide_kernel(const R0JobW *__restrict__ jobs, int njobs, const PairDesc *__res
             const R0JobW job = jobs[jid];
             const PairDesc pd = pairs[job.pair];
             const int NT = pd.Np >> 6;
-            float *out = F + pd.F_off + cell_index(pd.M, job.i1, job.i1 + d) * wide_cell_floats(NT) +
+            float *out = F + pd.F_off + cell_index(pd.M, job.i1, job.i1 + job.d) * wide_cell_floats(NT) +
                          wide_tile_off(NT, BI, BJ);
             const int task = BI == BJ ? dd_task : mt_task;
             if (task >= 0) {
@@ -257,6 +291,7 @@ r0_wide_kernel(const R0JobW *__restrict__ jobs, int njobs, const PairDesc *__res
             const R0JobW nx = jobs[jid];
             items = job_items(nx);
             tile = nx.tile;
+            slab = nx.p0 < 0 ? -1 - nx.p0 : -1;
             it = 0;
             kbi = 0;
         }

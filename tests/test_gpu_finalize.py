@@ -46,8 +46,8 @@ def test_bulk_launches_vs_oracle(eng, oracle_mod, N):
 
 @pytest.mark.parametrize("N", [65, 66, 71, 72, 73, 96, 127, 128, 129, 137, 192, 193, 255, 320, 321, 385])
 def test_tile_tables_vs_oracle(eng, oracle_mod, N):
-    """Tables of 64x64 tiles: strand-2 lengths around whole tiles and whole 8x8 blocks. Few tiles: the
-    slabs over finished tiles run in their own launches."""
+    """Tables of 64x64 tiles: strand-2 lengths around whole tiles and whole 8x8 blocks, and fewer outer
+    diagonals than tile diagonals."""
     M = 6
     s1, s2 = W.pair(M, N, 3000 + N)
     w = W.random_weights(N) if N % 2 else W.INTEGER_WEIGHTS
@@ -60,7 +60,7 @@ def test_tile_tables_vs_oracle(eng, oracle_mod, N):
 
 @pytest.mark.parametrize("lo,hi", [(65, 128), (129, 192), (193, 200)])
 def test_tile_tables_of_many_cells_vs_oracle(eng, oracle_mod, lo, hi):
-    """More tiles in a launch than SMs: each CTA computes the slabs of its tile itself."""
+    """Many tiles of several outer diagonals, tile diagonals and pairs in one step."""
     rng = np.random.default_rng(lo)
     pairs = [(W.random_sequence(5, rng), W.random_sequence(int(rng.integers(lo, hi + 1)), rng)) for _ in range(40)]
     eng.set_weights(W.INTEGER_WEIGHTS)
