@@ -346,8 +346,13 @@ void build_tile_step(bpmax_ctx *ctx, Plan &P, int np, int step, long long reside
     const int NT = np / 64, n = (int)P.pairs.size();
     // jobs: one per output tile of a cell and chunk of k1 offset pairs, and per chunk of the 2t terms over
     // finished tiles, sized so that jobs cost about the same: cost per offset pair in warp task steps
-    // of both of its items, DD 3.3, DA and DB 12, F 16 per item
-    auto pair_cost = [](int t) { return t == 0 ? 2 * 3.3 : 2 * (24.0 + 16.0 * (t - 1)); };
+    // of both of its items, DD 3.3, DA and DB 12, F 16 per item, in a narrow last tile column less, but
+    // 5 at the least (the copies)
+    auto nbc = [&](int p, int J) { return J == NT - 1 ? (P.pairs[p].N - 64 * J + 7) / 8 : 8; };
+    auto item_cost = [&](int p, int J, double full) { return std::max(5.0, full * wide_cost(nbc(p, J)) / 16.0); };
+    auto pair_cost = [&](int p, int t, int J) {
+        return t == 0 ? 2 * 3.3 : 2 * (2 * item_cost(p, J, 12.0) + item_cost(p, J, 16.0) * (t - 1));
+    };
     auto each = [&](auto &&f) {  // (pair, d, t) of the step
         for (int p = 0; p < n; ++p)
             if (P.pairs[p].Np == np)
@@ -360,8 +365,9 @@ void build_tile_step(bpmax_ctx *ctx, Plan &P, int np, int step, long long reside
     Plan::Launch fl{step, np, (int)P.cell_jobs.size(), 0};
     fl.tile_first = (int)P.tile_jobs.size();
     each([&](int p, int d, int t) {
-        const double tiles = (double)(P.pairs[p].M - d) * (NT - t);
-        total += tiles * ((d + 1) / 2 * pair_cost(t) + (ctx->r0_only ? 0.0 : 2.0 * t * 16.0));
+        for (int J = t; J < NT; ++J)
+            total += (P.pairs[p].M - d) *
+                     ((d + 1) / 2 * pair_cost(p, t, J) + (ctx->r0_only ? 0.0 : 2.0 * t * item_cost(p, J, 16.0)));
     });
     const double target = std::max(total / (3.0 * resident), 4.0 * 16.0);
     const size_t first = P.r0w_jobs.size();
@@ -369,18 +375,19 @@ void build_tile_step(bpmax_ctx *ctx, Plan &P, int np, int step, long long reside
         each([&](int p, int d, int t) {
             if (t != T) return;
             const int P2 = (d + 1) / 2, cells = P.pairs[p].M - d;
-            const int q = std::max(1, (int)std::min<long long>(P2, std::llround(target / pair_cost(t))));
-            const int qs = std::max(1, (int)std::min<long long>(2 * t, std::llround(target / 16.0)));
             for (int I = 0; I + t < NT; ++I) {
+                const int J = I + t, tile = nbc(p, J) << 16 | I << 8 | J;
+                const int q = std::max(1, (int)std::min<long long>(P2, std::llround(target / pair_cost(p, t, J))));
+                const int qs = std::max(1, (int)std::min<long long>(2 * t, std::llround(target / item_cost(p, J, 16.0))));
                 if (!ctx->r0_only)
                     for (int n0 = 0; n0 < 2 * t; n0 += qs)
                         for (int i1 = 0; i1 < cells; ++i1)
-                            P.r0w_jobs.push_back(R0JobW{p, i1, d, I << 8 | (I + t), -1 - n0, std::min(n0 + qs, 2 * t)});
+                            P.r0w_jobs.push_back(R0JobW{p, i1, d, tile, -1 - n0, std::min(n0 + qs, 2 * t)});
                 for (int c0 = 0; c0 < P2; c0 += q)
                     for (int i1 = 0; i1 < cells; ++i1)
-                        P.r0w_jobs.push_back(R0JobW{p, i1, d, I << 8 | (I + t), c0, std::min(c0 + q, P2)});
+                        P.r0w_jobs.push_back(R0JobW{p, i1, d, tile, c0, std::min(c0 + q, P2)});
                 if (!ctx->r0_only)
-                    for (int i1 = 0; i1 < cells; ++i1) P.tile_jobs.push_back(TileJob{p, i1, d, I << 8 | (I + t)});
+                    for (int i1 = 0; i1 < cells; ++i1) P.tile_jobs.push_back(TileJob{p, i1, d, I << 8 | J});
             }
         });
     // jobs of the same offset pairs together (both uses of a table meet in L2), heavy tiles first

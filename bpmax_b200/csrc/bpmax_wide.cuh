@@ -35,12 +35,28 @@ __host__ __device__ __forceinline__ long long s2_image_off(int NT, int I, int J)
 // and R2 is A = tile (BI, KB) of S2, B = tile (KB, BJ) of F(i1, j1), KB = BI+1 .. BJ (S2 as dense tile
 // images with halo pieces; the one k between the two, 64(BI+1)-1 of R2, is left to tile_final_kernel).
 //
-// one job: output tile (BI, BJ) (tile = BI << 8 | BJ) of cell (i1, i1+d) of pair `pair`, k1 offset
+// Output tiles of the last tile column hold only nbc = ceil((N - 64 BJ) / 8) block columns of the table: their
+// jobs give every micro-tile of those columns wide_split(nbc) lanes instead of 2 and leave the rest of
+// the tile out (it is -inf), in the copies too, so a strand 2 of 130 costs little more than one of 128
+// (90x130: 16.6 -> 12.1 ms of products).
+//
+// one job: output tile (BI, BJ) (tile = nbc << 16 | BI << 8 | BJ) of cell (i1, i1+d) of pair `pair`, k1 offset
 // pairs p in [p0, p1) (offsets w = p and d-1-p, as R0Job); with p0 < 0 the R1/R2 items n in [-1-p0, p1),
 // the BJ-BI of R1 first
 struct R0JobW {
     int pair, i1, d, tile, p0, p1;
 };
+
+// lanes per micro-tile in output tiles of nbc block columns (8 nbc micro-tiles on 128 lanes), and what an
+// item of such a tile costs, in 1/16 of a full one (warps times steps of a lane)
+__host__ __device__ constexpr int wide_split(int nbc)
+{
+    return nbc <= 2 ? 8 : (nbc == 3 ? 5 : (nbc == 4 ? 4 : (nbc == 5 ? 3 : 2)));
+}
+constexpr int wide_cost(int nbc)
+{
+    return (8 * nbc * wide_split(nbc) + 31) / 32 * ((8 + wide_split(nbc) - 1) / wide_split(nbc));
+}
 
 // Shape variants: STAGES = 2 keeps three CTAs per SM (168 registers), 3 two CTAs per SM.
 template <int STAGES_>
@@ -86,72 +102,83 @@ r0_wide_kernel(const R0JobW *__restrict__ jobs, int njobs, const PairDesc *__res
     const unsigned smem_base = smem_u32(wsm);
     auto job_items = [&](const R0JobW &jb) {
         if (jb.p0 < 0) return jb.p1 + 1 + jb.p0;
-        return r0_job_items(R0Job{jb.pair, jb.i1, jb.p0, jb.p1}, jb.d) * ((jb.tile & 0xff) - (jb.tile >> 8) + 1);
+        return r0_job_items(R0Job{jb.pair, jb.i1, jb.p0, jb.p1}, jb.d) * ((jb.tile & 0xff) - (jb.tile >> 8 & 0xff) + 1);
     };
-    // the producer's current job and its pair's M, Np and F_off, one copy per warp in shared memory,
-    // refreshed when the warp's producer position moves to another job (as in r0_kernel: no
-    // dependent global loads per refill)
-    __shared__ R0JobW pjob_sh[C::WARPS];
-    __shared__ long long pfoff_sh[C::WARPS], ps2_sh[C::WARPS];
-    __shared__ int pm_sh[C::WARPS], pnp_sh[C::WARPS];
+    // the producer's current job, one copy per warp in shared memory, refreshed when the warp's producer
+    // position moves to another job (as in r0_kernel: no dependent global loads per refill). A refill is
+    // in the way of the whole ring, so its addresses take 32-bit arithmetic on these: a pair's triangle has
+    // fewer than 2^31 cells and a table fewer than 2^31 chunks.
+    struct PJob {
+        unsigned long long F, S2;  // byte addresses of the pair's tables and of its S2 images
+        unsigned cell;             // bytes of a table
+        int M, NT, i1, d, p0, tile;
+    };
+    __shared__ PJob pjob_sh[C::WARPS];
     const int warp_id = tid >> 5;
     auto load_pjob = [&](int j_) {
         __syncwarp();  // every lane of the warp is done with the previous copy
         if (lane == 0) {
             const R0JobW jb = jobs[j_];
-            pjob_sh[warp_id] = jb;
-            pm_sh[warp_id] = pairs[jb.pair].M;
-            pnp_sh[warp_id] = pairs[jb.pair].Np;
-            pfoff_sh[warp_id] = pairs[jb.pair].F_off;
-            ps2_sh[warp_id] = pairs[jb.pair].S2x_off;
+            const PairDesc *pd = pairs + jb.pair;
+            const int NT = pd->Np >> 6;
+            pjob_sh[warp_id] = PJob{(unsigned long long)(F + pd->F_off), (unsigned long long)(Sa + pd->S2x_off),
+                                    (unsigned)(4 * wide_cell_floats(NT)), pd->M, NT, jb.i1, jb.d, jb.p0, jb.tile};
         }
         __syncwarp();
     };
-    // arms stage s for item n of the producer's job (the warp's copy) and issues its two copies
-    // (one thread)
-    auto fill_stage = [&](int s, int n) {
-        const R0JobW jb = pjob_sh[warp_id];
-        const int M = pm_sh[warp_id];
-        const int BI = jb.tile >> 8, BJ = jb.tile & 0xff, NT = pnp_sh[warp_id] >> 6;
-        const int j1 = jb.i1 + jb.d;
-        const long long CELL = wide_cell_floats(NT);
-        const float *Fp = F + pfoff_sh[warp_id], *A, *B;
-        int ab = 16 * WIDE_DENSE_CHUNKS, bb = ab;
-        if (jb.p0 >= 0) {
-            const int nkb = BJ - BI + 1, KB = BI + n % nkb;
-            const int k1 = jb.i1 + r0_item_offset(R0Job{jb.pair, jb.i1, jb.p0, jb.p1}, jb.d, n / nkb);
-            A = Fp + cell_index(M, jb.i1, k1) * CELL + wide_tile_off(NT, BI, KB);
-            B = Fp + cell_index(M, k1 + 1, j1) * CELL + wide_tile_off(NT, KB, BJ);
-            if (KB == BI) ab = 16 * WIDE_DIAG_CHUNKS;
-            if (KB == BJ) bb = 16 * WIDE_DIAG_CHUNKS;
+    // arms stage s for the producer's item (k1 number pk of the job's, k tile pkb of it; R1/R2: pk) and
+    // issues its two copies (one thread)
+    auto fill_stage = [&](int s, int pk, int pkb) {
+        constexpr unsigned SD = WIDE_DIAG_CHUNKS, SQ = WIDE_DENSE_CHUNKS;
+        const PJob &jb = pjob_sh[warp_id];
+        const int M = jb.M, NT = jb.NT, i1 = jb.i1, j1 = i1 + jb.d, p0 = jb.p0, tile = jb.tile;
+        const int BI = tile >> 8 & 0xff, BJ = tile & 0xff, nbc = tile >> 16;
+        auto cell = [&](unsigned i, unsigned j) { return i * M - i * (i - 1) / 2 + (j - i); };
+        auto row = [&](unsigned I) { return I * (2 * NT - 1 - I) / 2; };  // dense tiles before tile row I
+        auto chunk = [&](unsigned I, unsigned J) { return I * SD + row(I) * SQ + (J > I ? SD + (J - I - 1) * SQ : 0); };
+        unsigned long long A, B;
+        bool a_diag, b_diag;
+        if (p0 >= 0) {
+            const int p = p0 + (pk >> 1), k1 = i1 + (pk & 1 ? jb.d - 1 - p : p), KB = BI + pkb;
+            A = jb.F + (unsigned long long)cell(i1, k1) * jb.cell + 16ull * chunk(BI, KB);
+            B = jb.F + (unsigned long long)cell(k1 + 1, j1) * jb.cell + 16ull * chunk(KB, BJ);
+            a_diag = pkb == 0;
+            b_diag = KB == BJ;
         } else {
-            const int m = n - 1 - jb.p0, t = BJ - BI;
-            const float *Fc = Fp + cell_index(M, jb.i1, j1) * CELL, *S2 = Sa + ps2_sh[warp_id];
-            if (m < t) {
-                A = Fc + wide_tile_off(NT, BI, BI + m);
-                B = S2 + s2_image_off(NT, BI + m, BJ);
-                if (m == 0) ab = 16 * WIDE_DIAG_CHUNKS;
-            } else {
-                A = S2 + s2_image_off(NT, BI, BI + 1 + m - t);
-                B = Fc + wide_tile_off(NT, BI + 1 + m - t, BJ);
-                if (m == 2 * t - 1) bb = 16 * WIDE_DIAG_CHUNKS;
-            }
+            const int m = pk - 1 - p0, t = BJ - BI;
+            const unsigned long long Fc = jb.F + (unsigned long long)cell(i1, j1) * jb.cell;
+            auto image = [&](unsigned I, unsigned J) { return jb.S2 + 16ull * SQ * (row(I) + J - I - 1); };
+            A = m < t ? Fc + 16ull * chunk(BI, BI + m) : image(BI, BI + 1 + m - t);
+            B = m < t ? image(BI + m, BJ) : Fc + 16ull * chunk(BI + 1 + m - t, BJ);
+            a_diag = m == 0;
+            b_diag = m == 2 * t - 1;
+        }
+        unsigned ab = a_diag ? SD : SQ, bb = b_diag ? SD : SQ;  // chunks to copy
+        if (nbc < 8) {  // of a tile of the last column, its nbc block columns (a prefix of the image)
+            bb = b_diag ? c_img_colbase[8][nbc] : c_wide_dense_colbase[nbc];
+            if (b_diag) ab = a_diag ? c_img_colbase[8][nbc] : c_wide_dense_colbase[nbc];
         }
         const unsigned bar = smem_u32(bars + s);
-        mbar_arrive_tx(bar, (unsigned)(ab + bb));
+        mbar_arrive_tx(bar, 16 * (ab + bb));
         armed[s] += 1;
         const unsigned dst = smem_base + (unsigned)(s * C::STAGE_BYTES);
-        bulk_g2s(dst, A, (unsigned)ab, bar);
-        bulk_g2s(dst + 16 * C::SLOT, B, (unsigned)bb, bar);
+        bulk_g2s(dst, reinterpret_cast<const void *>(A), 16 * ab, bar);
+        bulk_g2s(dst + 16 * C::SLOT, reinterpret_cast<const void *>(B), 16 * bb, bar);
     };
 
     // consumer position (job jid, item it of items) and producer position S items ahead
     int items = job_items(jobs[jid]), it = 0;
-    int pj = jid, pit = 0, pitems = items;
+    int pj = jid, pitems = items, pk = 0, pkb = 0;
     // the producer's advance (every warp the same way) also refreshes the warp's copy of its job
     auto advance_p = [&]() {
-        if (++pit >= pitems) {
-            pit = 0;
+        --pitems;
+        if (pjob_sh[warp_id].p0 < 0 || ++pkb > (pjob_sh[warp_id].tile & 0xff) - (pjob_sh[warp_id].tile >> 8 & 0xff)) {
+            pkb = 0;
+            ++pk;
+        }
+        if (pitems == 0) {
+            pk = 0;
+            pkb = 0;
             pj += gridDim.x;
             if (pj < njobs) {
                 pitems = job_items(jobs[pj]);
@@ -163,7 +190,7 @@ r0_wide_kernel(const R0JobW *__restrict__ jobs, int njobs, const PairDesc *__res
     chain_wait();
     for (int s = 0; s < S; ++s)
         if (pj < njobs) {
-            if (tid == 0 && !ctl.inject) fill_stage(s, pit);
+            if (tid == 0 && !ctl.inject) fill_stage(s, pk, pkb);
             advance_p();
         }
 
@@ -174,7 +201,14 @@ r0_wide_kernel(const R0JobW *__restrict__ jobs, int njobs, const PairDesc *__res
     const int dd_task = c_r0_lane[7][tid][0] == 255
                             ? -1
                             : (c_r0_lane[7][tid][1] | c_r0_lane[7][tid][2] << 4 | c_r0_lane[7][tid][3] << 8);
-    const int mt_task = c_tile_lane[tid][0] | c_tile_lane[tid][1] << 4 | c_tile_lane[tid][2] << 8;
+    const int full_task = c_tile_lane[tid][0] | c_tile_lane[tid][1] << 4 | c_tile_lane[tid][2] << 8;
+    // the lane's micro-tile and share of its k blocks in a job's output tile (-1: none)
+    auto tile_task = [&](int tile) {
+        const int nbc = tile >> 16;
+        if (nbc == 8) return full_task;
+        const int h = tid / (8 * nbc), m = tid - 8 * nbc * h;
+        return h < wide_split(nbc) ? (m & 7) | (m >> 3) << 4 | h << 8 : -1;
+    };
     float acc[8][8];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
@@ -185,10 +219,10 @@ r0_wide_kernel(const R0JobW *__restrict__ jobs, int njobs, const PairDesc *__res
     int stage = 0;
     bool bad = false;  // as in r0_kernel: a wait ran out; no more copies, leave at the next job end
     // the job's output tile; k tile of the item = BI + kbi; first R1/R2 item of the job (-1: R0 items)
-    int tile = jobs[jid].tile, slab = jobs[jid].p0 < 0 ? -1 - jobs[jid].p0 : -1, kbi = 0;
+    int tile = jobs[jid].tile, mt_task = tile_task(tile), slab = jobs[jid].p0 < 0 ? -1 - jobs[jid].p0 : -1, kbi = 0;
 #pragma unroll 1
     while (true) {
-        const int BI = tile >> 8, BJ = tile & 0xff;
+        const int BI = tile >> 8 & 0xff, BJ = tile & 0xff;
         if (slab >= 0) kbi = slab + it < BJ - BI ? slab + it : slab + it - (BJ - BI) + 1;
         const int KB = BI + kbi;
         if (!bad && !mbar_wait(smem_u32(bars + stage), (phase >> stage) & 1u, ctl.wait_ns)) {
@@ -222,18 +256,22 @@ r0_wide_kernel(const R0JobW *__restrict__ jobs, int njobs, const PairDesc *__res
                         for (int j = 0; j < 8; ++j) acc[0][j] = fmaxf(acc[0][j], s1a + rv[j]);
                     }
                 }
-            } else {
+            } else if (mt_task >= 0) {
                 const int bi = mt_task & 15, bj = (mt_task >> 4) & 15, h = mt_task >> 8;
                 const bool a_diag = KB == BI, b_diag = KB == BJ;
-                int k0 = 4 * h, n = 4;
-                if (a_diag || b_diag) {
+                int k0 = 4 * h, k1 = k0 + 4, dk = 1;  // k blocks of the lane
+                if (tile >> 16 < 8) {
+                    k0 = (a_diag ? bi : 0) + h;
+                    k1 = b_diag ? bj + 1 : 8;
+                    dk = wide_split(tile >> 16);
+                } else if (a_diag || b_diag) {
                     const int lo = a_diag ? bi : 0, cnt = a_diag ? 8 - bi : bj + 1, half = (cnt + 1) >> 1;
                     k0 = h == 0 ? lo : lo + half;
-                    n = h == 0 ? half : cnt - half;
+                    k1 = h == 0 ? lo + half : lo + cnt;
                 }
                 const float *bcol = Bs + 4 * ((b_diag ? c_img_colbase[8][bj] : c_wide_dense_colbase[bj]) + 2);
 #pragma unroll 1
-                for (int kb = k0; kb < k0 + n; ++kb)
+                for (int kb = k0; kb < k1; kb += dk)
                     r0_task<0>(As + 4 * ((a_diag ? c_img_colbase[8][kb] : c_wide_dense_colbase[kb]) + 17 * bi),
                                bcol + 4 * 17 * kb, acc);
                 if (a_diag && h == 0) {  // kb == bi is the first block of this lane: the k = 8bi-1 term
@@ -256,7 +294,7 @@ r0_wide_kernel(const R0JobW *__restrict__ jobs, int njobs, const PairDesc *__res
             const bool refill = pj < njobs && !__any_sync(0xffffffffu, bad);  // (test mode: every warp is bad)
             if (lane == 0) {
                 done_cnt[stage] = 0;
-                if (refill) fill_stage(stage, pit);
+                if (refill) fill_stage(stage, pk, pkb);
             }
         }
         if (pj < njobs) advance_p();
@@ -291,6 +329,7 @@ r0_wide_kernel(const R0JobW *__restrict__ jobs, int njobs, const PairDesc *__res
             const R0JobW nx = jobs[jid];
             items = job_items(nx);
             tile = nx.tile;
+            mt_task = tile_task(tile);
             slab = nx.p0 < 0 ? -1 - nx.p0 : -1;
             it = 0;
             kbi = 0;
