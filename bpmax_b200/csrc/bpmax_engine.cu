@@ -507,9 +507,8 @@ int build_plan(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int
             if (d == 0) continue;
             {
                 // Strips of T cells (bpmax_strip.cuh), once per T diagonals d .. d+T-1 (d = 1 mod T): the
-                // offsets [T-1, d-1], which read only diagonals < d for every cell of a strip. The T-1
-                // offset pairs (w, d-1-w) at the ends of every cell's range are the jobs of r0_kernel,
-                // diagonal by diagonal (they repeat up to T-1 offsets of the strip: a maximum). Diagonals
+                // offsets [0, d-1], of which cell t of a strip takes those >= t. The first t offset pairs
+                // of diagonal d+t, which meet diagonals >= d, are the jobs of r0_kernel. Diagonals
                 // with little work keep r0_kernel alone: a strip launch adds a launch to the chain and
                 // clears T merge tiles per CTA. Fill ms with strips everywhere / from 3,400 tasks (28
                 // width-64 items) per SM / nowhere: 37x23 0.66 / 0.57 / 0.55, 128x64 6.69 / 6.57 / 6.52,
@@ -522,11 +521,10 @@ int build_plan(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int
                 for (int p = 0; p < n; ++p)
                     if (P.pairs[p].Np == np && Ms[p] > d0) cells0 += Ms[p] - d0;
                 // tasks of an item: NB(NB+1)(NB+2)/6
-                if (NB >= STRIP_MIN_NB && d0 >= T &&
-                    cells0 * (d0 - T + 1) * (NB * (NB + 1) * (NB + 2) / 6) >= P.strip_tasks * ctx->sms) {
-                    edge = std::min<long long>(P2, T - 1);
+                if (NB >= STRIP_MIN_NB && cells0 * d0 * (NB * (NB + 1) * (NB + 2) / 6) >= P.strip_tasks * ctx->sms) {
+                    edge = std::min<long long>(P2, d - d0);
                     if (d == d0) {
-                        const long long stages = (d - T + G) / G;  // of G offsets
+                        const long long stages = (d + G - 1) / G;  // of G offsets
                         const long long resident = capped(np, ctx->sms);
                         const long long q =
                             strip_stages_per_job(cells, stages, resident, std::max<long long>(1, 2LL * P.pairs_per_job / G),
@@ -534,7 +532,7 @@ int build_plan(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int
                         Plan::Launch sl{d, np, (int)P.strip_jobs.size(), 0};
                         sl.strip = true;
                         sl.cap = (int)resident;
-                        for (long long w0 = T - 1; w0 < d; w0 += q * G)
+                        for (long long w0 = 0; w0 < d; w0 += q * G)
                             for (int p = 0; p < n; ++p)
                                 if (P.pairs[p].Np == np && Ms[p] > d)
                                     for (int i1 = 0; i1 < Ms[p] - d; ++i1)
@@ -543,6 +541,7 @@ int build_plan(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int
                         P.r0_launches.push_back(sl);
                     }
                 }
+                if (edge == 0) continue;
                 // jobs of q offset pairs, ordered by pair chunk, then pair, then cell: the two uses of a
                 // table (A of cell (a, a+d) at offset w, B of cell (a+w-d, a+w) at offset d-1-w) fall in
                 // the same pair chunk

@@ -6,8 +6,9 @@
 // k1 the T cells share the operand A = F(i1, k1), and their operands B_t = F(k1+1, i1+d+t) are
 // neighbours in memory (row-major outer triangle), so one step of K values of k1 lands K images of A
 // and K runs of T images of B with 2K bulk copies, (1+T)/(2T) of the bytes that T separate cells
-// need. Offsets T-1 <= w <= d-1 read only tables of diagonals < d for every cell of the strip; the
-// remaining offsets of each cell (at both ends of its range) are r0_kernel's, per diagonal.
+// need. Cell t's offsets t <= w <= d-1 read only tables of diagonals < d (its B at offset w lies on diagonal
+// d+t-1-w); the remaining ones, w < t and w >= d, are the first t of its offset pairs (w, d+t-1-w), and
+// r0_kernel's, per diagonal.
 //
 // One CTA per SM: T groups of warps, group t computing cell t with the lane table and warp programs of
 // the width class. A warp waits for a stage of the shared-memory ring, does its tasks and counts
@@ -28,6 +29,8 @@
 // whole ring waits for it), hence the cursor that only adds. r0_kernel took 1,240 with 20,160 bytes
 // per item, against 13,440 here. Fill: 1024x64 766 -> 661 ms, the 512-pair batch 523 -> 460 ms.
 #pragma once
+#include <cstddef>
+
 #include "bpmax_r0.cuh"
 
 namespace bpmax {
@@ -82,7 +85,7 @@ struct StripCfg {
 
 // what a stage holds, written by the producing warp before it announces the stage's bytes
 struct __align__(16) StripRec {
-    int info;       // k1 values in the stage | cells of the strip inside the table << 8; -1: no more stages
+    int info;       // k1 values in the stage | cells of the strip that take them << 8; -1: no more stages
     int last;       // the job ends with this stage
     long long out;  // float offset of the table of cell t = 0 (the others follow it)
 };
@@ -90,14 +93,17 @@ struct __align__(16) StripRec {
 // the producing warp's position, in shared memory (the product tile leaves no registers for it)
 struct __align__(16) StripCursor {
     unsigned long long a_src, b_src;  // next A image and next run of B images (byte addresses)
-    int left;                         // k1 of the job still to be produced
+    int left, w;                      // k1 of the job still to be produced, offset of the next
     int b_step;                       // cells from one run of B images to the next (one less each time)
     int pair, job;                    // job >= njobs: no more; 0x7fffffff once the closing record is out
-    StripRec rec;                     // the record of the job's stages
-    StripJob next;                    // prefetched: the job gridDim.x further on
+    long long out;                    // float offset of the table of cell t = 0
+    int cells;                        // cells of the strip inside the table
+    alignas(16) StripJob next;        // prefetched (16 bytes by cp.async): the job gridDim.x further on
     unsigned long long F_pair;        // byte address of the pair's tables
     int M;
 };
+
+static_assert(sizeof(StripJob) == 16 && offsetof(StripCursor, next) % 16 == 0, "cp.async of the next job");
 
 // (group, table warp) of consumer warp c, whose SM sub-partition is c % 4: the warp programs' step
 // counts (128, 92, 80, 49) summed per sub-partition come to at most 336 for programs 0 0 1 2 (mean
@@ -179,8 +185,10 @@ r0_strip_kernel(const StripJob *__restrict__ jobs, int njobs, const PairDesc *__
         cur.b_src = cur.F_pair + (unsigned long long)cell32(M, k1 + 1, j1) * (4 * CELL);
         cur.b_step = M - k1 - 2;  // from row k1+1 to row k1+2
         cur.left = jb.w1 - jb.w0;
+        cur.w = jb.w0;
         const float *out = reinterpret_cast<const float *>(cur.F_pair) + cell32(M, jb.i1, j1) * CELL;
-        cur.rec = StripRec{C::K | min(C::T, M - j1) << 8, 0, out - F};
+        cur.out = out - F;
+        cur.cells = min(C::T, M - j1);
     };
     // the producing warp fills a free stage with the next K k1 of its jobs; after the last, the closing
     // record that lets the warps leave
@@ -195,22 +203,23 @@ r0_strip_kernel(const StripJob *__restrict__ jobs, int njobs, const PairDesc *__
             __syncwarp();
             return;
         }
-        const int left = cur.left, b_step = cur.b_step;
+        const int left = cur.left, b_step = cur.b_step, w = cur.w;
         const unsigned long long a_src = cur.a_src, b_src = cur.b_src;
-        StripRec r = cur.rec;
-        const int cells = r.info >> 8, valid = min(C::K, left);
+        // offsets below a cell's place in the strip are not its: one k1 a stage there, for cells 0 .. w
+        const int valid = C::K == 1 || w < C::T - 1 ? 1 : min(C::K, left), cells = min(cur.cells, w + 1);
+        const long long out = cur.out;
         const unsigned bar = full_u + 8 * stage, dst = smem_u32(sm) + stage * C::STAGE_BYTES;
         if constexpr (C::K > 1) __syncwarp();  // every lane has read the cursor
         if (lane == 0) {
-            if (left <= C::K) r = StripRec{valid | cells << 8, 1, r.out};
-            rec[stage] = r;
+            rec[stage] = StripRec{valid | cells << 8, left == valid, out};
             mbar_arrive_tx(bar, (unsigned)(valid * (1 + cells) * C::IMG * 16));
             armed[stage] += 1;
-            cur.left = left - C::K;
-            cur.a_src = a_src + C::K * 4 * CELL;
-            // K steps of b_step, b_step - 1, ... cells
-            cur.b_src = b_src + (long long)(C::K * b_step - C::K * (C::K - 1) / 2) * (4 * CELL);
-            cur.b_step = b_step - C::K;
+            cur.left = left - valid;
+            cur.w = w + valid;
+            cur.a_src = a_src + valid * 4 * CELL;
+            // `valid` steps of b_step, b_step - 1, ... cells
+            cur.b_src = b_src + (long long)(valid * b_step - valid * (valid - 1) / 2) * (4 * CELL);
+            cur.b_step = b_step - valid;
         }
         if constexpr (C::K > 1) __syncwarp();  // the bytes are announced
         for (int kk = lane; kk < valid; kk += 32) {
@@ -220,7 +229,7 @@ r0_strip_kernel(const StripJob *__restrict__ jobs, int njobs, const PairDesc *__
                      reinterpret_cast<const void *>(b_src + (long long)(kk * b_step - kk * (kk - 1) / 2) * (4 * CELL)),
                      (unsigned)(cells * C::IMG * 16), bar);
         }
-        if (lane == 0 && left <= C::K) {
+        if (lane == 0 && left == valid) {
             cp_async_wait<0>();
             open_job(cur.job + gridDim.x, cur.next);
         }
