@@ -680,7 +680,7 @@ void launch_fin_t(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
 template <int NB>
 void launch_fin(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
 {
-    if (L.count >= FIN_BULK_CELLS) return launch_fin_t<NB, fin_bulk_threads(8 * NB)>(ctx, L, s);
+    if (L.count >= FIN_BULK_CELLS) return launch_fin_t<NB, FIN_BULK_THREADS>(ctx, L, s);
     launch_fin_t<NB, fin_threads(8 * NB)>(ctx, L, s);
 }
 
@@ -722,7 +722,7 @@ int set_smem_attr(bpmax_ctx *ctx)
     if ((st = prefer_smem(ctx, r0_kernel<NB>)) || (st = prefer_smem(ctx, r0_kernel<NB, 1>)) ||
         (st = prefer_smem(ctx, finalize_small_kernel<8 * NB>)) || (st = prefer_smem(ctx, r0only_finalize_small_kernel<8 * NB>)))
         return st;
-    if ((st = prefer_smem(ctx, finalize_small_kernel<8 * NB, fin_bulk_threads(8 * NB)>))) return st;
+    if ((st = prefer_smem(ctx, finalize_small_kernel<8 * NB, FIN_BULK_THREADS>))) return st;
     if constexpr (NB >= STRIP_MIN_NB) {
         if ((st = prefer_smem(ctx, r0_strip_kernel<NB>))) return st;
         CK(cudaFuncSetAttribute(r0_strip_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)StripCfg<NB>::SMEM));
@@ -737,9 +737,9 @@ int set_smem_attr(bpmax_ctx *ctx)
                                                      R0Cfg<NB, 1>::SMEM));
     CK(cudaFuncSetAttribute(finalize_small_kernel<8 * NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                             (int)FinShape<8 * NB>::SMEM));
-    CK(cudaFuncSetAttribute(finalize_small_kernel<8 * NB, fin_bulk_threads(8 * NB)>,
+    CK(cudaFuncSetAttribute(finalize_small_kernel<8 * NB, FIN_BULK_THREADS>,
                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)FinShape<8 * NB, fin_bulk_threads(8 * NB)>::SMEM));
+                            (int)FinShape<8 * NB, FIN_BULK_THREADS>::SMEM));
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctx->r0_occ_v[0][NB], r0_kernel<NB>, R0Cfg<NB>::THREADS,
                                                      R0Cfg<NB>::SMEM));
     CK(cudaFuncSetAttribute(fill_persistent_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)R0Cfg<NB>::SMEM));

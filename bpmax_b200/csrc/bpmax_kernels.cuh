@@ -208,21 +208,14 @@ __global__ void single_strand_kernel(const PairDesc *__restrict__ pairs, const u
 // writes a table before its own finalize, and those of diagonal d may run before the finalize of
 // d-1 and d-2. Every literal-0 candidate is covered because every value is >= +0. Writes the cell's
 // blocks (-inf outside the logical triangle, S1(i1,j1) on the subdiagonal) and its S1 pieces.
-// The inner wavefront goes by batches of FIN_BATCH = 5 inner diagonals of the cell's table in shared
-// memory, D[e][i2] = F[i2][i2+e], each open entry holding its running maximum. A final diagonal e
-// gives every entry (i2, j2) of diagonal e2 > e the candidates
-//   R1 with k2 = i2+e:    F[i2][i2+e] + S2(i2+e+1, j2)
-//   R2 with k2 = j2-e-1:  S2(i2, j2-e-1) + F[j2-e][j2]
-// S2 is 0 on spans <= 3, so those of e = e2-1 are F[i2][j2-1] and F[i2+1][j2] themselves, which are
-// never less than the ones of e = e2-2 .. e2-4 (each of those is a candidate of them, plus 0): only
-// e <= e2-5 is left to add. So within a batch an entry needs no more than its two neighbours of the
-// previous diagonal and SW2, and one warp runs the batch's five steps in registers, two rows per
-// lane and one shuffle per step, without a CTA barrier; the sums go to later batches in bulk: to the
-// next batch first, by all warps, then, while the first warp runs that batch, to all others by the
-// other warps. Two CTA barriers per batch (26 at width 64; one step per barrier took 63).
-// Bound: latency, about 6 us of a 64-wide cell in the inner wavefront and 3 us of dependent global loads
-// before it. Fill ms with one barriered step per inner diagonal / with batches: 37x23 0.57 / 0.53,
-// 128x64 6.52 / 4.83, 200x64 13.7 / 11.0, 1024x64 661 / 640, the 512-pair batch 460 / 428.
+// The inner wavefront goes by 8x8 blocks of the table in shared memory (block_wave).
+// Bound: latency of the wavefront where a launch has few cells (at width 64, 8 block diagonals of
+// 600-1,230 cycles of products and 930 of the blocks' own wavefronts), instructions where it has many.
+// Before, batches of five inner diagonals, the next batch's in the registers of one warp while the
+// others pushed the last one's candidates to all later entries: 19,400 cycles at width 64. Fill ms
+// by batches / by blocks: 64x64 1.52 / 1.39, 128x32 1.98 / 1.82, 128x64 4.26 / 4.09, 1024x64 614 / 601,
+// the 512-pair batch 424 / 418. Tried: the blocks' start values loaded ahead of their wavefronts, 1,150
+// cycles; their S2 values picked from registers per column, 3,240 (divergent branches).
 // CTAs after the first njobs compute S1 on diagonal d+1 (V3/bpmax_verify.c:533-544), one warp
 // per cell, from S1 diagonals <= d (S1 is cleared to 0 before the fill; j-i <= 3 stays 0).
 // ------------------------------------------------------------------------------------------
@@ -230,15 +223,15 @@ struct CellJob {
     int pair, i1;
 };
 
-// threads per cell. Few cells: what counts is the latency of one cell, which the bulk sums to later
-// batches set, so many threads. Launches of FIN_BULK_CELLS cells or more (batches) fill every SM
-// several times over: fewer threads per cell then issue fewer idle lanes and barrier waits. Fill ms
-// at 128 / 256 / 384 / 512 / 768 threads: 128x32 2.82 / 2.50 / 2.46 / 2.47 / -, 128x64 - / 5.35 /
-// 4.94 / 4.81 / 4.74, 256x64 - / 18.97 / 18.33 / 18.11 / 18.72; the 512-pair batch 426-430 with the
-// smaller ones, 442 and 452 with 768 and 1024.
-constexpr int fin_threads(int NP) { return NP >= 48 ? 512 : (NP >= 24 ? 384 : 128); }
-constexpr int fin_bulk_threads(int NP) { return NP >= 48 ? 256 : 128; }
-constexpr int FIN_BULK_CELLS = 1024;
+// threads per cell. Up to one cell per SM what counts is the latency of one cell: many threads for its
+// loads and products. Launches of more cells run several CTAs per SM, which hide each other's latency,
+// and four warps per cell then idle least at the barriers. Fill ms with the latency threads for up to
+// 1,024 / 296 / 148 cells: 1024x64 622 / 602 / 601, 256x64 16.2 / 16.2 / 15.8; the 512-pair batch at
+// 256 / 160 / 128 threads beyond: 428 / 419 / 418. Up to 148 cells 128x64 takes 4.44 with 256 threads
+// and 4.09 with 512, 64x32 0.83 with 128, 0.73 with 256 and 0.71 with 384.
+constexpr int fin_threads(int NP) { return NP >= 48 ? 512 : (NP >= 32 ? 384 : 128); }
+constexpr int FIN_BULK_THREADS = 128;
+constexpr int FIN_BULK_CELLS = 149;
 // element (r, c) of tile (I2, J2) of an outer cell in the reference layout (tiles of T+1 rows, the
 // last one the halo; R = padding rows/columns of the first tile row/column); val(i2, j2) gives the
 // cell's inner value for 0 <= i2 <= j2 < N, the only entries read
@@ -286,22 +279,15 @@ struct RefOut {
     int T, Ns;
 };
 
-constexpr int FIN_BATCH = 5;  // inner diagonals per batch: 1 + the largest span with S2 = 0, + 1
-
 template <int NP, int T = fin_threads(NP)>
 struct FinShape {
     static constexpr int THREADS = T;
     static constexpr int WARPS = THREADS / 32;
-    static constexpr int MINB = 1280 / THREADS;  // 40 resident warps per SM (48 registers)
-    // row pitch of D and of S2 by diagonals: entry (r, c) lies at (c-r)*LD + r, so rows r of a block
-    // column are LD-1 (odd) words apart and diagonals start on 8 bytes
-    static constexpr int LD = NP + 2;
-    static constexpr size_t SMEM = 2 * (size_t)NP * LD * sizeof(float) + NP;  // D, S2, bases
-    static_assert(WARPS >= 2 && NP <= 64, "one warp runs the batches, two rows per lane");
+    static constexpr int LD = NP + 4;  // row pitch of the tables: an odd number of 16-byte chunks
+    // table (4 words before it, one row after it), two copies of S2, bases
+    static constexpr size_t SMEM = ((size_t)4 + (3 * NP + 1) * LD) * sizeof(float) + NP;
+    static constexpr int MINB = 768 / THREADS;  // at most 80 registers
 };
-
-// first float of row e of a triangular diagonal-major table of width NP (row e holds NP - e entries)
-__host__ __device__ __forceinline__ int drow(int NP, int e) { return e * NP - e * (e - 1) / 2; }
 
 // (BI, BJ) of the q-th block of the upper block triangle (row-major triangle order)
 __device__ __forceinline__ void blk_decode(int NB, int q, int &BI, int &BJ)
@@ -309,6 +295,125 @@ __device__ __forceinline__ void blk_decode(int NB, int q, int &BI, int &BJ)
     BI = 0;
     while (q >= NB - BI) { q -= NB - BI; ++BI; }
     BJ = BI + q;
+}
+
+// ------------------------------------------------------------------------------------------
+// The inner wavefront of R1, R2 and SW2 inside a table (tri: an upper triangle of nb block rows) or a
+// 64x64 tile, by 8x8 blocks, block diagonal by block diagonal; all threads of the CTA. T[r][c] holds the
+// start values (-inf below the diagonal, in columns >= ncol, in column -1 and in the row after the
+// last) and receives the final ones; SJ[x][y] = S2(x, y) of the columns' strand piece (-inf in columns
+// >= ncol), SX[x][y] = S2(x, y-1) of the rows'; wt[LD*b + c] = the SW2 weight of row base b and column c;
+// rb = the rows' bases; entry (r, c) spans j2-i2 = e0 + c - r.
+//   1. one warp per block adds the terms over the finished blocks of its row and column,
+//        R1  T[r][k] + S2(k+1, c),  R2  S2(r, k-1) + T[k][c],
+//      as products, four lanes sharing the k of a 2x4 piece, and SW2 from outside the block;
+//   2. one warp per four blocks runs the blocks' own wavefronts over their 15 diagonals in registers, a row
+//      per lane. S2 is 0 on spans <= 3, so inside a block an entry needs its two neighbours of the
+//      previous diagonal (never less than the candidates of two to four diagonals back, each of which is a
+//      candidate of theirs plus 0), SW2, and what lies five to seven columns left or rows below.
+// The candidates of neighbours outside the block are in the products.
+// ------------------------------------------------------------------------------------------
+template <int LD, int WARPS>
+__device__ __forceinline__ void block_wave(float *T, const float *SX, const float *SJ, const float *wt, const uint8_t *rb,
+                                           bool tri, int nb, int ncol, int e0)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nbc = (ncol + 7) >> 3;
+    const int kp = lane & 3, st = lane >> 2, la = lane & 7;
+    for (int D = tri ? 0 : 1 - nb; D < nbc; ++D) {
+        const int first = max(0, -D), count = min(nb - first, nbc - max(0, D));  // blocks (first + m, first + m + D)
+        __syncthreads();  // the blocks of earlier block diagonals are final
+        if (!tri || D > 0) {
+            for (int m = warp; m < count; m += WARPS) {
+                const int bi = first + m, bj = bi + D;
+                // rows r0, r0+1, columns c0 .. c0+3, k = 2kp, 2kp+1 of every k block; in the end row r,
+                // columns c, c+1, whose words from outside the block are loaded first
+                const int r0 = 8 * bi + 2 * (st >> 1), c0 = 8 * bj + 4 * (st & 1);
+                const int r = r0 + (kp & 1), c = c0 + (kp & 2);
+                float2 *o = reinterpret_cast<float2 *>(T + r * LD + c);
+                const float2 x = *o, wr = *reinterpret_cast<const float2 *>(wt + LD * rb[r] + c);
+                const float q0 = T[(r + 1) * LD + c - 1], q1 = T[(r + 1) * LD + c];
+                float v[2][4];
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) v[i][j] = NEG_INF;
+                auto step = [&](const float *A, const float *B) {  // A: row r0, k = 2kp; B: row 2kp, column c0
+                    const float2 x0 = *reinterpret_cast<const float2 *>(A), x1 = *reinterpret_cast<const float2 *>(A + LD);
+                    const float4 y0 = *reinterpret_cast<const float4 *>(B), y1 = *reinterpret_cast<const float4 *>(B + LD);
+                    v[0][0] = fmax3(v[0][0], x0.x + y0.x, x0.y + y1.x);
+                    v[0][1] = fmax3(v[0][1], x0.x + y0.y, x0.y + y1.y);
+                    v[0][2] = fmax3(v[0][2], x0.x + y0.z, x0.y + y1.z);
+                    v[0][3] = fmax3(v[0][3], x0.x + y0.w, x0.y + y1.w);
+                    v[1][0] = fmax3(v[1][0], x1.x + y0.x, x1.y + y1.x);
+                    v[1][1] = fmax3(v[1][1], x1.x + y0.y, x1.y + y1.y);
+                    v[1][2] = fmax3(v[1][2], x1.x + y0.z, x1.y + y1.z);
+                    v[1][3] = fmax3(v[1][3], x1.x + y0.w, x1.y + y1.w);
+                };
+                const float *A1 = T + r0 * LD + 2 * kp, *B1 = SJ + (2 * kp + 1) * LD + c0;  // R1: k blocks k1 .. bj-1
+                const float *A2 = SX + r0 * LD + 2 * kp, *B2 = T + 2 * kp * LD + c0;        // R2: k blocks bi+1 .. k2
+                const int k1 = tri ? bi : 0, n1 = bj - k1, n2 = (tri ? bj : nb - 1) - bi;
+                int t = 0;
+                for (; t < min(n1, n2); ++t) {
+                    step(A1 + 8 * (k1 + t), B1 + 8 * LD * (k1 + t));
+                    step(A2 + 8 * (bi + 1 + t), B2 + 8 * LD * (bi + 1 + t));
+                }
+                for (int u = t; u < n1; ++u) step(A1 + 8 * (k1 + u), B1 + 8 * LD * (k1 + u));
+                for (int u = t; u < n2; ++u) step(A2 + 8 * (bi + 1 + u), B2 + 8 * LD * (bi + 1 + u));
+                float h[4], g[2];  // lane kp keeps row kp & 1, then columns kp & 2 and the next
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float keep = kp & 1 ? v[1][j] : v[0][j], give = kp & 1 ? v[0][j] : v[1][j];
+                    h[j] = fmaxf(keep, __shfl_xor_sync(0xffffffffu, give, 1));
+                }
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const float keep = kp & 2 ? h[j + 2] : h[j], give = kp & 2 ? h[j] : h[j + 2];
+                    g[j] = fmaxf(keep, __shfl_xor_sync(0xffffffffu, give, 2));
+                }
+                const bool last = (r & 7) == 7;  // SW2 of the block's last row and first column
+                const float w0 = (last || (c & 7) == 0) && e0 + c - r >= 4 ? q0 + wr.x : NEG_INF;
+                const float w1 = last && e0 + c + 1 - r >= 4 ? q1 + wr.y : NEG_INF;
+                *o = make_float2(fmax3(x.x, g[0], w0), fmax3(x.y, g[1], w1));
+            }
+            __syncthreads();
+        }
+        for (int w = warp; 4 * w < count; w += WARPS) {
+            const int m = 4 * w + (lane >> 3), bi = first + min(m, count - 1), bj = bi + D;
+            const int row = 8 * bi + la, cols = m < count ? min(8, ncol - 8 * bj) : 0, e1 = e0 + 8 * D;
+            // lane la has row 8bi+la; at step s it computes column 8bj + b, b = s - 7 + la
+            float *Tr = T + row * LD + 8 * bj;
+            const float *wr = wt + LD * rb[row] + 8 * bj, *Sb = SJ + 8 * bj * LD + 8 * bj;
+            float cx[3];  // S2(r, r+4 ..): R2 from rows five to seven below, inside the block
+#pragma unroll
+            for (int x = 0; x < 3; ++x) cx[x] = la + x + 5 < 8 ? SX[row * LD + row + 5 + x] : NEG_INF;
+            float n[15], under = NEG_INF, left = NEG_INF, diag = NEG_INF;  // (r+1, b), (r, b-1), (r+1, b-1)
+#pragma unroll
+            for (int s = 0; s < 15; ++s) {
+                const int b = s - 7 + la, bc = min(max(b, 0), 7);
+                float v = Tr[bc];
+                const float w2 = e1 + s - 7 >= 4 ? wr[bc] : NEG_INF;
+#pragma unroll
+                for (int x = 0; x < 3; ++x)
+                    if (s >= 5 + x) {  // five to seven diagonals back: R1 in the lane, R2 from lane la + 5 + x
+                        const float r1 = n[s - 5 - x] + Sb[max(bc - 4 - x, 0) * LD + bc];  // S2(c-5-x + 1, c)
+                        const float r2 = __shfl_down_sync(0xffffffffu, n[s - 5 - x], 5 + x, 8) + cx[x];
+                        v = fmax3(v, r1, r2);
+                    }
+                under = s > 0 ? __shfl_down_sync(0xffffffffu, n[s - 1], 1, 8) : NEG_INF;
+                if (la == 7) under = NEG_INF;
+                const float r = fmaxf(fmax3(v, left, under), diag + w2);
+                n[s] = b >= 0 && b < cols ? r : NEG_INF;
+                diag = under;
+                left = n[s];
+            }
+#pragma unroll
+            for (int s = 0; s < 15; ++s) {
+                const int b = s - 7 + la;
+                if (b >= 0 && b < cols) Tr[b] = n[s];
+            }
+        }
+    }
+    __syncthreads();
 }
 
 template <int NP, int T = fin_threads(NP)>
@@ -322,8 +427,9 @@ finalize_small_kernel(const CellJob *__restrict__ jobs, int njobs, const CellJob
     constexpr long long CELL = 4LL * R0_TAB_COLBASE[NB][NB];
     extern __shared__ __align__(16) float fsm[];
     constexpr int LD = Sh::LD;
-    float *D = fsm, *Sd = fsm + NP * LD;  // Sd[e][i] = S2(i, i+e)
-    uint8_t *sb = reinterpret_cast<uint8_t *>(fsm + 2 * NP * LD);
+    float *D = fsm + 4, *SX = D + (NP + 1) * LD, *SJ = SX + NP * LD;  // the table; S2(r, c-1) and S2(r, c)
+    uint8_t *sb = reinterpret_cast<uint8_t *>(SJ + NP * LD);
+    __shared__ __align__(16) float wt[5 * LD];  // wt[LD*x + c]: intra-strand weight of base x and column c
     __shared__ int cbs[NB];    // float offset of each block column in the cell image
     __shared__ float wsh[12];  // the weight table (indexed by pair type)
     __shared__ float w5[25];   // intra-strand weight of bases a, b at 5a + b
@@ -366,14 +472,20 @@ finalize_small_kernel(const CellJob *__restrict__ jobs, int njobs, const CellJob
     const uint8_t *s1 = bases + pd.seq1_off;
     const uint8_t *s2r = bases + pd.seq2_off;
     for (int q = tid; q < NP; q += Sh::THREADS) sb[q] = q < N ? s2r[q] : 4;
+    for (int q = tid; q < 5 * LD; q += Sh::THREADS) {
+        const int c = q % LD;
+        wt[q] = w5[5 * (q / LD) + (c < N ? s2r[c] : 4)];
+    }
     const int x1 = s1[i1], y1 = s1[j1];
     chain_wait();
     const float s1v = S1[i1 * M + j1];
     // start values (accumulated products, S1+S2, SW1; the inter-strand base on the diagonal of the
-    // diagonal cells) and S2, both by diagonals, 4 columns of one block row per step
+    // diagonal cells; -inf elsewhere) and S2, 4 columns of one block row per step
     const bool sw1 = d >= 4;
     const float w1 = sw1 ? score_w(wsh, x1, y1) : 0.0f;
     const float *Fi = F + pd.F_off + (sw1 ? cell_index(M, i1 + 1, j1 - 1) * CELL : 0);
+    if (tid < 4) D[tid - 4] = NEG_INF;
+    for (int q = tid; q < 4 * NP; q += Sh::THREADS) D[(q >> 2) * LD + NP + (q & 3)] = NEG_INF;  // the pad columns
     for (int q4 = tid; q4 < NBLK * 16; q4 += Sh::THREADS) {
         int BI, BJ;
         blk_decode(NB, q4 >> 4, BI, BJ);
@@ -381,77 +493,20 @@ finalize_small_kernel(const CellJob *__restrict__ jobs, int njobs, const CellJob
         const float4 f4 = *reinterpret_cast<const float4 *>(Fc + o), s4 = *reinterpret_cast<const float4 *>(S2 + r * NP + c0);
         float4 p4 = make_float4(NEG_INF, NEG_INF, NEG_INF, NEG_INF);
         if (sw1) p4 = *reinterpret_cast<const float4 *>(Fi + o);
-        const float fv[4] = {f4.x, f4.y, f4.z, f4.w}, sv[4] = {s4.x, s4.y, s4.z, s4.w}, pv[4] = {p4.x, p4.y, p4.z, p4.w};
+        const float fv[4] = {f4.x, f4.y, f4.z, f4.w}, pv[4] = {p4.x, p4.y, p4.z, p4.w};
+        float sv[4] = {s4.x, s4.y, s4.z, s4.w}, v[4];
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
             const int c = c0 + t;
-            if (r <= c && c < N) {
-                D[(c - r) * LD + r] = d == 0 && r == c ? score_w(wsh + 6, x1, s2r[r])
-                                                       : fmax3(fv[t], s1v + sv[t], pv[t] + w1);
-                Sd[(c - r) * LD + r] = sv[t];
-            }
+            SX[r * LD + c + 1] = sv[t];  // (column NP is pad)
+            v[t] = r <= c && c < N ? (d == 0 && r == c ? score_w(wsh + 6, x1, s2r[r]) : fmax3(fv[t], s1v + sv[t], pv[t] + w1))
+                                   : NEG_INF;
+            if (c >= N) sv[t] = NEG_INF;
         }
+        *reinterpret_cast<float4 *>(D + r * LD + c0) = make_float4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<float4 *>(SJ + r * LD + c0) = make_float4(sv[0], sv[1], sv[2], sv[3]);
     }
-    __syncthreads();
-    // the first warp's state: rows 2*lane and 2*lane+1 of the last two diagonals (p of e-1, q of e-2),
-    // and row 2*lane+2 of each
-    const int i0 = 2 * lane;
-    float p0 = 0.0f, p1 = 0.0f, q1 = 0.0f, q2 = 0.0f;
-    const int b0 = 5 * sb[min(i0, NP - 1)], b1 = 5 * sb[min(i0 + 1, NP - 1)];
-    auto run_batch = [&](int e0) {
-        float2 a[FIN_BATCH];
-        float wa[FIN_BATCH], wb[FIN_BATCH];
-#pragma unroll
-        for (int s = 0; s < FIN_BATCH; ++s) {
-            const int e = min(e0 + s, NP - 1);
-            a[s] = *reinterpret_cast<const float2 *>(D + e * LD + min(i0, NP - 2));
-            wa[s] = e >= 4 ? w5[b0 + sb[min(i0 + e, NP - 1)]] : NEG_INF;
-            wb[s] = e >= 4 ? w5[b1 + sb[min(i0 + 1 + e, NP - 1)]] : NEG_INF;
-        }
-#pragma unroll
-        for (int s = 0; s < FIN_BATCH; ++s) {
-            const int e = e0 + s;
-            if (e >= N) break;
-            float n0 = a[s].x, n1 = a[s].y;
-            const float p2 = __shfl_down_sync(0xffffffffu, p0, 1);
-            if (e > 0) {
-                n0 = fmaxf(fmax3(n0, p0, p1), q1 + wa[s]);
-                n1 = fmaxf(fmax3(n1, p1, p2), q2 + wb[s]);
-                if (i0 < NP) *reinterpret_cast<float2 *>(D + e * LD + i0) = make_float2(n0, n1);
-            }
-            q1 = p1;
-            q2 = p2;
-            p0 = n0;
-            p1 = n1;
-        }
-    };
-    // candidates of the final diagonals e0 .. e0+4 for entry i of diagonal e2, those with e <= e2-5
-    auto push = [&](int e0, int e2, int i, int n) {
-        const float *De = D + e0 * LD + i, *Dj = De + (e2 - e0);              // F[i][i+e], F[j-e][j]
-        const float *Sj = Sd + (e2 - e0 - 1) * LD + i, *Se = Sj + e0 + 1;     // S2(i, j-e-1), S2(i+e+1, j)
-        float v = D[e2 * LD + i];
-#pragma unroll
-        for (int t = 0; t < FIN_BATCH; ++t)
-            if (t < n) v = fmax3(v, De[t * LD] + Se[-t * (LD - 1)], Sj[-t * LD] + Dj[t * (LD - 1)]);
-        D[e2 * LD + i] = v;
-    };
-    if (warp == 0) run_batch(0);
-    for (int e0 = 0; e0 + FIN_BATCH < N; e0 += FIN_BATCH) {  // diagonals e0 .. e0+4 are final
-        const int e1 = e0 + FIN_BATCH;
-        __syncthreads();
-        for (int u = warp; u < FIN_BATCH * ((NP + 31) / 32); u += Sh::WARPS) {  // to the next batch
-            const int s = FIN_BATCH - 1 - u % FIN_BATCH, i = lane + 32 * (u / FIN_BATCH);
-            if (i < N - (e1 + s)) push(e0, e1 + s, i, s + 1);
-        }
-        __syncthreads();
-        if (warp == 0) {
-            run_batch(e1);
-        } else {
-            for (int e2 = e1 + FIN_BATCH + warp - 1; e2 < N; e2 += Sh::WARPS - 1)
-                for (int i = lane; i < N - e2; i += 32) push(e0, e2, i, FIN_BATCH);
-        }
-    }
-    __syncthreads();
+    block_wave<LD, Sh::WARPS>(D, SX, SJ, wt, sb, true, NB, N, 0);  // (starts and ends with a barrier)
     // write-back, 4 columns of one block row per step
     for (int q4 = tid; q4 < NBLK * 16; q4 += Sh::THREADS) {
         int BI, BJ;
@@ -461,7 +516,7 @@ finalize_small_kernel(const CellJob *__restrict__ jobs, int njobs, const CellJob
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
             const int c = c0 + t;
-            v[t] = r <= c && c < N ? D[(c - r) * LD + r] : (r == c + 1 ? s1v : NEG_INF);  // S1 on the subdiagonal
+            v[t] = r <= c && c < N ? D[r * LD + c] : (r == c + 1 ? s1v : NEG_INF);  // S1 on the subdiagonal
         }
         // block (BI, BJ), row r & 7, half
         *reinterpret_cast<float4 *>(Fc + cbs[BJ] + 68 * BI + 4 * (q4 & 15)) = make_float4(v[0], v[1], v[2], v[3]);
@@ -476,7 +531,7 @@ finalize_small_kernel(const CellJob *__restrict__ jobs, int njobs, const CellJob
                    // values the image holds), one warp per tile row of T floats
         const int TT = ro.T, R = (TT - N % TT) % TT, tile_rows = TT + 1, rows = ro.Ns * ro.Ns * tile_rows;
         float *dst = ro.out + ((long long)d * M - (long long)d * (d - 1) / 2 + i1) * ((long long)rows * TT);
-        auto dval = [&](int i2, int j2) { return D[(j2 - i2) * LD + i2]; };
+        auto dval = [&](int i2, int j2) { return D[i2 * LD + j2]; };
         for (int rr = warp; rr < rows; rr += Sh::WARPS) {
             const int I2 = rr / (ro.Ns * tile_rows), rem = rr % (ro.Ns * tile_rows);
             const int J2 = rem / tile_rows, r = rem % tile_rows;

@@ -290,7 +290,7 @@ fill_persistent_kernel(PersistCtl pc, const PairDesc *__restrict__ pairs, float 
         }
 
         // -------------------------------------------------------------------- finalize of the cell
-        // (the inner wavefront of finalize_small_kernel with this CTA's threads; its tables live in
+        // (one inner diagonal after another with this CTA's threads; its tables live in
         // the stages of the product ring, idle between jobs)
         const int N = pd.N;
         float *Fc = F + pd.F_off + cell_index(M, i1, j1) * CELL;

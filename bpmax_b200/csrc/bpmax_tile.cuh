@@ -11,16 +11,11 @@
 // diagonals of later outer diagonals: M + NT - 1 steps of two launches, r0_wide_kernel (the products of
 // the step's tiles, and the terms over finished tiles as items of the same kind) and tile_final_kernel
 // (one CTA per tile of the step: start values, SW1, the tile's own terms, the tile image).
-// The tile's own terms go by 8x8 blocks, block diagonal by block
-// diagonal, one warp per block: first the terms over the finished blocks of the tile as products, four
-// lanes sharing the k of an 8-entry piece, then the block's own wavefront over its 15 diagonals in
-// registers, one row per lane and one shuffle per step. S2 is 0 on spans <= 3, so inside a block an
-// entry needs its two neighbours of the previous diagonal (never less than the candidates of two to
-// four diagonals back), SW2, and what lies five to seven columns left or rows below. The candidates
-// of neighbours outside a block or tile are in the products; SW2 from outside is read where it lies.
+// The tile's own terms go by 8x8 blocks (block_wave in bpmax_kernels.cuh); SW2 from outside the tile is
+// read where it lies.
 //
-// Bound: latency of a tile's own terms (a tile of t >= 1 takes 26 us alone on an SM: 10 us in 15 block
-// diagonals of products, 11 us in their wavefronts, 5 us of loads). Fill ms with one CTA per cell
+// Bound: latency of a tile's own terms (a tile of t >= 1 runs 15 block diagonals of products
+// and of the blocks' wavefronts, about 1,000 cycles each, and 5 us of loads). Fill ms with one CTA per cell
 // walking every inner diagonal (up to width 320; above, row-major tables with a barrier per tile
 // diagonal) / with the tile diagonals of one outer diagonal after another, the terms over finished tiles
 // in launches of their own / in steps as here: 90x130 32.0 / 24.1 / 19.1,
@@ -246,97 +241,7 @@ tile_final_kernel(const TileJob *__restrict__ jobs, int njobs, const CellJob *__
         if (y + 3 >= ncol) v.w = NEG_INF;
         *reinterpret_cast<float4 *>(SJ + x * LD + y) = v;
     }
-    // block diagonal D = bj - bi: warp w has the w-th block (bi, bj)
-    const int kp = lane & 3, st = lane >> 2, la = lane & 7;
-    for (int D = t == 0 ? 0 : -7; 8 * D < ncol; ++D) {
-        __syncthreads();  // the blocks of earlier block diagonals are final
-        const int bi = max(0, -D) + warp, bj = bi + D;
-        if (bi > 7 || 8 * bj >= ncol) continue;  // (warp-uniform; every warp takes part in the barriers)
-        // products over the finished blocks of the row and the column: rows r0, r0+1, columns c0 .. c0+3,
-        // k = 2kp, 2kp+1 of every k block
-        const int r0 = 8 * bi + 2 * (st >> 1), c0 = 8 * bj + 4 * (st & 1);
-        float v[2][4];
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) v[i][j] = NEG_INF;
-        auto step = [&](const float *A, const float *B) {  // A: row r0, k = 2kp; B: row 2kp, column c0
-            const float2 x0 = *reinterpret_cast<const float2 *>(A), x1 = *reinterpret_cast<const float2 *>(A + LD);
-            const float4 y0 = *reinterpret_cast<const float4 *>(B), y1 = *reinterpret_cast<const float4 *>(B + LD);
-            v[0][0] = fmax3(v[0][0], x0.x + y0.x, x0.y + y1.x);
-            v[0][1] = fmax3(v[0][1], x0.x + y0.y, x0.y + y1.y);
-            v[0][2] = fmax3(v[0][2], x0.x + y0.z, x0.y + y1.z);
-            v[0][3] = fmax3(v[0][3], x0.x + y0.w, x0.y + y1.w);
-            v[1][0] = fmax3(v[1][0], x1.x + y0.x, x1.y + y1.x);
-            v[1][1] = fmax3(v[1][1], x1.x + y0.y, x1.y + y1.y);
-            v[1][2] = fmax3(v[1][2], x1.x + y0.z, x1.y + y1.z);
-            v[1][3] = fmax3(v[1][3], x1.x + y0.w, x1.y + y1.w);
-        };
-#pragma unroll 4
-        for (int kb = t == 0 ? bi : 0; kb < bj; ++kb)  // R1: F[i][k] + S2(k+1, j)
-            step(T + r0 * LD + 8 * kb + 2 * kp, SJ + (8 * kb + 2 * kp + 1) * LD + c0);
-#pragma unroll 4
-        for (int kb = bi + 1; kb <= (t == 0 ? bj : 7); ++kb)  // R2: S2(i, k-1) + F[k][j]
-            step(SX + r0 * LD + 8 * kb + 2 * kp, T + (8 * kb + 2 * kp) * LD + c0);
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                v[i][j] = fmaxf(v[i][j], __shfl_xor_sync(0xffffffffu, v[i][j], 1));
-                v[i][j] = fmaxf(v[i][j], __shfl_xor_sync(0xffffffffu, v[i][j], 2));
-            }
-        if (kp < 2) {  // lane kp takes row r0 + kp
-            float4 *o = reinterpret_cast<float4 *>(T + (r0 + kp) * LD + c0);
-            float4 x = *o;
-            x.x = fmaxf(x.x, v[kp == 0 ? 0 : 1][0]);
-            x.y = fmaxf(x.y, v[kp == 0 ? 0 : 1][1]);
-            x.z = fmaxf(x.z, v[kp == 0 ? 0 : 1][2]);
-            x.w = fmaxf(x.w, v[kp == 0 ? 0 : 1][3]);
-            *o = x;
-        }
-        __syncwarp();
-        // the block's own wavefront: lane la has row 8bi+la; at step s it computes column 8bj + b,
-        // b = s - 7 + la (the lanes 8.. repeat lanes 0..7)
-        const int row = 8 * bi + la, e0 = 64 * t + 8 * D;
-        const float *Tr = T + row * LD + 8 * bj, *wr = wt + LD * bI[row] + 8 * bj;
-        float vs[15], ws[15], qs[8];
-#pragma unroll
-        for (int s = 0; s < 15; ++s) {
-            const int b = min(max(s - 7 + la, 0), 7);
-            vs[s] = Tr[b];
-            ws[s] = wr[b];
-            if (e0 + s - 7 < 4) ws[s] = NEG_INF;  // SW2 needs j2-i2 >= 4
-        }
-        // SW2 from outside the block: of column 0 (any row), and of the last row
-#pragma unroll
-        for (int s = 0; s < 8; ++s) qs[s] = Tr[LD + (la == 7 ? s - 1 : -1)];
-        float cx[3];  // S2(i2, i2+4 ..) for R2 from rows five to seven below, inside the block
-#pragma unroll
-        for (int x = 0; x < 3; ++x) cx[x] = la + x + 5 < 8 ? SX[row * LD + row + 5 + x] : NEG_INF;
-        float n[15], under = NEG_INF, left = NEG_INF, diag = NEG_INF;  // (row+1, b), (row, b-1), (row+1, b-1)
-#pragma unroll
-        for (int s = 0; s < 15; ++s) {
-            const int b = s - 7 + la;
-            float far = NEG_INF;
-#pragma unroll
-            for (int x = 0; x < 3; ++x)
-                if (s >= 5 + x) {  // five, six, seven diagonals back: R1 in the lane, R2 from lane la + 5 + x
-                    const int bc = min(max(b - 4 - x, 0), 7);  // S2(8bj + b-5-x + 1, 8bj + b)
-                    const float r1 = n[s - 5 - x] + SJ[(8 * bj + bc) * LD + 8 * bj + min(max(b, 0), 7)];
-                    const float r2 = __shfl_down_sync(0xffffffffu, n[s - 5 - x], 5 + x, 8) + cx[x];
-                    far = fmax3(far, r1, r2);
-                }
-            under = s > 0 ? __shfl_down_sync(0xffffffffu, n[s - 1], 1, 8) : NEG_INF;
-            if (la == 7) under = NEG_INF;
-            const float q = la == 7 ? qs[s < 8 ? s : 7] : (b == 0 ? qs[0] : diag);
-            const float r = fmaxf(fmax3(fmaxf(vs[s], far), left, under), q + ws[s]);
-            n[s] = b >= 0 && b < 8 && 8 * bj + b < ncol ? r : NEG_INF;
-            if (lane < 8 && b >= 0 && b < 8 && 8 * bj + b < ncol) T[row * LD + 8 * bj + b] = n[s];
-            diag = under;
-            left = n[s];
-        }
-    }
-    __syncthreads();
+    block_wave<LD, TILE_THREADS / 32>(T, SX, SJ, wt, bI, t == 0, 8, ncol, 64 * t);  // (starts and ends with a barrier)
     // the tile image: S1(i1,j1) on the subdiagonal of a diagonal tile, -inf elsewhere outside the table;
     // then the closing pieces of the block columns: S1 pieces, or row 0 of the tile below (halo)
     for (int q4 = tid; q4 < nblk * 16 + 16; q4 += TILE_THREADS) {

@@ -1,6 +1,6 @@
 """The finalize of tables up to width 64 bit for bit against the oracle: strand-2 lengths around its
-batches of five inner diagonals, around the 32 lanes of a warp and at the ends of every width class,
-and launches of enough cells for the form with fewer threads per cell."""
+8x8 blocks and at the ends of every width class, and launches of enough cells for the
+form with fewer threads per cell."""
 import numpy as np
 import pytest
 
