@@ -104,7 +104,8 @@ struct Plan {
     int bases_bytes = 0;
     int maxM = 0;
     // per step and Np class: ranges in the job arrays. d = the step: the outer diagonal, for tile tables the
-    // outer diagonal plus the tile diagonal. np = inner table width class; strip (product launches): strips of diagonals d .. d+T-1
+    // outer diagonal plus the tile diagonal. np = inner table width class; strip (product launches): strips
+    // of diagonals d .. d+T-1
     // cap: at most this many CTAs (0: as many as are resident), from the class shares
     // r0_kernel launches of one pair: q offset pairs per job of `edge` (0: jobs from the list)
     struct Launch {
@@ -175,7 +176,7 @@ struct bpmax_ctx {
     int wide_stages = 2;                            // shared-memory stages of the tile-image product (2 or 3)
     int class_share = 0;                            // cap each width class's product CTAs by its share of the work
     int persist = 0;  // width classes <= 64 by the persistent kernel: 0 no, 1 side by side, 2 one after another
-    long strip_tasks = 3400;                        // least product tasks per SM of a strip launch
+    long strip_tasks = 1200;                        // least product tasks per SM of a strip launch
     int persist_occ[9] = {};                        // resident persistent-fill CTAs per SM, per width class
     // bounded waits of the product kernels: time limit of one wait, and the one-shot test mode in
     // which the next fill's product kernels issue no copies (their first waits run out)
@@ -510,9 +511,11 @@ int build_plan(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int
                 // offsets [0, d-1], of which cell t of a strip takes those >= t. The first t offset pairs
                 // of diagonal d+t, which meet diagonals >= d, are the jobs of r0_kernel. Diagonals
                 // with little work keep r0_kernel alone: a strip launch adds a launch to the chain and
-                // clears T merge tiles per CTA. Fill ms with strips everywhere / from 3,400 tasks (28
-                // width-64 items) per SM / nowhere: 37x23 0.66 / 0.57 / 0.55, 128x64 6.69 / 6.57 / 6.52,
-                // 200x40 7.93 / 7.63 / 7.64, 200x64 13.8 / 13.7 / 14.2, 256x64 21.8 / 21.4 / 23.4.
+                // clears T merge tiles per CTA. Fill ms with strips everywhere / from 400 / 1,200 (10 width-64
+                // items) / 3,400 tasks per SM / nowhere: 37x23 0.41 / 0.35 / 0.35 / 0.35 / 0.35, 100x64
+                // 2.56 / 2.56 / 2.56 / 2.66 / 2.67, 128x64 3.86 / 3.86 / 3.86 / 4.10 / 4.10, 128x32 1.93 /
+                // 1.88 / 1.81 / 1.82 / 1.81, 200x64 9.1 / 9.1 / 9.1 / 9.1 / 10.2, 256x64 15.5 / 15.5 / 15.5 /
+                // 15.5 / 18.1.
                 const int NB = np / 8, G = R0_TAB_ITEMS[NB];
                 const long long P2 = (d + 1) / 2;  // offset pairs per cell
                 long long edge = P2;               // offset pairs per cell of r0_kernel's jobs
@@ -607,9 +610,9 @@ template <int STAGES>
 void launch_r0_wide_t(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
 {
     const int grid = std::min(L.count, L.cap > 0 ? L.cap : std::max(1, ctx->wide_occ[STAGES]) * ctx->sms);
-    launch_chain(
-        false, grid, WideCfg<STAGES>::THREADS, WideCfg<STAGES>::SMEM, s, r0_wide_kernel<STAGES>, (const R0JobW *)ctx->r0wjobs.p + L.first, L.count, (const PairDesc *)ctx->pairs.p, (float *)ctx->F.p,
-        (const float *)ctx->S.p, wait_ctl(ctx));
+    launch_chain(false, grid, WideCfg<STAGES>::THREADS, WideCfg<STAGES>::SMEM, s, r0_wide_kernel<STAGES>,
+                 (const R0JobW *)ctx->r0wjobs.p + L.first, L.count, (const PairDesc *)ctx->pairs.p, (float *)ctx->F.p,
+                 (const float *)ctx->S.p, wait_ctl(ctx));
 }
 
 void launch_r0_wide(bpmax_ctx *ctx, const Plan &P, const Plan::Launch &L, cudaStream_t s)
@@ -623,10 +626,12 @@ void launch_r0_wide(bpmax_ctx *ctx, const Plan &P, const Plan::Launch &L, cudaSt
 // the tiles of one step, and S1 of outer diagonal step+1
 void launch_fin_tiles(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
 {
-    launch_chain(false, L.tile_count + (L.s1_count + TILE_THREADS / 32 - 1) / (TILE_THREADS / 32), TILE_THREADS, TILE_SMEM, s,
-                 tile_final_kernel, (const TileJob *)ctx->tilejobs.p + L.tile_first, L.tile_count,
-                 (const CellJob *)ctx->celljobs.p + L.s1_first, L.s1_count, (const PairDesc *)ctx->pairs.p, (float *)ctx->F.p,
-                 (float *)ctx->S.p, (const uint8_t *)ctx->bases.p, ctx->W, L.d);
+    const int grid = L.tile_count + (L.s1_count + TILE_THREADS / 32 - 1) / (TILE_THREADS / 32);
+    launch_chain(false, grid, TILE_THREADS, TILE_SMEM, s,
+                 L.tile_count > 2 * ctx->sms ? tile_final_kernel<3> : tile_final_kernel<2>,
+                 (const TileJob *)ctx->tilejobs.p + L.tile_first, L.tile_count,
+                 (const CellJob *)ctx->celljobs.p + L.s1_first, L.s1_count, (const PairDesc *)ctx->pairs.p,
+                 (float *)ctx->F.p, (float *)ctx->S.p, (const uint8_t *)ctx->bases.p, ctx->W, L.d);
 }
 
 template <int NB, int V>
@@ -642,9 +647,9 @@ void launch_r0_v(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
 template <int NB>
 void launch_strip(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
 {
-    launch_chain(
-        ctx->one_chain, std::min(L.count, L.cap), StripCfg<NB>::THREADS, StripCfg<NB>::SMEM, s, r0_strip_kernel<NB>, (const StripJob *)ctx->stripjobs.p + L.first, L.count, (const PairDesc *)ctx->pairs.p, (float *)ctx->F.p, L.d,
-        wait_ctl(ctx));
+    launch_chain(ctx->one_chain, std::min(L.count, L.cap), StripCfg<NB>::THREADS, StripCfg<NB>::SMEM, s,
+                 r0_strip_kernel<NB>, (const StripJob *)ctx->stripjobs.p + L.first, L.count,
+                 (const PairDesc *)ctx->pairs.p, (float *)ctx->F.p, L.d, wait_ctl(ctx));
 }
 
 template <int NB>
@@ -670,17 +675,18 @@ template <int NB, int T>
 void launch_fin_t(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
 {
     using Sh = FinShape<8 * NB, T>;
-    launch_chain(
-        ctx->one_chain && T < 512, L.count + (L.s1_count + Sh::WARPS - 1) / Sh::WARPS, Sh::THREADS, Sh::SMEM, s, finalize_small_kernel<8 * NB, T>,
-        (const CellJob *)ctx->celljobs.p + L.first, L.count, (const CellJob *)ctx->celljobs.p + L.s1_first, L.s1_count,
-        (const PairDesc *)ctx->pairs.p, (float *)ctx->F.p, (float *)ctx->S.p, (const uint8_t *)ctx->bases.p, ctx->W,
-        L.d, ctx->plan.ref);
+    launch_chain(ctx->one_chain && T < 512, L.count + (L.s1_count + Sh::WARPS - 1) / Sh::WARPS, Sh::THREADS,
+                 Sh::SMEM, s, finalize_small_kernel<8 * NB, T>, (const CellJob *)ctx->celljobs.p + L.first, L.count,
+                 (const CellJob *)ctx->celljobs.p + L.s1_first, L.s1_count, (const PairDesc *)ctx->pairs.p,
+                 (float *)ctx->F.p, (float *)ctx->S.p, (const uint8_t *)ctx->bases.p, ctx->W, L.d, ctx->plan.ref);
 }
 
 template <int NB>
 void launch_fin(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
 {
-    if (L.count >= FIN_BULK_CELLS) return launch_fin_t<NB, FIN_BULK_THREADS>(ctx, L, s);
+    if (L.count >= fin_bulk_cells(8 * NB)) return launch_fin_t<NB, FIN_BULK_THREADS>(ctx, L, s);
+    if constexpr (fin_bulk_cells(8 * NB) > FIN_MID_CELLS)
+        if (L.count >= FIN_MID_CELLS) return launch_fin_t<NB, FIN_MID_THREADS>(ctx, L, s);
     launch_fin_t<NB, fin_threads(8 * NB)>(ctx, L, s);
 }
 
@@ -689,18 +695,22 @@ void launch_r0only_fin(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
     const CellJob *jobs = (const CellJob *)ctx->celljobs.p + L.first;
     const PairDesc *pd = (const PairDesc *)ctx->pairs.p;
     const float *vals = (const float *)ctx->r0vals.p;
+    auto go = [&](auto kernel) {
+        launch_chain(ctx->one_chain, L.count, 128, 0, s, kernel, jobs, pd, (float *)ctx->F.p, vals, L.d);
+    };
     switch (L.np > MAX_SMALL_NP ? 0 : L.np / 8) {
     case 0:
-        launch_chain(ctx->one_chain, dim3(L.count, L.np / 64), 256, 0, s, r0only_finalize_tile_kernel, jobs, pd, (float *)ctx->F.p, vals, L.d);
+        launch_chain(ctx->one_chain, dim3(L.count, L.np / 64), 256, 0, s, r0only_finalize_tile_kernel, jobs, pd,
+                     (float *)ctx->F.p, vals, L.d);
         break;
-    case 1: launch_chain(ctx->one_chain, L.count, 128, 0, s, r0only_finalize_small_kernel<8>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
-    case 2: launch_chain(ctx->one_chain, L.count, 128, 0, s, r0only_finalize_small_kernel<16>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
-    case 3: launch_chain(ctx->one_chain, L.count, 128, 0, s, r0only_finalize_small_kernel<24>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
-    case 4: launch_chain(ctx->one_chain, L.count, 128, 0, s, r0only_finalize_small_kernel<32>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
-    case 5: launch_chain(ctx->one_chain, L.count, 128, 0, s, r0only_finalize_small_kernel<40>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
-    case 6: launch_chain(ctx->one_chain, L.count, 128, 0, s, r0only_finalize_small_kernel<48>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
-    case 7: launch_chain(ctx->one_chain, L.count, 128, 0, s, r0only_finalize_small_kernel<56>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
-    default: launch_chain(ctx->one_chain, L.count, 128, 0, s, r0only_finalize_small_kernel<64>, jobs, pd, (float *)ctx->F.p, vals, L.d); break;
+    case 1: go(r0only_finalize_small_kernel<8>); break;
+    case 2: go(r0only_finalize_small_kernel<16>); break;
+    case 3: go(r0only_finalize_small_kernel<24>); break;
+    case 4: go(r0only_finalize_small_kernel<32>); break;
+    case 5: go(r0only_finalize_small_kernel<40>); break;
+    case 6: go(r0only_finalize_small_kernel<48>); break;
+    case 7: go(r0only_finalize_small_kernel<56>); break;
+    default: go(r0only_finalize_small_kernel<64>); break;
     }
 }
 
@@ -723,13 +733,19 @@ int set_smem_attr(bpmax_ctx *ctx)
         (st = prefer_smem(ctx, finalize_small_kernel<8 * NB>)) || (st = prefer_smem(ctx, r0only_finalize_small_kernel<8 * NB>)))
         return st;
     if ((st = prefer_smem(ctx, finalize_small_kernel<8 * NB, FIN_BULK_THREADS>))) return st;
+    if constexpr (fin_bulk_cells(8 * NB) > FIN_MID_CELLS) {
+        if ((st = prefer_smem(ctx, finalize_small_kernel<8 * NB, FIN_MID_THREADS>))) return st;
+        CK(cudaFuncSetAttribute(finalize_small_kernel<8 * NB, FIN_MID_THREADS>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)FinShape<8 * NB, FIN_MID_THREADS>::SMEM));
+    }
     if constexpr (NB >= STRIP_MIN_NB) {
         if ((st = prefer_smem(ctx, r0_strip_kernel<NB>))) return st;
         CK(cudaFuncSetAttribute(r0_strip_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)StripCfg<NB>::SMEM));
     }
     if (NB == 8)
         if ((st = prefer_smem(ctx, r0_wide_kernel<2>)) || (st = prefer_smem(ctx, r0_wide_kernel<3>)) ||
-            (st = prefer_smem(ctx, tile_final_kernel)))
+            (st = prefer_smem(ctx, tile_final_kernel<2>)) || (st = prefer_smem(ctx, tile_final_kernel<3>)))
             return st;
     CK(cudaFuncSetAttribute(r0_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)R0Cfg<NB>::SMEM));
     CK(cudaFuncSetAttribute(r0_kernel<NB, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)R0Cfg<NB, 1>::SMEM));
@@ -751,7 +767,8 @@ int set_smem_attr(bpmax_ctx *ctx)
         CK(cudaFuncSetAttribute(r0_wide_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WideCfg<3>::SMEM));
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctx->wide_occ[2], r0_wide_kernel<2>, 128, WideCfg<2>::SMEM));
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctx->wide_occ[3], r0_wide_kernel<3>, 128, WideCfg<3>::SMEM));
-        CK(cudaFuncSetAttribute(tile_final_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TILE_SMEM));
+        CK(cudaFuncSetAttribute(tile_final_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TILE_SMEM));
+        CK(cudaFuncSetAttribute(tile_final_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TILE_SMEM));
     }
     return BPMAX_OK;
 }
@@ -800,7 +817,8 @@ int enqueue_fill(bpmax_ctx *ctx, Plan &P, KernelProfile *kp = nullptr)
             if (P.pairs[p].Np > S2_ONE_CTA_NP)
                 for (int d = 4; d < P.pairs[p].N; ++d, ++launches)
                     launch_chain(
-                        ctx->one_chain, (P.pairs[p].N - d + 7) / 8, 256, 0, ctx->stream, s2_diag_kernel, (const PairDesc *)ctx->pairs.p, p, (const uint8_t *)ctx->bases.p, (float *)ctx->S.p, ctx->W, d);
+                        ctx->one_chain, (P.pairs[p].N - d + 7) / 8, 256, 0, ctx->stream, s2_diag_kernel,
+                        (const PairDesc *)ctx->pairs.p, p, (const uint8_t *)ctx->bases.p, (float *)ctx->S.p, ctx->W, d);
         launches += 1;
         if (P.classes.back() > MAX_SMALL_NP) {
             launch_chain(ctx->one_chain, dim3(64, (int)P.pairs.size()), 256, 0, ctx->stream, s2_aux_kernel,

@@ -91,8 +91,8 @@ __device__ __forceinline__ void chain_wait()
 __device__ __forceinline__ float fmax3(float a, float b, float c) { return fmaxf(fmaxf(a, b), c); }
 
 // ------------------------------------------------------------------------------------------
-// Tile images: inner tables of width Np = 64 * NT > 64 are stored per outer cell as the upper triangle of NT x NT tiles of 64 x 64 in row-major tile-triangle order. A
-// diagonal tile is a width-64 cell image (above); an off-diagonal ("dense") tile holds all 64 of
+// Tile images: inner tables of width Np = 64 * NT > 64 are stored per outer cell as the upper triangle of
+// NT x NT tiles of 64 x 64 in row-major tile-triangle order. A diagonal tile is a width-64 cell image (above); an off-diagonal ("dense") tile holds all 64 of
 // its 8x8 blocks in block columns at WIDE_DENSE_COLBASE (wide_tables.inc), each column closed by a
 // halo piece: row 0 of block (0, bj) of the tile below, the row after the tile, so the row-shifted
 // operand of any tile is one image. Rows and columns >= N are -inf.
@@ -225,13 +225,15 @@ struct CellJob {
 
 // threads per cell. Up to one cell per SM what counts is the latency of one cell: many threads for its
 // loads and products. Launches of more cells run several CTAs per SM, which hide each other's latency,
-// and four warps per cell then idle least at the barriers. Fill ms with the latency threads for up to
-// 1,024 / 296 / 148 cells: 1024x64 622 / 602 / 601, 256x64 16.2 / 16.2 / 15.8; the 512-pair batch at
-// 256 / 160 / 128 threads beyond: 428 / 419 / 418. Up to 148 cells 128x64 takes 4.44 with 256 threads
+// and four warps per cell then idle least at the barriers; in between, up to three cells per SM, eight
+// warps for widths >= 48 (256x64 15.8 -> 15.6, 200x56 7.80 -> 7.64, 512x64 86.9 -> 86.0). Fill ms with the
+// latency threads for up to 1,024 / 296 / 148 cells: 1024x64 622 / 602 / 601, 256x64 16.2 / 16.2 / 15.8;
+// the 512-pair batch at 256 / 160 / 128 threads beyond: 428 / 419 / 418. Up to 148 cells 128x64 takes 4.44 with 256 threads
 // and 4.09 with 512, 64x32 0.83 with 128, 0.73 with 256 and 0.71 with 384.
 constexpr int fin_threads(int NP) { return NP >= 48 ? 512 : (NP >= 32 ? 384 : 128); }
 constexpr int FIN_BULK_THREADS = 128;
-constexpr int FIN_BULK_CELLS = 149;
+constexpr int FIN_MID_THREADS = 256, FIN_MID_CELLS = 149;  // from this many cells
+constexpr int fin_bulk_cells(int NP) { return NP >= 48 ? 445 : FIN_MID_CELLS; }
 // element (r, c) of tile (I2, J2) of an outer cell in the reference layout (tiles of T+1 rows, the
 // last one the halo; R = padding rows/columns of the first tile row/column); val(i2, j2) gives the
 // cell's inner value for 0 <= i2 <= j2 < N, the only entries read

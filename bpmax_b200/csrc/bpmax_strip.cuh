@@ -27,7 +27,9 @@
 // tasks alone on resident stages take 835. Measured per item (M = 512, d = 244, 193,842 items): 957
 // cycles, 943 with the copies left out; the refill's address arithmetic once took 105 of 1,092 (the
 // whole ring waits for it), hence the cursor that only adds. r0_kernel took 1,240 with 20,160 bytes
-// per item, against 13,440 here. Fill: 1024x64 766 -> 661 ms, the 512-pair batch 523 -> 460 ms.
+// per item, against 13,440 here. Fill: 1024x64 766 -> 661 ms, the 512-pair batch 523 -> 460 ms;
+// 661 -> 616 and 428 -> 424 since cell t takes every offset that meets final tables (before, only those that
+// all T cells share).
 #pragma once
 #include <cstddef>
 

@@ -116,8 +116,11 @@ __device__ __forceinline__ void s1_cell(const CellJob &job, const PairDesc *__re
     if (lane == 0) S1[i * M + j] = fmaxf(S1[(i + 1) * M + (j - 1)] + score_w(w, s1[i], s1[j]), red);
 }
 
-// CTAs [0, njobs): one tile each; after them one warp per S1 cell (i, i+step+1)
-__global__ void __launch_bounds__(TILE_THREADS, 2)
+// CTAs [0, njobs): one tile each; after them one warp per S1 cell (i, i+step+1). MINB: CTAs per SM, 2
+// (128 registers) or, for steps of more tiles than two per SM, 3 (80). Fill ms at 2 / 3: 90x70 (at most 90
+// tiles) 6.12 / 6.24, 90x130 14.5 / 14.7, 256x256 680 / 676, 32x1024 81.2 / 80.1.
+template <int MINB>
+__global__ void __launch_bounds__(TILE_THREADS, MINB)
 tile_final_kernel(const TileJob *__restrict__ jobs, int njobs, const CellJob *__restrict__ s1jobs, int ns1,
                   const PairDesc *__restrict__ pairs, float *__restrict__ F, float *__restrict__ S,
                   const uint8_t *__restrict__ bases, Weights W, int step)
