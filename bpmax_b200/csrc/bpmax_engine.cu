@@ -1159,12 +1159,18 @@ int copy_out(bpmax_ctx *ctx, void *dst, const void *src, size_t bytes)
 {
     const int threads = (int)std::min<size_t>(std::min<size_t>(COPY_THREADS, bytes / COPY_CHUNK),
                                               std::max(1u, std::thread::hardware_concurrency()));
-    if (bytes < COPY_SPLIT || threads < 2 || is_pinned(dst)) {
+    bool split = bytes >= COPY_SPLIT && threads >= 2 && !is_pinned(dst);
+    if (split && !ctx->copy_stage &&
+        cudaMallocHost(&ctx->copy_stage, 2 * COPY_THREADS * COPY_CHUNK) != cudaSuccess) {
+        cudaGetLastError();  // no pinned memory left: one copy, as for small tables
+        ctx->copy_stage = nullptr;
+        split = false;
+    }
+    if (!split) {
         CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
         return BPMAX_OK;
     }
-    if (!ctx->copy_stage) CK(cudaMallocHost(&ctx->copy_stage, 2 * COPY_THREADS * COPY_CHUNK));
     CK(cudaEventRecord(ctx->fork_ev, ctx->stream));
     cudaError_t errs[COPY_THREADS] = {};
     auto work = [&](int t) {
