@@ -422,10 +422,10 @@ def main_b200(args, world, rank, local):
 
 
 # DRAM bytes (read + write) per product item (one outer cell and one k1) of the R0 kernel with
-# inner width 64: ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch of a 512 x 64 fill
-# (outer diagonal 256: 256 cells x 256 items, 1.079 GB) divided by its items. The kernel's traffic
+# inner width 64: ncu dram__bytes_read.sum + dram__bytes_write.sum of one strip launch of a 512 x 64
+# fill (outer diagonals 241-243: 194,402 items, 1.395 GB) divided by its items. The kernel's traffic
 # grows with the items it processes, so a launch's traffic is this figure times its items.
-R0_DRAM_BYTES_PER_ITEM_NP64 = 16466
+R0_DRAM_BYTES_PER_ITEM_NP64 = 7176
 
 
 def r0_roofline(wl, r0_ms, r0_n, r0_terms, peak_terms_s, clocks):
@@ -439,7 +439,7 @@ def r0_roofline(wl, r0_ms, r0_n, r0_terms, peak_terms_s, clocks):
     terms_per_launch = r0_terms / max(r0_n, 1)
     achieved = 2 * terms_per_launch / per_launch_s / 1e12  # TFLOP/s
     peak = 2 * peak_terms_s / 1e12
-    out = {"bound": "fp32_alu", "kernel": "r0_kernel (R0+R3+R4 max-plus product)", "achieved": achieved, "peak": peak,
+    out = {"bound": "fp32_alu", "kernel": "r0_strip_kernel and r0_kernel (R0+R3+R4 max-plus product)", "achieved": achieved, "peak": peak,
            "unit": "TFLOP/s", "frac": achieved / peak, "traffic": None,
            "peak_source": "measured live: bpmax_gpu_maxplus_peak (packed fp32 add + 3-input max, every sum new, register resident, all SMs)",
            "ops_per_term": 2, "achieved_Gterms_s": achieved / 2 * 1e3, "launches": r0_n,
