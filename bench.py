@@ -439,7 +439,7 @@ def r0_roofline(wl, r0_ms, r0_n, r0_terms, peak_terms_s, clocks):
     terms_per_launch = r0_terms / max(r0_n, 1)
     achieved = 2 * terms_per_launch / per_launch_s / 1e12  # TFLOP/s
     peak = 2 * peak_terms_s / 1e12
-    out = {"bound": "fp32_alu", "kernel": "r0_strip_kernel and r0_kernel (R0+R3+R4 max-plus product)", "achieved": achieved, "peak": peak,
+    out = {"bound": "fp32_alu", "kernel": "product kernels (R0+R3+R4 max-plus)", "achieved": achieved, "peak": peak,
            "unit": "TFLOP/s", "frac": achieved / peak, "traffic": None,
            "peak_source": "measured live: bpmax_gpu_maxplus_peak (packed fp32 add + 3-input max, every sum new, register resident, all SMs)",
            "ops_per_term": 2, "achieved_Gterms_s": achieved / 2 * 1e3, "launches": r0_n,
