@@ -126,6 +126,7 @@ struct Plan {
     int steps = 0;  // of the fill: outer diagonals, and the tile diagonals after the last
     std::vector<CellJob> cell_jobs;
     std::vector<int> classes;  // distinct inner widths, ascending
+    std::vector<int> wide_pairs;  // indices of the pairs with tile tables
     int pairs_per_job = 0, merge_items = 0, class_streams = 1;  // tunables the plan was built with
     int r0_variant = 0, wide_stages = 2, class_share = 0, persist = 0;
     long strip_tasks = 0;
@@ -157,7 +158,7 @@ struct bpmax_ctx {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     Weights W;
     std::string err;
-    DevBuf F, S, bases, pairs, r0jobs, stripjobs, r0wjobs, tilejobs, celljobs, scores, conv, tbstack, grads, tbstatus, errflag;
+    DevBuf F, S, bases, pairs, r0jobs, stripjobs, r0wjobs, tilejobs, celljobs, widepairs, scores, conv, tbstack, grads, tbstatus, errflag;
     DevBuf r0vals;         // R0-only mode: seq1 then seq2 of the pair, as floats
     DevBuf pq, pcnt, pneed;  // persistent fill: work queue; counters (class heads, diagonals, cells); jobs per cell
     bool copyout = false;    // the next fill copies the reference layout out per diagonal (graph path)
@@ -446,6 +447,7 @@ int build_plan(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int
         if (pd.Np > MAX_SMALL_NP) {  // S2 as tile images
             pd.S2x_off = s;
             s = align64(s + (long long)pd.Np * pd.Np);
+            P.wide_pairs.push_back(p);
         }
         pd.seq1_off = b;
         b += Ms[p];
@@ -820,9 +822,9 @@ int enqueue_fill(bpmax_ctx *ctx, Plan &P, KernelProfile *kp = nullptr)
                         ctx->one_chain, (P.pairs[p].N - d + 7) / 8, 256, 0, ctx->stream, s2_diag_kernel,
                         (const PairDesc *)ctx->pairs.p, p, (const uint8_t *)ctx->bases.p, (float *)ctx->S.p, ctx->W, d);
         launches += 1;
-        if (P.classes.back() > MAX_SMALL_NP) {
-            launch_chain(ctx->one_chain, dim3(64, (int)P.pairs.size()), 256, 0, ctx->stream, s2_aux_kernel,
-                         (const PairDesc *)ctx->pairs.p, (float *)ctx->S.p);
+        if (!P.wide_pairs.empty()) {
+            launch_chain(ctx->one_chain, dim3((int)P.wide_pairs.size(), 64), 256, 0, ctx->stream, s2_aux_kernel,
+                         (const int *)ctx->widepairs.p, (const PairDesc *)ctx->pairs.p, (float *)ctx->S.p);
             launches += 1;
         }
     }
@@ -982,6 +984,7 @@ int prepare(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int> &
         if ((st = ensure(ctx, ctx->stripjobs, P.strip_jobs.size() * sizeof(StripJob))) != BPMAX_OK) return st;
         if ((st = ensure(ctx, ctx->r0wjobs, P.r0w_jobs.size() * sizeof(R0JobW))) != BPMAX_OK) return st;
         if ((st = ensure(ctx, ctx->tilejobs, P.tile_jobs.size() * sizeof(TileJob))) != BPMAX_OK) return st;
+        if ((st = ensure(ctx, ctx->widepairs, P.wide_pairs.size() * sizeof(int))) != BPMAX_OK) return st;
         if (P.persistent) {
             if ((st = ensure(ctx, ctx->pq, P.pitems.size() * sizeof(PItem))) != BPMAX_OK) return st;
             if ((st = ensure(ctx, ctx->pneed, P.prod_need.size() * sizeof(int))) != BPMAX_OK) return st;
@@ -1005,6 +1008,9 @@ int prepare(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int> &
                                ctx->stream));
         if (!P.tile_jobs.empty())
             CK(cudaMemcpyAsync(ctx->tilejobs.p, P.tile_jobs.data(), P.tile_jobs.size() * sizeof(TileJob),
+                               cudaMemcpyHostToDevice, ctx->stream));
+        if (!P.wide_pairs.empty())
+            CK(cudaMemcpyAsync(ctx->widepairs.p, P.wide_pairs.data(), P.wide_pairs.size() * sizeof(int),
                                cudaMemcpyHostToDevice, ctx->stream));
         CK(cudaMemcpyAsync(ctx->celljobs.p, P.cell_jobs.data(), P.cell_jobs.size() * sizeof(CellJob), cudaMemcpyHostToDevice, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
@@ -1289,7 +1295,7 @@ void bpmax_gpu_destroy(bpmax_ctx *ctx)
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     if (ctx->plan.graph) cudaGraphExecDestroy(ctx->plan.graph);
     for (DevBuf *b : {&ctx->tbstack, &ctx->grads, &ctx->tbstatus, &ctx->F, &ctx->S, &ctx->bases, &ctx->pairs,
-                      &ctx->r0jobs, &ctx->stripjobs, &ctx->r0wjobs, &ctx->tilejobs, &ctx->pq, &ctx->pcnt, &ctx->pneed, &ctx->celljobs,
+                      &ctx->r0jobs, &ctx->stripjobs, &ctx->r0wjobs, &ctx->tilejobs, &ctx->widepairs, &ctx->pq, &ctx->pcnt, &ctx->pneed, &ctx->celljobs,
                       &ctx->scores, &ctx->conv, &ctx->refdev, &ctx->errflag,
                       &ctx->r0vals})
         if (b->p) cudaFree(b->p);

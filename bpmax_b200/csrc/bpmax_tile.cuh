@@ -40,19 +40,20 @@ struct TileJob {
 };
 
 // ------------------------------------------------------------------------------------------
-// The dense tile images (with halo pieces) of S2 of every pair with Np > 64, S2 over the reversed strand
-// 2 (V3/bpmax_verify.c:560-571); -inf in columns >= N.
+// The dense tile images (with halo pieces) of S2 of the pairs with Np > 64, S2 over the reversed strand
+// 2 (V3/bpmax_verify.c:560-571); -inf in columns >= N. The pairs are on x: a batch may hold more of them than
+// a grid's y extent (65,535). Only wide pairs have CTAs: with 64 for every pair, one wide pair among 20,000 narrow
+// ones added 1.47 ms to the batch, now 0.13.
 // ------------------------------------------------------------------------------------------
-__global__ void s2_aux_kernel(const PairDesc *__restrict__ pairs, float *__restrict__ S)
+__global__ void s2_aux_kernel(const int *__restrict__ wide, const PairDesc *__restrict__ pairs, float *__restrict__ S)
 {
-    const PairDesc pd = pairs[blockIdx.y];
+    const PairDesc pd = pairs[wide[blockIdx.x]];
     const int Np = pd.Np, N = pd.N, NT = Np >> 6;
     chain_wait();
-    if (Np <= 64) return;
     const float *S2 = S + pd.S2_off;
     float *img = S + pd.S2x_off;
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < (long long)Np * Np;
-         q += (long long)gridDim.x * blockDim.x) {
+    for (long long q = blockIdx.y * (long long)blockDim.x + threadIdx.x; q < (long long)Np * Np;
+         q += (long long)gridDim.y * blockDim.x) {
         const int r = (int)(q / Np), c = (int)(q % Np), I = r >> 6, J = c >> 6, o = 4 * c_wide_dense_colbase[(c & 63) >> 3];
         const float v = c < N ? S2[q] : NEG_INF;
         if (I < J) img[s2_image_off(NT, I, J) + o + 4 * 17 * ((r & 63) >> 3) + 8 * (r & 7) + (c & 7)] = v;
