@@ -686,9 +686,9 @@ void launch_fin_t(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
 template <int NB>
 void launch_fin(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
 {
-    if (L.count >= fin_bulk_cells(8 * NB)) return launch_fin_t<NB, FIN_BULK_THREADS>(ctx, L, s);
-    if constexpr (fin_bulk_cells(8 * NB) > FIN_MID_CELLS)
-        if (L.count >= FIN_MID_CELLS) return launch_fin_t<NB, FIN_MID_THREADS>(ctx, L, s);
+    if (L.count > fin_bulk_per_sm(8 * NB) * ctx->sms) return launch_fin_t<NB, FIN_BULK_THREADS>(ctx, L, s);
+    if constexpr (fin_has_mid(8 * NB))
+        if (L.count > ctx->sms) return launch_fin_t<NB, FIN_MID_THREADS>(ctx, L, s);
     launch_fin_t<NB, fin_threads(8 * NB)>(ctx, L, s);
 }
 
@@ -735,7 +735,7 @@ int set_smem_attr(bpmax_ctx *ctx)
         (st = prefer_smem(ctx, finalize_small_kernel<8 * NB>)) || (st = prefer_smem(ctx, r0only_finalize_small_kernel<8 * NB>)))
         return st;
     if ((st = prefer_smem(ctx, finalize_small_kernel<8 * NB, FIN_BULK_THREADS>))) return st;
-    if constexpr (fin_bulk_cells(8 * NB) > FIN_MID_CELLS) {
+    if constexpr (fin_has_mid(8 * NB)) {
         if ((st = prefer_smem(ctx, finalize_small_kernel<8 * NB, FIN_MID_THREADS>))) return st;
         CK(cudaFuncSetAttribute(finalize_small_kernel<8 * NB, FIN_MID_THREADS>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize,

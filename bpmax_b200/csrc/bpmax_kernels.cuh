@@ -231,9 +231,9 @@ struct CellJob {
 // the 512-pair batch at 256 / 160 / 128 threads beyond: 428 / 419 / 418. Up to 148 cells 128x64 takes 4.44 with 256 threads
 // and 4.09 with 512, 64x32 0.83 with 128, 0.73 with 256 and 0.71 with 384.
 constexpr int fin_threads(int NP) { return NP >= 48 ? 512 : (NP >= 32 ? 384 : 128); }
-constexpr int FIN_BULK_THREADS = 128;
-constexpr int FIN_MID_THREADS = 256, FIN_MID_CELLS = 149;  // from this many cells
-constexpr int fin_bulk_cells(int NP) { return NP >= 48 ? 445 : FIN_MID_CELLS; }
+constexpr int FIN_BULK_THREADS = 128, FIN_MID_THREADS = 256;
+constexpr int fin_bulk_per_sm(int NP) { return NP >= 48 ? 3 : 1; }  // bulk launches: more cells per SM than this
+constexpr bool fin_has_mid(int NP) { return fin_bulk_per_sm(NP) > 1; }
 // element (r, c) of tile (I2, J2) of an outer cell in the reference layout (tiles of T+1 rows, the
 // last one the halo; R = padding rows/columns of the first tile row/column); val(i2, j2) gives the
 // cell's inner value for 0 <= i2 <= j2 < N, the only entries read
@@ -288,7 +288,7 @@ struct FinShape {
     static constexpr int LD = NP + 4;  // row pitch of the tables: an odd number of 16-byte chunks
     // table (4 words before it, one row after it), two copies of S2, bases
     static constexpr size_t SMEM = ((size_t)4 + (3 * NP + 1) * LD) * sizeof(float) + NP;
-    static constexpr int MINB = 768 / THREADS;  // at most 80 registers
+    static constexpr int MINB = 768 / THREADS;  // at most 80 registers (512 threads: 128, one CTA per SM)
 };
 
 // (BI, BJ) of the q-th block of the upper block triangle (row-major triangle order)
