@@ -574,10 +574,10 @@ int build_plan(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int
             }
         }
     }
-    // S1 of diagonal d+1 is computed by the finalize launch of diagonal d (same class)
+    // S1 of diagonal d+1 is computed by the finalize launch of diagonal d (same class); it stays 0 up to a span of 3
     for (auto &fl : P.fin_launches)
         for (const auto &nx : P.fin_launches)
-            if (nx.d == fl.d + 1 && nx.np == fl.np) { fl.s1_first = nx.first; fl.s1_count = nx.count; }
+            if (nx.d > 3 && nx.d == fl.d + 1 && nx.np == fl.np) { fl.s1_first = nx.first; fl.s1_count = nx.count; }
     // the persistent fill: width classes <= 64 only, not the R0-only mode, not the reference-layout
     // fill with its per-diagonal copy-out (both keep the graph of per-diagonal launches)
     P.copyout = ctx->copyout;
@@ -686,7 +686,7 @@ void launch_fin_t(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
 template <int NB>
 void launch_fin(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
 {
-    if (L.count > fin_bulk_per_sm(8 * NB) * ctx->sms) return launch_fin_t<NB, FIN_BULK_THREADS>(ctx, L, s);
+    if (L.count > fin_bulk_per_sm(8 * NB) * ctx->sms) return launch_fin_t<NB, fin_bulk_threads(8 * NB)>(ctx, L, s);
     if constexpr (fin_has_mid(8 * NB))
         if (L.count > ctx->sms) return launch_fin_t<NB, FIN_MID_THREADS>(ctx, L, s);
     launch_fin_t<NB, fin_threads(8 * NB)>(ctx, L, s);
@@ -734,7 +734,7 @@ int set_smem_attr(bpmax_ctx *ctx)
     if ((st = prefer_smem(ctx, r0_kernel<NB>)) || (st = prefer_smem(ctx, r0_kernel<NB, 1>)) ||
         (st = prefer_smem(ctx, finalize_small_kernel<8 * NB>)) || (st = prefer_smem(ctx, r0only_finalize_small_kernel<8 * NB>)))
         return st;
-    if ((st = prefer_smem(ctx, finalize_small_kernel<8 * NB, FIN_BULK_THREADS>))) return st;
+    if ((st = prefer_smem(ctx, finalize_small_kernel<8 * NB, fin_bulk_threads(8 * NB)>))) return st;
     if constexpr (fin_has_mid(8 * NB)) {
         if ((st = prefer_smem(ctx, finalize_small_kernel<8 * NB, FIN_MID_THREADS>))) return st;
         CK(cudaFuncSetAttribute(finalize_small_kernel<8 * NB, FIN_MID_THREADS>,
@@ -755,9 +755,9 @@ int set_smem_attr(bpmax_ctx *ctx)
                                                      R0Cfg<NB, 1>::SMEM));
     CK(cudaFuncSetAttribute(finalize_small_kernel<8 * NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                             (int)FinShape<8 * NB>::SMEM));
-    CK(cudaFuncSetAttribute(finalize_small_kernel<8 * NB, FIN_BULK_THREADS>,
+    CK(cudaFuncSetAttribute(finalize_small_kernel<8 * NB, fin_bulk_threads(8 * NB)>,
                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)FinShape<8 * NB, FIN_BULK_THREADS>::SMEM));
+                            (int)FinShape<8 * NB, fin_bulk_threads(8 * NB)>::SMEM));
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctx->r0_occ_v[0][NB], r0_kernel<NB>, R0Cfg<NB>::THREADS,
                                                      R0Cfg<NB>::SMEM));
     CK(cudaFuncSetAttribute(fill_persistent_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)R0Cfg<NB>::SMEM));

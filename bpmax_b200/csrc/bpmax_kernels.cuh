@@ -229,11 +229,17 @@ struct CellJob {
 // warps for widths >= 48 (256x64 15.8 -> 15.6, 200x56 7.80 -> 7.64, 512x64 86.9 -> 86.0). Fill ms with the
 // latency threads for up to 1,024 / 296 / 148 cells: 1024x64 622 / 602 / 601, 256x64 16.2 / 16.2 / 15.8;
 // the 512-pair batch at 256 / 160 / 128 threads beyond: 428 / 419 / 418. Up to 148 cells 128x64 takes 4.44 with 256 threads
-// and 4.09 with 512, 64x32 0.83 with 128, 0.73 with 256 and 0.71 with 384.
+// and 4.09 with 512, 64x32 0.83 with 128, 0.73 with 256 and 0.71 with 384. The one to three blocks of widths 8
+// and 16 are work for one warp: 32 threads, 32 CTAs per SM, from three cells per SM on (10,000 pairs 3x6 at 128 / 64 /
+// 32 threads 0.499 / 0.435 / 0.400, 1,000 pairs 16x16 2.49 / 2.34 / 2.24; up to three cells per SM 5 pairs 60x16
+// 0.616 / 0.624 / 0.657). Width 24 keeps 128 throughout: one warp gains 9% there at 1,000 pairs of 16 and loses 5% at 4
+// of 300.
 constexpr int fin_threads(int NP) { return NP >= 48 ? 512 : (NP >= 32 ? 384 : 128); }
-constexpr int FIN_BULK_THREADS = 128, FIN_MID_THREADS = 256;
-constexpr int fin_bulk_per_sm(int NP) { return NP >= 48 ? 3 : 1; }  // bulk launches: more cells per SM than this
-constexpr bool fin_has_mid(int NP) { return fin_bulk_per_sm(NP) > 1; }
+constexpr int fin_bulk_threads(int NP) { return NP <= 16 ? 32 : 128; }
+constexpr int FIN_MID_THREADS = 256;
+// bulk launches: more cells per SM than this
+constexpr int fin_bulk_per_sm(int NP) { return NP >= 48 || NP <= 16 ? 3 : 1; }
+constexpr bool fin_has_mid(int NP) { return NP >= 48; }
 // element (r, c) of tile (I2, J2) of an outer cell in the reference layout (tiles of T+1 rows, the
 // last one the halo; R = padding rows/columns of the first tile row/column); val(i2, j2) gives the
 // cell's inner value for 0 <= i2 <= j2 < N, the only entries read
@@ -288,7 +294,8 @@ struct FinShape {
     static constexpr int LD = NP + 4;  // row pitch of the tables: an odd number of 16-byte chunks
     // table (4 words before it, one row after it), two copies of S2, bases
     static constexpr size_t SMEM = ((size_t)4 + (3 * NP + 1) * LD) * sizeof(float) + NP;
-    static constexpr int MINB = 768 / THREADS;  // at most 80 registers (512 threads: 128, one CTA per SM)
+    // at most 80 registers (512 threads: 128, one CTA per SM; 32 threads: 64, every CTA slot of an SM)
+    static constexpr int MINB = THREADS == 32 ? 32 : 768 / THREADS;
 };
 
 // (BI, BJ) of the q-th block of the upper block triangle (row-major triangle order)
@@ -437,7 +444,8 @@ finalize_small_kernel(const CellJob *__restrict__ jobs, int njobs, const CellJob
     __shared__ float w5[25];   // intra-strand weight of bases a, b at 5a + b
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid < 12) wsh[tid] = W.w[tid];
-    if (tid >= 32 && tid < 57) w5[tid - 32] = score_w(W.w, (tid - 32) / 5, (tid - 32) % 5);
+    for (int q = tid - (T >= 64 ? 32 : 0); q < 25; q += T)
+        if (q >= 0) w5[q] = score_w(W.w, q / 5, q % 5);
     if (tid < NB) cbs[tid] = 4 * c_img_colbase[NB][tid];
     __syncthreads();
     if ((int)blockIdx.x >= njobs) {  // S1 cells (i, i+d+1), one per warp
