@@ -107,16 +107,12 @@ struct Plan {
     // outer diagonal plus the tile diagonal. np = inner table width class; strip (product launches): strips
     // of diagonals d .. d+T-1
     // cap: at most this many CTAs (0: as many as are resident), from the class shares
-    // r0_kernel launches of one pair: q offset pairs per job of `edge` (0: jobs from the list)
+    // r0_kernel launches of one pair: q offset pairs per job of `edge`, by arithmetic (0: jobs from the list)
     struct Launch {
         int d, np, first, count, s1_first = 0, s1_count = 0;
         bool strip = false;
         int cap = 0, cells = 0, q = 0, edge = 0;
         int tile_first = 0, tile_count = 0;  // finalize launches of tile tables: the tiles (count: cells)
-        R0Jobs jobs(const void *list) const
-        {
-            return q ? R0Jobs{nullptr, cells, q, edge} : R0Jobs{(const R0Job *)list + first, 0, 0, 0};
-        }
     };
     std::vector<Launch> r0_launches, fin_launches;
     std::vector<R0Job> r0_jobs;
@@ -556,7 +552,7 @@ int build_plan(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int
                 const long long q = r0_pairs_per_job(cells, edge, resident, qmin, qmax, P.merge_items);
                 Plan::Launch rl{d, np, (int)P.r0_jobs.size(), 0};
                 rl.cap = share.empty() ? 0 : (int)resident;
-                if (n == 1) {
+                if (n == 1 && P.r0_variant == 0) {
                     rl.cells = (int)cells;
                     rl.q = (int)q;
                     rl.edge = (int)edge;
@@ -642,8 +638,13 @@ void launch_r0_v(bpmax_ctx *ctx, const Plan::Launch &L, cudaStream_t s)
     using C = R0Cfg<NB, V>;
     // resident CTAs (or the class's share of them); each loops over jobs
     const int grid = std::min(L.count, L.cap > 0 ? L.cap : std::max(1, ctx->r0_occ_v[V][NB]) * ctx->sms);
-    launch_chain(ctx->one_chain, grid, C::THREADS, C::SMEM, s, r0_kernel<NB, V>, L.jobs(ctx->r0jobs.p), L.count,
-                 (const PairDesc *)ctx->pairs.p, (float *)ctx->F.p, L.d, wait_ctl(ctx));
+    auto go = [&](auto kernel, auto jobs) {
+        launch_chain(ctx->one_chain, grid, C::THREADS, C::SMEM, s, kernel, jobs, L.count, (const PairDesc *)ctx->pairs.p,
+                     (float *)ctx->F.p, L.d, wait_ctl(ctx));
+    };
+    if constexpr (V == 0)
+        if (L.q) return go(r0_kernel<NB, V, R0Jobs>, R0Jobs{L.cells, L.q, L.edge});
+    go(r0_kernel<NB, V>, R0List{(const R0Job *)ctx->r0jobs.p + L.first});
 }
 
 template <int NB>
@@ -731,7 +732,8 @@ template <int NB>
 int set_smem_attr(bpmax_ctx *ctx)
 {
     int st;
-    if ((st = prefer_smem(ctx, r0_kernel<NB>)) || (st = prefer_smem(ctx, r0_kernel<NB, 1>)) ||
+    if ((st = prefer_smem(ctx, r0_kernel<NB>)) || (st = prefer_smem(ctx, r0_kernel<NB, 0, R0Jobs>)) ||
+        (st = prefer_smem(ctx, r0_kernel<NB, 1>)) ||
         (st = prefer_smem(ctx, finalize_small_kernel<8 * NB>)) || (st = prefer_smem(ctx, r0only_finalize_small_kernel<8 * NB>)))
         return st;
     if ((st = prefer_smem(ctx, finalize_small_kernel<8 * NB, fin_bulk_threads(8 * NB)>))) return st;
@@ -750,6 +752,7 @@ int set_smem_attr(bpmax_ctx *ctx)
             (st = prefer_smem(ctx, tile_final_kernel<2>)) || (st = prefer_smem(ctx, tile_final_kernel<3>)))
             return st;
     CK(cudaFuncSetAttribute(r0_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)R0Cfg<NB>::SMEM));
+    CK(cudaFuncSetAttribute(r0_kernel<NB, 0, R0Jobs>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)R0Cfg<NB>::SMEM));
     CK(cudaFuncSetAttribute(r0_kernel<NB, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)R0Cfg<NB, 1>::SMEM));
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctx->r0_occ_v[1][NB], r0_kernel<NB, 1>, R0Cfg<NB, 1>::THREADS,
                                                      R0Cfg<NB, 1>::SMEM));
@@ -1839,11 +1842,10 @@ __global__ void noalloc_prep_kernel(const int *__restrict__ seqs, int M, int N, 
 template <int NB>
 int noalloc_set_attr(int *occ)
 {
-    if (cudaFuncSetAttribute(r0_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)R0Cfg<NB>::SMEM) !=
-        cudaSuccess)
+    const auto kernel = r0_kernel<NB, 0, R0Jobs>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)R0Cfg<NB>::SMEM) != cudaSuccess)
         return BPMAX_ECUDA;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[NB], r0_kernel<NB>, R0Cfg<NB>::THREADS, R0Cfg<NB>::SMEM) !=
-        cudaSuccess)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[NB], kernel, R0Cfg<NB>::THREADS, R0Cfg<NB>::SMEM) != cudaSuccess)
         return BPMAX_ECUDA;
     return cudaFuncSetAttribute(finalize_small_kernel<8 * NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)FinShape<8 * NB>::SMEM) == cudaSuccess ? BPMAX_OK : BPMAX_ECUDA;
@@ -1886,7 +1888,7 @@ void noalloc_launch_diag(cudaStream_t s, const NoallocDevice &nd, int d, const R
 {
     if (d > 0)
         launch_chain(true, std::min(n_r0, std::max(1, nd.occ[NB]) * nd.sms), R0Cfg<NB>::THREADS, R0Cfg<NB>::SMEM, s,
-                     r0_kernel<NB>, rj, n_r0, pd, F, d, WaitCtl{err, NOALLOC_WAIT_NS, 0});
+                     r0_kernel<NB, 0, R0Jobs>, rj, n_r0, pd, F, d, WaitCtl{err, NOALLOC_WAIT_NS, 0});
     const int n_s1 = n_cells - 1;  // S1 cells of diagonal d+1: the first n_cells-1 entries of cj
     using Sh = FinShape<8 * NB>;
     launch_chain(Sh::THREADS < 512, n_cells + (n_s1 + Sh::WARPS - 1) / Sh::WARPS, Sh::THREADS, Sh::SMEM, s,
@@ -1973,7 +1975,7 @@ extern "C" int bpmax_gpu_score_noalloc(const int *seq1, long M, const int *seq2,
     for (int d = 0; d < (int)M; ++d) {
         const int cells = (int)M - d;
         int n_r0 = 0;
-        R0Jobs rj{nullptr, cells, 1, (d + 1) / 2};
+        R0Jobs rj{cells, 1, (d + 1) / 2};
         if (d > 0) {
             rj.q = (int)r0_pairs_per_job(cells, rj.pairs, resident, qmin, 1 << 20, 2);
             n_r0 = cells * ((rj.pairs + rj.q - 1) / rj.q);
