@@ -508,8 +508,8 @@ int build_plan(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int
                 // Strips of T cells (bpmax_strip.cuh), once per T diagonals d .. d+T-1 (d = 1 mod T): the
                 // offsets [0, d-1], of which cell t of a strip takes those >= t. The first t offset pairs
                 // of diagonal d+t, which meet diagonals >= d, are the jobs of r0_kernel. Diagonals
-                // with little work keep r0_kernel alone: a strip launch adds a launch to the chain and
-                // clears T merge tiles per CTA. Fill ms with strips everywhere / from 400 / 1,200 (10 width-64
+                // with few offsets (strip_min_d) or little work keep r0_kernel alone: a strip launch adds a
+                // launch to the chain and clears T merge tiles per CTA (strip_tasks = 0: strips everywhere). Fill ms with strips everywhere / from 400 / 1,200 (10 width-64
                 // items) / 3,400 tasks per SM / nowhere: 37x23 0.41 / 0.35 / 0.35 / 0.35 / 0.35, 100x64
                 // 2.56 / 2.56 / 2.56 / 2.66 / 2.67, 128x64 3.86 / 3.86 / 3.86 / 4.10 / 4.10, 128x32 1.93 /
                 // 1.88 / 1.81 / 1.82 / 1.81, 200x64 9.1 / 9.1 / 9.1 / 9.1 / 10.2, 256x64 15.5 / 15.5 / 15.5 /
@@ -522,7 +522,9 @@ int build_plan(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int
                 for (int p = 0; p < n; ++p)
                     if (P.pairs[p].Np == np && Ms[p] > d0) cells0 += Ms[p] - d0;
                 // tasks of an item: NB(NB+1)(NB+2)/6
-                if (NB >= STRIP_MIN_NB && cells0 * d0 * (NB * (NB + 1) * (NB + 2) / 6) >= P.strip_tasks * ctx->sms) {
+                const bool enough = d0 >= strip_min_d(NB) &&
+                                    cells0 * d0 * (NB * (NB + 1) * (NB + 2) / 6) >= P.strip_tasks * ctx->sms;
+                if (NB >= STRIP_MIN_NB && (P.strip_tasks == 0 || enough)) {
                     edge = std::min<long long>(P2, d - d0);
                     if (d == d0) {
                         const long long stages = (d + G - 1) / G;  // of G offsets

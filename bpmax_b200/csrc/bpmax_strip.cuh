@@ -48,6 +48,15 @@ constexpr int STRIP_MIN_NB = 2;
 // (9 at NB = 2, whose two stages of 24 k1 leave no shared memory for a fourth cell)
 __host__ __device__ constexpr int strip_cells(int nb) { return nb == 7 ? 4 : 3; }
 
+// Strips are taken from this outer diagonal on: a job holds one strip's offsets, and with few of them
+// most of a stage's K values of k1 stay empty (as in the T-1 stages of one k1 at its head), while the first offset
+// pairs of the later cells are merged by r0_kernel besides. Fill ms with strips from diagonal 1 / 10 / 25 / 37 / 49 / 79 /
+// never: 100 pairs 60x16 (K = 24) 5.78 / 5.78 / 5.12 / 4.75 / 4.55 / 4.54 / 4.55, 20 of 200x16 20.1 / 20.1 / 19.6 / 19.2 / 18.9 /
+// 18.6 / 20.3; 30 of 90x24 (12) 5.87 / 5.87 / 5.58 / 5.50 / 5.49 / 5.71 / 5.72; 100 of 60x32 (6) 8.54 / 8.28 / 7.83 / 7.73 / 7.85 /
+// 8.04 / 8.43; 30 of 90x48 (2) 12.0 / 11.9 / 11.8 / 11.9 / 12.1 / 12.3 / 12.3; 100 of 60x64 (1) 21.7 / 21.6 / 22.4 / 23.5 / 24.8 /
+// 25.2 / 25.2.
+__host__ __device__ constexpr int strip_min_d(int nb) { return nb >= 7 ? 9 : (nb >= 5 ? 25 : (nb == 4 ? 37 : (nb == 3 ? 49 : 79))); }
+
 template <int NB>
 struct StripCfg {
     static constexpr int GT = R0_TAB_THREADS[NB];  // threads per group

@@ -142,7 +142,8 @@ int bpmax_gpu_grad_batch(bpmax_ctx *ctx, int num_pairs, const int *const *seq1s,
  *                                launches per outer diagonal. The R0-only mode and bpmax_gpu_fill's
  *                                per-diagonal copy-out keep the graph.
  *   BPMAX_TUNE_STRIP_TASKS       least product work of a strip launch (strand-2 lengths 9..64: one
- *                                launch for several outer diagonals), in 8x8x8 tasks per SM; 0: strips
+ *                                launch for several outer diagonals), in 8x8x8 tasks per SM, on the
+ *                                diagonals long enough for strips (from 9 to 79, by the length); 0: strips
  *                                wherever a diagonal has offsets for them (default 1200) */
 enum bpmax_tuning_key {
     BPMAX_TUNE_R0_PAIRS_PER_JOB = 0,
