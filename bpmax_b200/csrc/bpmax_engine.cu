@@ -21,9 +21,11 @@
 #include <mutex>
 #include <set>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
+
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include "../../include/bpmax_gpu.h"
 #include "bpmax_kernels.cuh"
@@ -182,6 +184,7 @@ struct bpmax_ctx {
     std::map<std::vector<int>, Tuned> tuned;  // shape signature (Ms then Ns) -> tunables
     float *host_stage[2] = {nullptr, nullptr};
     void *copy_stage = nullptr;  // pinned buffers of copy_out
+    size_t fresh_bytes = 0;      // copied into fresh pageable memory so far
     size_t host_stage_bytes = 0;
     cudaEvent_t stage_ev[2] = {nullptr, nullptr};
     Plan plan;
@@ -1156,24 +1159,58 @@ int ensure_host_stage(bpmax_ctx *ctx, size_t bytes)
     return BPMAX_OK;
 }
 
-bool is_pinned(const void *p);
+cudaMemoryType memory_type(const void *p)
+{
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return cudaMemoryTypeUnregistered;
+    }
+    return at.type;
+}
+
+bool is_pinned(const void *p) { return memory_type(p) == cudaMemoryTypeHost; }
+
+// Whether more than a sixteenth of the pages of [dst, dst + bytes) are missing, as in an array never written; not where
+// the system cannot tell.
+bool is_fresh(const void *dst, size_t bytes)
+{
+    constexpr size_t CHUNK = (size_t)2 << 20;
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    const uintptr_t lo = ((uintptr_t)dst + page - 1) / page * page, hi = ((uintptr_t)dst + bytes) / page * page;
+    unsigned char here[CHUNK / 4096];
+    size_t missing = 0;
+    for (uintptr_t p = lo; p < hi; p += CHUNK) {
+        const size_t n = std::min<uintptr_t>(CHUNK, hi - p), pages = n / page;
+        if (mincore((void *)p, n, here) != 0) return false;
+        missing += std::count_if(here, here + pages, [](unsigned char c) { return !(c & 1); });
+    }
+    return missing * page > bytes / 16;
+}
 
 // Copies `bytes` of device memory to dst, after the work queued on the context's stream, and waits. Into
-// pageable memory of COPY_SPLIT bytes or more: COPY_THREADS threads take chunks in turn, each through two
+// fresh pageable memory of COPY_SPLIT bytes or more: COPY_THREADS threads take chunks in turn, each through two
 // pinned buffers of its own on a class stream, so one chunk crosses PCIe while another is copied to its
-// place. One thread copies at 4 to 9 GB/s here and pays every first touch of a fresh array (33.8 MB: 5 to
-// 8 ms), which the driver's own staged copy leaves on one thread. 128x32 table: 10.1 -> 4.9 ms a call
-// (4.5 with chunks of 512 KB, whose 8 MB of pinned buffers cost a new context 5 ms, against 1).
-constexpr size_t COPY_SPLIT = (size_t)2 << 20, COPY_CHUNK = (size_t)128 << 10;
+// place. The driver's own staged copy runs at 16 to 19 GB/s, but faults in a fresh array's pages one after another,
+// at 2 GB/s (5 in 2 MB pages). ms per table, plain copy / threads: into an array in use 3.1 MB 0.25 / 0.30, 31 MB 2.0 / 2.4;
+// into a fresh one 1.46 / 0.43 and 14.2 / 2.7. The pinned buffers take 1 to 3 ms to allocate: a context has them
+// from its COPY_WORTH bytes into fresh memory on (first table of a context, plain / with that allocation: 6.2 MB
+// 3.2 / 3.5, 9.4 MB 4.9 / 4.0). 128x32 table into a new array: 10.1 -> 4.9 ms a call (4.5 with chunks of 512 KB, whose
+// 8 MB of pinned buffers cost a new context 5 ms).
+constexpr size_t COPY_SPLIT = (size_t)2 << 20, COPY_CHUNK = (size_t)128 << 10, COPY_WORTH = (size_t)8 << 20;
 constexpr int COPY_THREADS = MAX_CLASS_STREAMS;
 int copy_out(bpmax_ctx *ctx, void *dst, const void *src, size_t bytes)
 {
     const int threads = (int)std::min<size_t>(std::min<size_t>(COPY_THREADS, bytes / COPY_CHUNK),
                                               std::max(1u, std::thread::hardware_concurrency()));
-    bool split = bytes >= COPY_SPLIT && threads >= 2 && !is_pinned(dst);
+    bool split = bytes >= COPY_SPLIT && threads >= 2 && memory_type(dst) == cudaMemoryTypeUnregistered && is_fresh(dst, bytes);
+    if (split) {
+        ctx->fresh_bytes += bytes;
+        split = ctx->fresh_bytes >= COPY_WORTH;
+    }
     if (split && !ctx->copy_stage &&
         cudaMallocHost(&ctx->copy_stage, 2 * COPY_THREADS * COPY_CHUNK) != cudaSuccess) {
-        cudaGetLastError();  // no pinned memory left: one copy, as for small tables
+        cudaGetLastError();  // no pinned memory left: the plain copy
         ctx->copy_stage = nullptr;
         split = false;
     }
@@ -1209,23 +1246,13 @@ int copy_out(bpmax_ctx *ctx, void *dst, const void *src, size_t bytes)
     int started = 1;  // this thread is the first worker, and does the parts of any that could not start
     try {
         for (; started < threads; ++started) pool[started] = std::thread(work, started);
-    } catch (const std::system_error &) {
+    } catch (...) {
     }
     work(0);
     for (int t = started; t < threads; ++t) work(t);
     for (int t = 1; t < started; ++t) pool[t].join();
     for (int t = 0; t < threads; ++t) CK(errs[t]);
     return BPMAX_OK;
-}
-
-bool is_pinned(const void *p)
-{
-    cudaPointerAttributes at;
-    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return at.type == cudaMemoryTypeHost;
 }
 
 }  // namespace

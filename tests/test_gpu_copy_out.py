@@ -1,0 +1,84 @@
+"""Tables read into host memory: an array in use, fresh pages, odd addresses, device memory; and the first
+table of a context."""
+import ctypes
+import mmap
+import time
+
+import numpy as np
+import pytest
+import torch
+
+from bpmax_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+M, N = 60, 64
+
+
+@pytest.fixture()
+def eng():
+    from bpmax_b200 import Engine
+
+    e = Engine(0)
+    e.set_weights(W.INTEGER_WEIGHTS)
+    e.score(*W.pair(M, N, 3))
+    yield e
+    e.close()
+
+
+def read(e, rows, cols, address):
+    return e._L.bpmax_gpu_read_cells(e._ctx, 0, 0, rows, 0, cols, ctypes.c_void_p(address))
+
+
+@pytest.mark.parametrize("rows,cols", [(2, 60), (2, 64 - 4), (3, 43), (5, 60), (11, 47), (31, 60)])
+@pytest.mark.parametrize("offset", [0, 4, 4096 - 4, 4096 + 20])
+def test_fresh_pages_and_odd_addresses(eng, rows, cols, offset):
+    """Around 2 MB and above; the bytes before and after the table stay as they are."""
+    n = rows * cols * N * N
+    exp = eng.read_cells(0, 0, rows, 0, cols, N).reshape(-1)
+    buf = mmap.mmap(-1, 4 * n + 3 * 4096)
+    raw = np.frombuffer(buf, np.uint8)
+    raw[:offset] = 0x5A
+    raw[offset + 4 * n:] = 0xA5
+    assert read(eng, rows, cols, raw.ctypes.data + offset) == 0
+    got = raw[offset:offset + 4 * n].view(np.uint32)
+    assert np.array_equal(got, exp.view(np.uint32))
+    assert np.all(raw[:offset] == 0x5A) and np.all(raw[offset + 4 * n:] == 0xA5)
+
+
+def test_device_destination_is_treated_the_same_at_every_size(eng):
+    """Whatever the driver makes of a device address as the host destination, a large table is no
+    different from a small one."""
+    out = []
+    for rows, cols in ((1, 4), (40, 60)):
+        n = rows * cols * N * N
+        dst = torch.zeros(n, dtype=torch.float32, device="cuda")
+        torch.cuda.synchronize()
+        st = read(eng, rows, cols, dst.data_ptr())
+        out.append(st)
+        if st == 0:
+            torch.cuda.synchronize()
+            exp = eng.read_cells(0, 0, rows, 0, cols, N).reshape(-1)
+            assert np.array_equal(dst.cpu().numpy().view(np.uint32), exp.view(np.uint32))
+    assert out[0] == out[1]
+
+
+def test_first_table_of_a_context_costs_what_later_ones_do():
+    from bpmax_b200 import Engine
+
+    rows, cols = 4, 50
+    n = rows * cols * N * N  # 3.3 MB
+    warm = np.zeros(n, np.float32)
+    pin = torch.empty(n, pin_memory=True)
+    first, later = [], []
+    for _ in range(7):
+        e = Engine(0)
+        try:
+            e.score(*W.pair(M, N, 3))
+            assert read(e, rows, cols, pin.data_ptr()) == 0  # the conversion buffer
+            for k in range(6):
+                t = time.perf_counter()
+                assert read(e, rows, cols, warm.ctypes.data) == 0
+                (later if k else first).append(time.perf_counter() - t)
+        finally:
+            e.close()
+    assert np.median(first) < 2.5 * np.median(later), (first, later)
