@@ -1758,9 +1758,11 @@ int bpmax_gpu_autotune(bpmax_ctx *ctx, int num_pairs, const int *const *seq1s, c
         ctx->class_share = c[5];
         ctx->persist = c[6];
         float t = -1.f;
-        for (int r = 0; r < 1 + std::max(1, trials) && st == BPMAX_OK; ++r) {  // first run captures the graph
+        // the first run has no graph, the second captures it and is its first launch (37x23: 0.38 and 0.45 ms
+        // against 0.35 of a replay)
+        for (int r = 0; r < 2 + std::max(1, trials) && st == BPMAX_OK; ++r) {
             st = fill_pairs(ctx, num_pairs, seq1s, Ms, seq2s, Ns);
-            if (st == BPMAX_OK && r > 0 && (t < 0 || ctx->last_ms < t)) t = ctx->last_ms;
+            if (st == BPMAX_OK && r > 1 && (t < 0 || ctx->last_ms < t)) t = ctx->last_ms;
         }
         if (st == BPMAX_OK && (best_t < 0 || t < best_t)) {
             best_t = t;

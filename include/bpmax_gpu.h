@@ -161,7 +161,7 @@ int bpmax_gpu_set_tuning(bpmax_ctx *ctx, int key, long value);
 int bpmax_gpu_get_tuning(const bpmax_ctx *ctx, int key, long *value);
 
 /* Autotuner: fills the given pairs under candidate settings of the schedule tunables, timing
- * `trials` graph replays of each after one capture run, and keeps the fastest setting for these
+ * `trials` graph replays of each after two untimed runs (the second captures the graph), and keeps the fastest setting for these
  * shapes: later fills of the same shapes use it. It first tries every combination of pairs per job
  * (8 / 32 / unbounded), merge cost (1 / 4) and class streams (on / off, when the batch has several
  * width classes) with the default kernel shapes, then, on the best of those, the other product
