@@ -202,25 +202,25 @@ r0_strip_kernel(const StripJob *__restrict__ jobs, int njobs, const PairDesc *__
         cur.cells = min(C::T, M - j1);
     };
     // the producing warp fills a free stage with the next K k1 of its jobs; after the last, the closing
-    // record that lets the warps leave
-    auto produce = [&](int stage) {
-        if (cur.job >= njobs) {
-            if (lane == 0 && cur.job != 0x7fffffff) {
+    // record that lets the warps leave. With one k1 a stage (K == 1) lane 0 alone does this and nothing else
+    // touches the cursor; otherwise every lane issues copies, and lane 0 moves the cursor once all have read it.
+    auto produce_lanes = [&](int stage) {
+        const int job = cur.job, left = cur.left, b_step = cur.b_step, w = cur.w;
+        const unsigned long long a_src = cur.a_src, b_src = cur.b_src;
+        // offsets below a cell's place in the strip are not its: one k1 a stage there, for cells 0 .. w
+        const int valid = C::K == 1 || w < C::T - 1 ? 1 : min(C::K, left), cells = min(cur.cells, w + 1);
+        const long long out = cur.out;
+        if constexpr (C::K > 1) __syncwarp();  // every lane has read the cursor
+        if (job >= njobs) {
+            if (lane == 0 && job != 0x7fffffff) {
                 rec[stage].info = -1;
                 mbar_arrive(full_u + 8 * stage);
                 armed[stage] += 1;
                 cur.job = 0x7fffffff;
             }
-            __syncwarp();
             return;
         }
-        const int left = cur.left, b_step = cur.b_step, w = cur.w;
-        const unsigned long long a_src = cur.a_src, b_src = cur.b_src;
-        // offsets below a cell's place in the strip are not its: one k1 a stage there, for cells 0 .. w
-        const int valid = C::K == 1 || w < C::T - 1 ? 1 : min(C::K, left), cells = min(cur.cells, w + 1);
-        const long long out = cur.out;
         const unsigned bar = full_u + 8 * stage, dst = smem_u32(sm) + stage * C::STAGE_BYTES;
-        if constexpr (C::K > 1) __syncwarp();  // every lane has read the cursor
         if (lane == 0) {
             rec[stage] = StripRec{valid | cells << 8, left == valid, out};
             mbar_arrive_tx(bar, (unsigned)(valid * (1 + cells) * C::IMG * 16));
@@ -242,8 +242,11 @@ r0_strip_kernel(const StripJob *__restrict__ jobs, int njobs, const PairDesc *__
         }
         if (lane == 0 && left == valid) {
             cp_async_wait<0>();
-            open_job(cur.job + gridDim.x, cur.next);
+            open_job(job + gridDim.x, cur.next);
         }
+    };
+    auto produce = [&](int stage) {
+        if (C::K > 1 || lane == 0) produce_lanes(stage);
         __syncwarp();
     };
     if (warp == C::PW) {
