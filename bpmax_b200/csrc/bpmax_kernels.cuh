@@ -310,9 +310,9 @@ __device__ __forceinline__ void blk_decode(int NB, int q, int &BI, int &BJ)
 // The inner wavefront of R1, R2 and SW2 inside a table (tri: an upper triangle of nb block rows) or a
 // 64x64 tile, by 8x8 blocks, block diagonal by block diagonal; all threads of the CTA. T[r][c] holds the
 // start values (-inf below the diagonal, in columns >= ncol, in column -1 and in the row after the
-// last) and receives the final ones; SJ[x][y] = S2(x, y) of the columns' strand piece (-inf in columns
-// >= ncol), SX[x][y] = S2(x, y-1) of the rows'; wt[LD*b + c] = the SW2 weight of row base b and column c;
-// rb = the rows' bases; entry (r, c) spans j2-i2 = e0 + c - r.
+// last) and receives the final ones; SJ[x][y] = S2(x, y) of the columns' strand piece, SX[x][y] = S2(x, y-1)
+// of the rows'; wt[LD*b + c] = the SW2 weight of row base b and column c; SJ and wt are -inf in columns >= ncol,
+// which keeps T -inf there; rb = the rows' bases; entry (r, c) spans j2-i2 = e0 + c - r.
 //   1. one warp per block adds the terms over the finished blocks of its row and column,
 //        R1  T[r][k] + S2(k+1, c),  R2  S2(r, k-1) + T[k][c],
 //      as products, four lanes sharing the k of a 2x4 piece, and SW2 from outside the block;
@@ -438,7 +438,7 @@ finalize_small_kernel(const CellJob *__restrict__ jobs, int njobs, const CellJob
     constexpr int LD = Sh::LD;
     float *D = fsm + 4, *SX = D + (NP + 1) * LD, *SJ = SX + NP * LD;  // the table; S2(r, c-1) and S2(r, c)
     uint8_t *sb = reinterpret_cast<uint8_t *>(SJ + NP * LD);
-    __shared__ __align__(16) float wt[5 * LD];  // wt[LD*x + c]: intra-strand weight of base x and column c
+    __shared__ __align__(16) float wt[5 * LD];  // wt[LD*x + c]: intra-strand weight of base x and column c, -inf from N on
     __shared__ int cbs[NB];    // float offset of each block column in the cell image
     __shared__ float wsh[12];  // the weight table (indexed by pair type)
     __shared__ float w5[25];   // intra-strand weight of bases a, b at 5a + b
@@ -484,7 +484,7 @@ finalize_small_kernel(const CellJob *__restrict__ jobs, int njobs, const CellJob
     for (int q = tid; q < NP; q += Sh::THREADS) sb[q] = q < N ? s2r[q] : 4;
     for (int q = tid; q < 5 * LD; q += Sh::THREADS) {
         const int c = q % LD;
-        wt[q] = w5[5 * (q / LD) + (c < N ? s2r[c] : 4)];
+        wt[q] = c < N ? w5[5 * (q / LD) + s2r[c]] : NEG_INF;
     }
     const int x1 = s1[i1], y1 = s1[j1];
     chain_wait();

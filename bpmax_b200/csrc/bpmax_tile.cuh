@@ -130,7 +130,7 @@ tile_final_kernel(const TileJob *__restrict__ jobs, int njobs, const CellJob *__
     extern __shared__ __align__(16) float tsm[];
     float *T = tsm + 4;
     __shared__ float wsh[12], w5[25];
-    __shared__ __align__(16) float wt[5 * LD];  // wt[LD*x + c]: weight of base x and column c of the tile
+    __shared__ __align__(16) float wt[5 * LD];  // wt[LD*x + c]: weight of base x and column c of the tile, -inf from ncol on
     __shared__ uint8_t bI[64], bJ[64];
     __shared__ float below[64], s2r_end[64];  // F[64(I+1)][64J+c] and S2(64I+r, 64I+63)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -178,7 +178,7 @@ tile_final_kernel(const TileJob *__restrict__ jobs, int njobs, const CellJob *__
         if (t == 0 || q < 0 || q % LD >= ncol || q >= 64 * LD) T[q] = NEG_INF;
     for (int q = tid; q < 5 * LD; q += TILE_THREADS) {
         const int c = q % LD;
-        wt[q] = w5[5 * (q / LD) + (c < 64 ? bJ[c] : 4)];
+        wt[q] = c < ncol ? w5[5 * (q / LD) + bJ[c]] : NEG_INF;
     }
     // four columns of one block row per step; every load of a thread is issued before the first is used
     constexpr int Q = 1024 / TILE_THREADS;
