@@ -164,11 +164,9 @@ __global__ void single_strand_kernel(const PairDesc *__restrict__ pairs, const u
 {
     const PairDesc pd = pairs[blockIdx.x];
     if (pd.Np > S2_ONE_CTA_NP) return;  // one launch per diagonal (s2_diag_kernel)
-    const bool second = true;
-    const int L = second ? pd.N : pd.M;
-    const int ld = second ? pd.Np : pd.M;
-    const uint8_t *s = bases + (second ? pd.seq2_off : pd.seq1_off);
-    float *T = S + (second ? pd.S2_off : pd.S1_off);
+    const int L = pd.N, ld = pd.Np;
+    const uint8_t *s = bases + pd.seq2_off;
+    float *T = S + pd.S2_off;
     for (int idx = threadIdx.x; idx < ld * ld; idx += blockDim.x) T[idx] = 0.0f;
     __syncthreads();
     for (int d = 4; d < L; ++d) {
