@@ -40,9 +40,10 @@ _REF_CLI_CHECK = os.path.join(HERE, "_ref", "bpmax_gpu_cli_check")  # the same, 
 
 
 def reference_root() -> str | None:
-    """The reference project's root: $REFERENCE_ROOT, else its mount in the build container."""
+    """The reference project's root: $REFERENCE_ROOT, else its mount in the build container; None where its
+    sources are not there (an empty mount)."""
     root = os.environ.get("REFERENCE_ROOT") or "/root/reference"
-    return root if os.path.isdir(root) else None
+    return root if os.path.isdir(os.path.join(root, "TPDS", "source")) else None
 
 
 def build(targets=()) -> None:
