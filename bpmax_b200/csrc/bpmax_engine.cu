@@ -8,7 +8,8 @@
 //       offset pairs (w, d-1-w), ordered by offset pair so both uses of a table meet in L2; from a
 //       certain size on, the strip kernel takes most offsets of several diagonals in one launch;
 //     finalize kernel over the same cells (init, SW1, inner R1/R2/SW2 wavefront).
-// The whole sequence is captured once per shape as a CUDA graph and replayed.
+// A plan's first run launches the sequence as it is; when its shapes come again it is captured as a CUDA
+// graph, which the later runs replay.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -512,7 +513,8 @@ int build_plan(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int
                 // offsets [0, d-1], of which cell t of a strip takes those >= t. The first t offset pairs
                 // of diagonal d+t, which meet diagonals >= d, are the jobs of r0_kernel. Diagonals
                 // with few offsets (strip_min_d) or little work keep r0_kernel alone: a strip launch adds a
-                // launch to the chain and clears T merge tiles per CTA (strip_tasks = 0: strips everywhere). Fill ms with strips everywhere / from 400 / 1,200 (10 width-64
+                // launch to the chain and clears T merge tiles per CTA (strip_tasks = 0: strips everywhere).
+                // Fill ms, with strips from diagonal 1 on, everywhere / from 400 / 1,200 (10 width-64
                 // items) / 3,400 tasks per SM / nowhere: 37x23 0.41 / 0.35 / 0.35 / 0.35 / 0.35, 100x64
                 // 2.56 / 2.56 / 2.56 / 2.66 / 2.67, 128x64 3.86 / 3.86 / 3.86 / 4.10 / 4.10, 128x32 1.93 /
                 // 1.88 / 1.81 / 1.82 / 1.81, 200x64 9.1 / 9.1 / 9.1 / 9.1 / 10.2, 256x64 15.5 / 15.5 / 15.5 /
@@ -936,7 +938,7 @@ int enqueue_fill(bpmax_ctx *ctx, Plan &P, KernelProfile *kp = nullptr)
             }
         }
         // outer diagonal d is final: rows of the reference layout that end on it can be copied out
-        // (events recorded as external nodes of the captured graph; eager runs record none)
+        // (in a captured graph the events are external nodes)
         if (!P.diag_ev.empty() && !prof && d >= lag && P.diag_ev[d - lag])
             CK(cudaEventRecordWithFlags(P.diag_ev[d - lag], ctx->stream, capturing ? cudaEventRecordExternal : cudaEventRecordDefault));
     }
@@ -1046,7 +1048,7 @@ int prepare(bpmax_ctx *ctx, const std::vector<int> &Ms, const std::vector<int> &
     return BPMAX_OK;
 }
 
-// Launches the fill of the current plan (graph captured on first use) on the context's stream.
+// Launches the fill of the current plan on the context's stream.
 int launch_fill(bpmax_ctx *ctx)
 {
     Plan &P = ctx->plan;

@@ -29,7 +29,7 @@
 // whole ring waits for it), hence the cursor that only adds. r0_kernel took 1,240 with 20,160 bytes
 // per item, against 13,440 here. Fill: 1024x64 766 -> 661 ms, the 512-pair batch 523 -> 460 ms;
 // 661 -> 616 and 428 -> 424 since cell t takes every offset that meets final tables (before, only those that
-// all T cells share).
+// all T cells share); 601 -> 595.5 since lane 0 alone refills stages of one k1.
 #pragma once
 #include <cstddef>
 

@@ -125,7 +125,7 @@ int bpmax_gpu_grad_batch(bpmax_ctx *ctx, int num_pairs, const int *const *seq1s,
  *                                without issuing any operand copy, so their first waits run out with
  *                                no copy in flight; the call returns BPMAX_ETIMEOUT and later calls
  *                                are unaffected. A test of the timeout path; 0 otherwise.
- *   BPMAX_TUNE_WIDE_STAGES       shared-memory stages of the product kernel for strand-2 lengths 65..320
+ *   BPMAX_TUNE_WIDE_STAGES       shared-memory stages of the product kernel for strand-2 lengths over 64
  *                                (2: three CTAs per SM; 3: two CTAs per SM with a deeper copy ring)
  *   BPMAX_TUNE_R0_VARIANT        shape of the product kernel for strand-2 lengths <= 64 (0: three CTAs
  *                                per SM, 168 registers, 2-4 stages; 1: two CTAs per SM, up to 255
@@ -138,9 +138,11 @@ int bpmax_gpu_grad_batch(bpmax_ctx *ctx, int num_pairs, const int *const *seq1s,
  *                                persistent launch per width class that walks the outer diagonals as a
  *                                wavefront with device-side dependency counters (bounded waits); with
  *                                several width classes, 1 runs them side by side (each on its share of
- *                                the SMs), 2 one after another (each on every SM); 0: a graph of two
- *                                launches per outer diagonal. The R0-only mode and bpmax_gpu_fill's
- *                                per-diagonal copy-out keep the graph.
+ *                                the SMs), 2 one after another (each on every SM); 0: a few launches
+ *                                per outer diagonal (product and finalize, strips of several diagonals;
+ *                                skewed steps for lengths over 64), as they are in a plan's first run and as
+ *                                a graph from its second on. The R0-only mode and bpmax_gpu_fill's
+ *                                copy-out keep these launches.
  *   BPMAX_TUNE_STRIP_TASKS       least product work of a strip launch (strand-2 lengths 9..64: one
  *                                launch for several outer diagonals), in 8x8x8 tasks per SM, on the
  *                                diagonals long enough for strips (from 9 to 79, by the length); 0: strips
@@ -166,7 +168,7 @@ int bpmax_gpu_get_tuning(const bpmax_ctx *ctx, int key, long *value);
  * (8 / 32 / unbounded), merge cost (1 / 4) and class streams (on / off, when the batch has several
  * width classes) with the default kernel shapes, then, on the best of those, the other product
  * kernel shape (BPMAX_TUNE_R0_VARIANT 1, when a strand-2 length is <= 64) and the deeper tile ring
- * (BPMAX_TUNE_WIDE_STAGES 3, when one is in 65..320), after trying class shares
+ * (BPMAX_TUNE_WIDE_STAGES 3, when one is over 64), after trying class shares
  * (BPMAX_TUNE_CLASS_SHARE 1, when class streams won with several width classes), then the persistent
  * fill with each pairs-per-job candidate (BPMAX_TUNE_PERSISTENT 1, or 2 with several width classes,
  * when every strand-2 length is <= 64).
