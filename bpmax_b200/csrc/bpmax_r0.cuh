@@ -67,7 +67,7 @@ struct R0Jobs {
     int cells, q, pairs;
     __device__ __forceinline__ R0Job operator[](int j) const
     {
-        const int c = j / cells;
+        const int c = (int)((unsigned)j / (unsigned)cells);
         return R0Job{0, j - c * cells, c * q, min(c * q + q, pairs)};
     }
 };
